@@ -4,10 +4,9 @@
 // filling: 15,876 to 2.9 M amplitudes) psi and sigma of all B parameter sets
 // are stored state-minor, amplitude i of slot s at [i * B + s], so the B
 // slots of one amplitude are contiguous and every access below is coalesced
-// across slots.  A program step is one launch over (pair, slot): the pairs
-// are the alpha-list x beta-list products of the step's record (the same
-// records as the shared-memory path, qfb_sector.cuh), read from global
-// memory.  sigma = H psi runs one warp per output amplitude with the lanes
+// across slots.  Runs of program steps go out as windows (qfb_swin.cuh); a
+// step by itself is one launch over (pair, slot): the pairs are the alpha-list
+// x beta-list products of the step's record, read from global memory.  sigma = H psi runs one warp per output amplitude with the lanes
 // over slots, from the sector's H rows, or (rows over their budget) one
 // x-group of H per launch from pair records.  When H and every step are real
 // the states are stored as doubles (V = double), else as complex (double2).
@@ -50,7 +49,7 @@ using qfbs::v_zero;
 // One step record over (pair, slot): lane l of a warp takes slot
 // group * spw + l % spw and pair sub-index l / spw.  ROT rotates psi (and
 // sigma when TWO) by sign * gamma * theta_slot; IP accumulates <sigma|K|psi>
-// per slot into partial[(row * B + s) * gridDim.x + blockIdx.x].
+// per slot (real part: the gradient's) into partial[s * gridDim.x + blockIdx.x].
 // Programmatic dependent launch: a kernel launched with programmatic stream
 // serialization waits here for the grid before it in the stream (and its
 // memory), then lets the grid after it begin launching, so at most two grids
@@ -63,8 +62,8 @@ __device__ __forceinline__ void g_pdl_enter() {
 
 template <bool ROT, bool IP, bool TWO, class V>
 __global__ void __launch_bounds__(256) k_cg_step(GLaunch L, const uint4 *__restrict__ rec,
-                                                 int param, int sign, int row,
-                                                 double2 *__restrict__ partial) {
+                                                 int param, int sign,
+                                                 double *__restrict__ partial) {
     g_pdl_enter();
     V *psi = reinterpret_cast<V *>(L.psi), *sig = reinterpret_cast<V *>(L.sig);
     __shared__ double2 s_acc[8][32];
@@ -124,7 +123,7 @@ __global__ void __launch_bounds__(256) k_cg_step(GLaunch L, const uint4 *__restr
         double2 t = make_double2(0.0, 0.0);
         for (int w = 0; w < nwarp; ++w) t = g_cadd(t, s_acc[w][threadIdx.x]);
         const int ss = blockIdx.y * L.spw + threadIdx.x;
-        if (ss < L.B) partial[((size_t)row * L.B + ss) * gridDim.x + blockIdx.x] = t;
+        if (ss < L.B) partial[(size_t)ss * gridDim.x + blockIdx.x] = t.x;
     }
 }
 

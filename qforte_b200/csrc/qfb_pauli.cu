@@ -47,6 +47,7 @@
 #include "qfb_common.cuh"
 #include "qfb_csec.cuh"
 #include "qfb_sector.cuh"
+#include "qfb_swin.cuh"
 #include "qfb_window.cuh"
 
 using namespace qfb;
@@ -2277,7 +2278,31 @@ struct PairPlanDev {
     ~PairPlanDev() { dev_free(blob); }
 };
 
+// A plan's steps as windows on blocks of the sector (qfb_swin.cuh), with the
+// device tables its evaluators share.
+struct WinProg {
+    struct Op {
+        int rec = -1;        // >= 0: one step by itself (record of the stream)
+        int param = 0, fl = 0;
+        int64_t poff = 0;    // its partials (R_IP)
+        qfbv::VWin w{};
+    };
+    std::vector<Op> ops;
+    qfbv::VTabs tabs{};
+    int nang = 0;
+    const double *gamma = nullptr;  // angle table: factor and parameter per step
+    const int32_t *aparam = nullptr;
+    unsigned dgrid = 1;             // blocks of the steps by themselves
+    int64_t npart = 0;              // partials (per slot)
+    const int2 *pspan = nullptr;    // per parameter: its spans ...
+    const longlong2 *span = nullptr;  // ... of partials (offset, count)
+    void *blob = nullptr;
+    size_t bytes = 0;
+    ~WinProg() { dev_free(blob); }
+};
+
 struct SectorPlan {
+    std::shared_ptr<WinProg> wfwd, wsweep;  // global-memory path
     int na_orb = 0, nb_orb = 0, nalpha = 0, nbeta = 0, nsec = 0, ref_i = 0;
     int ka = 0, kb = 0;  // alpha and beta electrons of the sector
     std::shared_ptr<SectorPlanDev> dev;
@@ -2636,6 +2661,331 @@ static int pair_plan(SectorPlan &sp, int S, std::shared_ptr<PairPlanDev> *out) {
     return QFB_OK;
 }
 
+// ---- windows of steps on blocks of the sector (qfb_swin.cuh) ---------------
+
+// Amplitudes of the largest block of a window, and of the blocks small
+// windows are filled up to.  Larger blocks mean fewer windows, each with its
+// launch and its read and write of the state, but more pairs a step (more
+// rounds) and fewer blocks to fill the SMs.  Forward + sweep of the SD
+// program, us at caps of 420 / 800 / 1300 / 2000 amplitudes: 18 qubits, one
+// set 376 / 315 / 298 / 296; 18 qubits, 24 sets 929 / 823 / 757 / 748; 20
+// qubits, one set 836 / 606 / 548 / 495; 20 qubits, 6 sets 1643 / 1295 / 1166 / 1134.
+constexpr int kWinCap = 2000;
+constexpr int kWinFill = 300;
+constexpr size_t kWinSmemMax = 220 * 1024;
+constexpr int64_t kWinPairs = 16384;  // pair words of one block
+constexpr int kWinMinSteps = 3;  // shorter runs take one launch per step
+
+struct WinRef {
+    const CStep *cs;
+    int flags, rec;
+};
+
+// One spin's strings split into classes by their bits outside Q.
+struct WinClasses {
+    std::vector<int32_t> cls, loc;           // per rank
+    std::vector<std::vector<uint16_t>> str;  // ranks per class
+};
+
+static WinClasses win_classes(const std::vector<uint64_t> &det, uint64_t Q) {
+    WinClasses c;
+    std::unordered_map<uint64_t, int32_t> id;
+    for (size_t r = 0; r < det.size(); ++r) {
+        auto it = id.emplace(det[r] & ~Q, (int32_t)c.str.size());
+        if (it.second) c.str.emplace_back();
+        const int32_t k = it.first->second;
+        c.cls.push_back(k);
+        c.loc.push_back((int32_t)c.str[(size_t)k].size());
+        c.str[(size_t)k].push_back((uint16_t)r);
+    }
+    return c;
+}
+
+// Strings of the largest class: q of m orbitals inside, k electrons.
+static int64_t win_max_class(int m, int k, int q) {
+    auto binom = [](int n, int r) -> int64_t {
+        if (r < 0 || r > n) return 0;
+        int64_t b = 1;
+        for (int i = 0; i < r; ++i) b = b * (n - i) / (i + 1);
+        return b;
+    };
+    int64_t best = 0;
+    for (int o = 0; o <= m - q; ++o) best = std::max(best, binom(q, k - o));
+    return best;
+}
+
+static int build_windows(const SectorPlan &sp, const std::vector<WinRef> &refs, int nparam,
+                         std::shared_ptr<WinProg> *out) {
+    const size_t n = refs.size();
+    auto P = std::make_shared<WinProg>();
+    std::vector<uint64_t> xa(n, 0), xb(n, 0);
+    for (size_t i = 0; i < n; ++i)
+        if (!refs[i].cs->pats.empty()) {
+            const auto &pt = refs[i].cs->pats[0];
+            xa[i] = sp.adet[pt.a[0].r0] ^ sp.adet[pt.a[0].r1];
+            xb[i] = sp.bdet[pt.b[0].r0] ^ sp.bdet[pt.b[0].r1];
+        }
+    auto block = [&](uint64_t qa, uint64_t qb) {
+        return win_max_class(sp.na_orb, sp.ka, __builtin_popcountll(qa)) *
+               win_max_class(sp.nb_orb, sp.kb, __builtin_popcountll(qb));
+    };
+    std::vector<qfbv::VClass> cls;
+    std::vector<uint16_t> rank;
+    std::vector<uint32_t> blob;
+    std::vector<qfbv::VItem> items;
+    std::vector<double> gamma;
+    std::vector<int32_t> aparam;
+    std::vector<std::vector<longlong2>> spans((size_t)std::max(nparam, 1));
+    int64_t dmax = 1;
+    for (const WinRef &r : refs) {
+        int64_t pairs = 0;
+        for (const auto &pt : r.cs->pats) pairs += (int64_t)pt.a.size() * (int64_t)pt.b.size();
+        dmax = std::max(dmax, pairs);
+    }
+    P->dgrid = (unsigned)std::min<int64_t>(1024, (dmax + 63) / 64);
+    std::map<uint64_t, WinClasses> ca_of, cb_of;  // by Q
+    auto classes = [](std::map<uint64_t, WinClasses> &m, const std::vector<uint64_t> &det,
+                      uint64_t Q) -> const WinClasses & {
+        auto it = m.find(Q);
+        if (it == m.end()) it = m.emplace(Q, win_classes(det, Q)).first;
+        return it->second;
+    };
+    // one spin's classes and blobs of the items, and each item's largest count
+    // in a class; false when a blob outgrows its limit
+    auto emit_spin = [&](const WinClasses &C, const std::vector<const std::vector<qfbs::SEntry> *> &lists,
+                         int32_t &c0, int32_t &mwords, int32_t &mstr, std::vector<int64_t> &most) {
+        const size_t nc = C.str.size(), ni = lists.size();
+        std::vector<std::vector<uint32_t>> ent(nc), off(nc);
+        for (size_t k = 0; k < ni; ++k) {
+            for (size_t c = 0; c < nc; ++c) off[c].push_back((uint32_t)ent[c].size());
+            for (const qfbs::SEntry &e : *lists[k])
+                ent[(size_t)C.cls[e.r0]].push_back((uint32_t)C.loc[e.r0] |
+                                                   (uint32_t)C.loc[e.r1] << qfbv::kWinIdx |
+                                                   (e.s & 1u) << (2 * qfbv::kWinIdx));
+        }
+        most.assign(ni, 0);
+        for (size_t c = 0; c < nc; ++c)
+            for (size_t k = 0; k < ni; ++k)
+                most[k] = std::max(most[k], (int64_t)((k + 1 < ni ? off[c][k + 1] : ent[c].size()) - off[c][k]));
+        const uint32_t head = (uint32_t)(2 * ni + 1);
+        mwords = mstr = 0;
+        for (size_t c = 0; c < nc; ++c) {
+            off[c].push_back((uint32_t)ent[c].size());
+            if (head + ent[c].size() > (size_t)qfbv::kWinBlobMax) return false;
+            mwords = std::max(mwords, (int32_t)(head + ent[c].size()));
+            mstr = std::max(mstr, (int32_t)C.str[c].size());
+        }
+        c0 = (int32_t)cls.size();
+        for (size_t c = 0; c < nc; ++c) {
+            cls.push_back(qfbv::VClass{(int32_t)rank.size(), (int32_t)C.str[c].size(), (int32_t)blob.size(),
+                                       (int32_t)(head + ent[c].size())});
+            rank.insert(rank.end(), C.str[c].begin(), C.str[c].end());
+            for (size_t k = 0; k <= ni; ++k) blob.push_back(head + off[c][k]);
+            for (size_t k = 0; k < ni; ++k) {
+                const uint32_t m = off[c][k + 1] - off[c][k];
+                blob.push_back(m < 2 ? 0u : (uint32_t)(((1ull << 32) + m - 1) / m));
+            }
+            blob.insert(blob.end(), ent[c].begin(), ent[c].end());
+        }
+        return true;
+    };
+    auto step_angle = [&](const WinRef &r) {
+        gamma.push_back(r.cs->gamma);
+        aparam.push_back(r.cs->param);
+        return (int32_t)gamma.size() - 1;
+    };
+    size_t lim = n;  // end of the window at hand when its pairs outgrew kWinPairs
+    for (size_t i = 0; i < n;) {
+        uint64_t qa = 0, qb = 0;
+        size_t j = i, ni = 0;
+        while (j < lim) {
+            const size_t k = ni + refs[j].cs->pats.size();
+            if (k > (size_t)qfbv::kWinItems || block(qa | xa[j], qb | xb[j]) > kWinCap) break;
+            qa |= xa[j];
+            qb |= xb[j];
+            ni = k;
+            ++j;
+        }
+        if (j - i >= (size_t)kWinMinSteps && ni > 0) {
+            // small blocks: more orbitals into Q, lowest first, the spin with fewer
+            while (true) {
+                const int pa = __builtin_popcountll(qa), pb = __builtin_popcountll(qb);
+                int orb = -1, odd = -1;
+                for (int o : {pa <= pb ? 0 : 1, pa <= pb ? 1 : 0}) {
+                    const int m = o ? sp.nb_orb : sp.na_orb;
+                    for (int q = 0; q < m && orb < 0; ++q)
+                        if (!((o ? qb : qa) >> (2 * q + o) & 1ull)) {
+                            orb = q;
+                            odd = o;
+                        }
+                    if (orb >= 0) break;
+                }
+                if (orb < 0) break;
+                const uint64_t bit = 1ull << (2 * orb + odd);
+                const uint64_t ta = odd ? qa : qa | bit, tb = odd ? qb | bit : qb;
+                if (block(ta, tb) > kWinFill) break;
+                qa = ta;
+                qb = tb;
+            }
+            const WinClasses &CA = classes(ca_of, sp.adet, qa), &CB = classes(cb_of, sp.bdet, qb);
+            std::vector<const std::vector<qfbs::SEntry> *> la, lb;
+            for (size_t s = i; s < j; ++s)
+                for (const auto &pt : refs[s].cs->pats) {
+                    la.push_back(&pt.a);
+                    lb.push_back(&pt.b);
+                }
+            WinProg::Op op;
+            qfbv::VWin &w = op.w;
+            const size_t m0 = cls.size(), m1 = rank.size(), m2 = blob.size();
+            int32_t wa = 0, wb = 0, sa = 0, sb = 0;
+            std::vector<int64_t> pa, pb;
+            int64_t pairs = 0;
+            const bool fits = emit_spin(CA, la, w.ca0, wa, sa, pa) && emit_spin(CB, lb, w.cb0, wb, sb, pb);
+            // warps a slot: the count whose rounds take least, a round of 1, 2,
+            // 4, 8 warps costing as its barrier does
+            double best = 1e300;
+            for (int lg = 0; fits && lg <= 3; ++lg) {
+                static const double cost[4] = {1.0, 1.06, 1.2, 1.5};
+                int64_t nr = 0;
+                for (size_t k = 0; k < pa.size(); ++k)
+                    nr += std::max<int64_t>(1, (pa[k] * pb[k] + (32 << lg) - 1) >> (5 + lg));
+                if ((double)nr * cost[lg] < best) {
+                    best = (double)nr * cost[lg];
+                    w.lg = lg;
+                    w.nround = (int32_t)nr;
+                    pairs = nr << (5 + lg);
+                }
+            }
+            bool ok = fits;
+            if (ok && pairs > kWinPairs && j - i > (size_t)kWinMinSteps) {  // fewer steps
+                cls.resize(m0);
+                rank.resize(m1);
+                blob.resize(m2);
+                lim = i + std::max<size_t>(kWinMinSteps, (size_t)((double)(j - i) * 0.9 * kWinPairs / pairs));
+                continue;
+            }
+            ok = ok && pairs <= kWinPairs;
+            lim = n;
+            if (ok) {
+                w.nca = (int32_t)CA.str.size();
+                w.ncb = (int32_t)CB.str.size();
+                w.item0 = (int32_t)items.size();
+                w.nitem = (int32_t)la.size();
+                w.mab = sa * sb;
+                w.mranks = sa + sb;
+                w.mwords = wa + wb;
+                const int64_t nblk = (int64_t)w.nca * w.ncb;
+                size_t at = 0;
+                int32_t r0 = 0;
+                for (size_t s = i; s < j; ++s) {
+                    if (refs[s].cs->pats.empty()) continue;
+                    const int32_t ang = step_angle(refs[s]);
+                    for (const auto &pt : refs[s].cs->pats) {
+                        qfbv::VItem it{};
+                        it.gamma = refs[s].cs->gamma;
+                        it.ang = ang;
+                        it.fl = refs[s].flags;
+                        it.gn = pt.gn;
+                        it.hn = pt.hn;
+                        it.r0 = r0;
+                        r0 += (int32_t)std::max<int64_t>(1, (pa[at] * pb[at] + (32 << w.lg) - 1) >> (5 + w.lg));
+                        it.r1 = r0;
+                        ++at;
+                        if (it.fl & qfbs::R_IP) {
+                            it.poff = P->npart;
+                            spans[(size_t)refs[s].cs->param].push_back(make_longlong2(P->npart, nblk));
+                            P->npart += nblk;
+                        }
+                        items.push_back(it);
+                    }
+                }
+                P->ops.push_back(op);
+                i = j;
+                continue;
+            }
+            cls.resize(m0);
+            rank.resize(m1);
+            blob.resize(m2);
+        }
+        lim = n;
+        j = std::max(j, i + 1);
+        for (; i < j; ++i) {
+            if (refs[i].cs->pats.empty()) continue;
+            WinProg::Op op;
+            op.rec = refs[i].rec;
+            op.param = refs[i].cs->param;
+            op.fl = refs[i].flags;
+            if (op.fl & qfbs::R_IP) {
+                op.poff = P->npart;
+                spans[(size_t)op.param].push_back(make_longlong2(P->npart, (int64_t)P->dgrid));
+                P->npart += P->dgrid;
+            }
+            P->ops.push_back(op);
+        }
+    }
+    std::vector<int2> pspan;
+    std::vector<longlong2> span;
+    for (const auto &v : spans) {
+        pspan.push_back(make_int2((int)span.size(), (int)(span.size() + v.size())));
+        span.insert(span.end(), v.begin(), v.end());
+    }
+    P->nang = (int)gamma.size();
+    struct Up {
+        const void *p;
+        size_t n, o;
+    } ups[] = {{cls.data(), sizeof(qfbv::VClass) * cls.size(), 0},
+               {rank.data(), sizeof(uint16_t) * rank.size(), 0},
+               {blob.data(), sizeof(uint32_t) * blob.size(), 0},
+               {items.data(), sizeof(qfbv::VItem) * items.size(), 0},
+               {gamma.data(), sizeof(double) * gamma.size(), 0},
+               {aparam.data(), sizeof(int32_t) * aparam.size(), 0},
+               {pspan.data(), sizeof(int2) * pspan.size(), 0},
+               {span.data(), sizeof(longlong2) * span.size(), 0}};
+    size_t off = 0;
+    for (Up &x : ups) {
+        x.o = off;
+        off += (std::max<size_t>(x.n, 16) + 255) & ~(size_t)255;
+    }
+    const int rc = dev_alloc(&P->blob, off);
+    if (rc) return rc;
+    P->bytes = off;
+    char *base = (char *)P->blob;
+    for (const Up &x : ups)
+        if (x.n) QFB_CUDA(cudaMemcpyAsync(base + x.o, x.p, x.n, cudaMemcpyHostToDevice, t_stream));
+    QFB_CUDA(cudaStreamSynchronize(t_stream));
+    P->tabs.cls = (const qfbv::VClass *)(base + ups[0].o);
+    P->tabs.rank = (const uint16_t *)(base + ups[1].o);
+    P->tabs.blob = (const uint32_t *)(base + ups[2].o);
+    P->tabs.item = (const qfbv::VItem *)(base + ups[3].o);
+    P->gamma = (const double *)(base + ups[4].o);
+    P->aparam = (const int32_t *)(base + ups[5].o);
+    P->pspan = (const int2 *)(base + ups[6].o);
+    P->span = (const longlong2 *)(base + ups[7].o);
+    *out = P;
+    return QFB_OK;
+}
+
+// The forward and sweep windows of a plan, built once.
+static int plan_windows(SectorPlan &sp, int nparam) {
+    if (!sp.wfwd) {
+        std::vector<WinRef> refs;
+        for (size_t i = 0; i < sp.fsteps.size(); ++i)
+            refs.push_back(WinRef{&sp.fsteps[i], qfbs::R_ROT, (int)i});
+        const int rc = build_windows(sp, refs, nparam, &sp.wfwd);
+        if (rc) return rc;
+    }
+    if (!sp.wsweep) {
+        std::vector<WinRef> refs;
+        for (size_t i = 0; i < sp.sweep_items.size(); ++i) {
+            const auto &it = sp.sweep_items[i];
+            refs.push_back(WinRef{it.unrot ? &sp.usteps[it.step] : &sp.ksteps[it.step], it.flags, (int)i});
+        }
+        const int rc = build_windows(sp, refs, nparam, &sp.wsweep);
+        if (rc) return rc;
+    }
+    return QFB_OK;
+}
+
 struct qfb_ucc_s {
     qfb_prog_s *fwd = nullptr;
     qfb_prog_s *grad = nullptr;   // K_mu (inner products)
@@ -2675,8 +3025,11 @@ struct qfb_ucc_s {
     int gsec = 0;
     qfbg::GLaunch GL{};
     const uint4 *g_frec = nullptr, *g_srec = nullptr;  // device copies of the record streams
-    unsigned g_sgrid = 1, g_hgrid = 1, g_ygrid = 1;
+    unsigned g_hgrid = 1, g_ygrid = 1;
     double2 *g_epart = nullptr;
+    void *wblob = nullptr;       // windows: angle tables and gradient partials
+    double2 *g_fang = nullptr, *g_sang = nullptr;
+    double *g_wpart = nullptr;
     // H without rows: the x-groups' launches run on kHChains concurrent
     // chains, chain k adding into its own sigma copy (k = 0: GL.sig)
     void *hblob = nullptr;  // sigma copies of chains 1..
@@ -3136,6 +3489,22 @@ static void sector_h_shape(qfb_ucc u, int nsec) {
     u->h_slices = best;
 }
 
+static int win_smem_attr() {
+    static std::once_flag once;
+    static cudaError_t err = cudaSuccess;
+    std::call_once(once, [] {
+        auto attr = [](const void *f) {
+            if (err == cudaSuccess)
+                err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWinSmemMax);
+        };
+        attr((const void *)qfbv::k_win<false, double>);
+        attr((const void *)qfbv::k_win<true, double>);
+        attr((const void *)qfbv::k_win<false, double2>);
+        attr((const void *)qfbv::k_win<true, double2>);
+    });
+    return err == cudaSuccess ? QFB_OK : cuda_fail(err, "window shared memory");
+}
+
 // Attach a compact plan and its H rows to an evaluator (shared memory or,
 // with `global`, global memory states).
 static int sector_attach(qfb_ucc u, qfb_sum_s *ham, const std::shared_ptr<SectorPlan> &plan,
@@ -3195,6 +3564,20 @@ static int sector_attach(qfb_ucc u, qfb_sum_s *ham, const std::shared_ptr<Sector
         if (e != cudaSuccess) return cuda_fail(e, "sector H chains");
     }
     if (global) {
+        rc = plan_windows(sp, u->nparam);
+        if (rc) return rc;
+        const size_t B = (size_t)u->nbatch;
+        auto al = [](size_t x) { return (std::max<size_t>(x, 16) + 255) & ~(size_t)255; };
+        const size_t bf = al(sizeof(double2) * B * sp.wfwd->nang), bs = al(sizeof(double2) * B * sp.wsweep->nang);
+        const size_t bp = al(sizeof(double) * B * (size_t)sp.wsweep->npart);
+        rc = dev_alloc(&u->wblob, bf + bs + bp);
+        if (rc) return rc;
+        u->bytes += bf + bs + bp + sp.wfwd->bytes + sp.wsweep->bytes;
+        u->g_fang = (double2 *)u->wblob;
+        u->g_sang = (double2 *)((char *)u->wblob + bf);
+        u->g_wpart = (double *)((char *)u->wblob + bf + bs);
+        rc = win_smem_attr();
+        if (rc) return rc;
         u->g_frec = d.frec;
         u->g_srec = d.srec;
         u->g_rowptr = rows->rowptr;
@@ -3373,11 +3756,12 @@ static unsigned global_grid(int64_t pairs, int spw) {
 // g_pdl_enter): chains of short dependent launches overlap each launch's
 // latency with the previous grid's run.
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, cudaStream_t st, Args... args) {
+static cudaError_t launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                              Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -3387,13 +3771,73 @@ static cudaError_t launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, cudaSt
     return cudaLaunchKernelEx(&cfg, k, args...);
 }
 
+// Shape of a window launch for B slots: 1 << lspc slots a CTA.
+static void win_shape(const qfbv::VWin &w, int B, bool sweep, size_t elem, int &lspc, size_t &smem) {
+    lspc = 0;
+    // more slots a CTA (they share the lists) once the grid fills the SMs
+    const int64_t nblk = (int64_t)w.nca * w.ncb;
+    while ((1 << lspc) < B && (32 << (w.lg + lspc)) < qfbv::kWinThreads && lspc < 3 &&
+           (nblk * B >> lspc) > (int64_t)2 * sm_count())
+        ++lspc;
+    for (;; --lspc) {
+        smem = qfbv::win_smem(w, 1 << lspc, 1 << (w.lg + lspc), sweep, elem);
+        if (smem <= 110 * 1024 || lspc == 0) break;
+    }
+}
+
+// A window program on L's states: the angle table, then its windows and
+// single steps in order (rev: in reverse order, the inverse program).
+template <class V>
+static int win_program(qfb_ucc u, const WinProg &P, bool sweep, const qfbg::GLaunch &L, const uint4 *recs,
+                       double2 *ang, int sign, bool rev, bool angles) {
+    const SectorPlan &sp = *u->splan;
+    const StreamHost &S = sweep ? sp.sweep : sp.fwd;
+    const int B = L.B;
+    if (angles && P.nang > 0) {
+        const int64_t n = (int64_t)P.nang * B;
+        qfbv::k_win_angles<<<(unsigned)((n + 255) / 256), 256, 0, t_stream>>>(P.gamma, P.aparam, P.nang, B,
+                                                                           L.params, L.nparam, ang);
+        QFB_LAUNCHED();
+    }
+    for (size_t i = 0; i < P.ops.size(); ++i) {
+        const WinProg::Op &op = P.ops[rev ? P.ops.size() - 1 - i : i];
+        if (op.rec >= 0) {
+            const dim3 grid(P.dgrid, u->g_ygrid);
+            const uint4 *rec = recs + S.span[(size_t)op.rec].x;
+            double *part = sweep ? u->g_wpart + op.poff * B : nullptr;
+            if (!sweep)
+                QFB_CUDA(launch_pdl(qfbg::k_cg_step<true, false, false, V>, grid, dim3(256), 0, t_stream, L,
+                                    rec, op.param, sign, part));
+            else if (op.fl == (qfbs::R_ROT | qfbs::R_IP | qfbs::R_TWO))
+                QFB_CUDA(launch_pdl(qfbg::k_cg_step<true, true, true, V>, grid, dim3(256), 0, t_stream, L,
+                                    rec, op.param, sign, part));
+            else if (op.fl == qfbs::R_IP)
+                QFB_CUDA(launch_pdl(qfbg::k_cg_step<false, true, false, V>, grid, dim3(256), 0, t_stream, L,
+                                    rec, op.param, sign, part));
+            else
+                QFB_CUDA(launch_pdl(qfbg::k_cg_step<true, false, true, V>, grid, dim3(256), 0, t_stream, L,
+                                    rec, op.param, sign, part));
+        } else {
+            int lspc;
+            size_t smem;
+            win_shape(op.w, B, sweep, sizeof(V), lspc, smem);
+            const dim3 grid((unsigned)(op.w.nca * op.w.ncb), (unsigned)((B + (1 << lspc) - 1) >> lspc));
+            const dim3 block(32u << (op.w.lg + lspc));
+            QFB_CUDA(launch_pdl(sweep ? qfbv::k_win<true, V> : qfbv::k_win<false, V>, grid, block, smem, t_stream,
+                                L, op.w, P.tabs, (const double2 *)ang, (double)sign, rev ? 1 : 0, lspc,
+                                u->g_wpart));
+        }
+        QFB_LAUNCHED();
+    }
+    return QFB_OK;
+}
+
 // Compact sector in global memory: stage 0 the reference, 1 the forward
-// records, 2 sigma = H psi and the energy, 3 the sweep records.
+// program, 2 sigma = H psi and the energy, 3 the sweep.
 template <class V>
 static int ucc_stage_global_v(qfb_ucc u, int stage, int with_grad) {
     const qfbg::GLaunch &L = u->GL;
     const SectorPlan &sp = *u->splan;
-    const dim3 grid(u->g_sgrid, u->g_ygrid);
     switch (stage) {
         case 0:
             QFB_CUDA(cudaMemsetAsync(L.psi, 0, sizeof(V) * (size_t)L.nsec * L.B, t_stream));
@@ -3401,13 +3845,7 @@ static int ucc_stage_global_v(qfb_ucc u, int stage, int with_grad) {
             QFB_LAUNCHED();
             break;
         case 1:
-            for (size_t r = 0; r < sp.fwd.span.size(); ++r) {
-                QFB_CUDA(launch_pdl(qfbg::k_cg_step<true, false, false, V>, grid, dim3(256), t_stream, L,
-                                    u->g_frec + sp.fwd.span[r].x, sp.fwd.param[r], 1, -1,
-                                    (double2 *)nullptr));
-                QFB_LAUNCHED();
-            }
-            break;
+            return win_program<V>(u, *sp.wfwd, false, L, u->g_frec, u->g_fang, 1, false, true);
         case 2: {
             const dim3 hg(u->g_hgrid, u->g_ygrid);
             if (u->rows->too_big) {
@@ -3443,10 +3881,10 @@ static int ucc_stage_global_v(qfb_ucc u, int stage, int with_grad) {
                     const dim3 rg(global_grid(r.pairs, L.spw), u->g_ygrid);
                     const uint4 *rec = R.d_hrec + r.span.x;
                     if (r.table)
-                        QFB_CUDA(launch_pdl(qfbg::k_cg_h_group<true, V>, rg, dim3(256), sk[k], Lk[k], rec,
+                        QFB_CUDA(launch_pdl(qfbg::k_cg_h_group<true, V>, rg, dim3(256), 0, sk[k], Lk[k], rec,
                                             R.det, gt, u->ham->d_rterms, r.t0, r.t1, r.real, r.x));
                     else
-                        QFB_CUDA(launch_pdl(qfbg::k_cg_h_group<false, V>, rg, dim3(256), sk[k], Lk[k], rec,
+                        QFB_CUDA(launch_pdl(qfbg::k_cg_h_group<false, V>, rg, dim3(256), 0, sk[k], Lk[k], rec,
                                             R.det, gt, u->ham->d_rterms, r.t0, r.t1, r.real, r.x));
                     QFB_LAUNCHED();
                 }
@@ -3476,25 +3914,10 @@ static int ucc_stage_global_v(qfb_ucc u, int stage, int with_grad) {
         }
         default: {
             if (!(with_grad && u->grad && u->nparam > 0)) break;
-            for (size_t r = 0; r < sp.sweep.span.size(); ++r) {
-                qfbs::RHead hd;
-                std::memcpy(&hd, &sp.sweep.rec[sp.sweep.span[r].x], sizeof(hd));
-                const int fl = hd.npf >> 8;
-                const uint4 *rec = u->g_srec + sp.sweep.span[r].x;
-                const int par = sp.sweep.param[r];
-                if (fl == (qfbs::R_ROT | qfbs::R_IP | qfbs::R_TWO))
-                    QFB_CUDA(launch_pdl(qfbg::k_cg_step<true, true, true, V>, grid, dim3(256), t_stream, L,
-                                        rec, par, -1, (int)hd.row, u->gpart));
-                else if (fl == qfbs::R_IP)
-                    QFB_CUDA(launch_pdl(qfbg::k_cg_step<false, true, false, V>, grid, dim3(256), t_stream,
-                                        L, rec, par, -1, (int)hd.row, u->gpart));
-                else
-                    QFB_CUDA(launch_pdl(qfbg::k_cg_step<true, false, true, V>, grid, dim3(256), t_stream, L,
-                                        rec, par, -1, -1, (double2 *)nullptr));
-                QFB_LAUNCHED();
-            }
-            k_grad_final<<<dim3(u->nparam, L.B), 128, 0, t_stream>>>(u->gpart, u->psteps, u->gchunks,
-                                                                   u->gradv);
+            const int rc = win_program<V>(u, *sp.wsweep, true, L, u->g_srec, u->g_sang, -1, false, true);
+            if (rc) return rc;
+            qfbv::k_win_grad<<<dim3(u->nparam, L.B), 128, 0, t_stream>>>(u->g_wpart, sp.wsweep->pspan,
+                                                                       sp.wsweep->span, u->gradv);
             QFB_LAUNCHED();
             break;
         }
@@ -3622,17 +4045,11 @@ static int ucc_resid_stage(qfb_ucc u) {
     if (u->gsec) {
         qfbg::GLaunch Ls = u->GL;  // rotate sigma: the step kernel rotates L.psi
         Ls.psi = u->GL.sig;
-        const SectorPlan &sp = *u->splan;
-        const dim3 grid(u->g_sgrid, u->g_ygrid);
-        for (size_t r = sp.fwd.span.size(); r-- > 0;) {
-            if (u->greal)
-                qfbg::k_cg_step<true, false, false, double><<<grid, 256, 0, t_stream>>>(
-                    Ls, u->g_frec + sp.fwd.span[r].x, sp.fwd.param[r], -1, -1, nullptr);
-            else
-                qfbg::k_cg_step<true, false, false, double2><<<grid, 256, 0, t_stream>>>(
-                    Ls, u->g_frec + sp.fwd.span[r].x, sp.fwd.param[r], -1, -1, nullptr);
-            QFB_LAUNCHED();
-        }
+        // (the angle table is the forward program's, on the same parameters)
+        const WinProg &P = *u->splan->wfwd;
+        const int rc = u->greal ? win_program<double>(u, P, false, Ls, u->g_frec, u->g_fang, -1, true, false)
+                                : win_program<double2>(u, P, false, Ls, u->g_frec, u->g_fang, -1, true, false);
+        if (rc) return rc;
         if (u->greal)
             k_resid_gather<double><<<gg, 256, 0, t_stream>>>((const double *)u->GL.sig, u->ridx,
                                                              (uint64_t)B, 1, u->rphase, u->nres, B,
@@ -3760,9 +4177,6 @@ static int ucc_create_impl(qfb_prog fprog, qfb_prog gprog, qfb_prog uprog, qfb_s
     }
     if (compact || gsec) sector.clear();
     const int spw = gsec ? (int)std::min<int64_t>(32, 1ll << (int)std::ceil(std::log2((double)nbatch))) : 32;
-    const unsigned sgrid = gsec ? global_grid(std::max(stream_max_pairs(splan.fwd),
-                                                       stream_max_pairs(splan.sweep)), spw)
-                                : 1;
     const unsigned hgrid = gsec ? (unsigned)std::min<int64_t>(1024, (splan.nsec + 7) / 8) : 1;
     qfb_ucc u = new qfb_ucc_s;
     u->compact = compact ? 1 : 0;
@@ -3779,7 +4193,7 @@ static int ucc_create_impl(qfb_prog fprog, qfb_prog gprog, qfb_prog uprog, qfb_s
     u->vchunks = grid_for(u->nbasis, 256, 2);
     if (u->vchunks * (unsigned)nbatch > 65535u) u->vchunks = std::max(1u, 65535u / nbatch);
     u->gchunks = compact ? qfbs::kSweepThreads / 32
-                         : gsec ? sgrid : (gprog ? grad_chunks(gprog, nqubit, nbatch) : 1);
+                         : gsec ? 1 : (gprog ? grad_chunks(gprog, nqubit, nbatch) : 1);
     const size_t B = nbatch, M = std::max(u->nparam, 1);
     const size_t nsteps = gprog ? std::max<size_t>(gprog->h_steps.size(), 1) : 1;
     const size_t b_state = (compact || gsec) ? 16 : sizeof(double2) * u->nbasis * B;
@@ -3793,7 +4207,7 @@ static int ucc_create_impl(qfb_prog fprog, qfb_prog gprog, qfb_prog uprog, qfb_s
     const size_t o_par = take(sizeof(double) * B * M), o_en = take(sizeof(double) * B);
     const size_t o_gr = take(sizeof(double) * B * M);
     const size_t o_vp = take(sizeof(double2) * B * u->vchunks);
-    const size_t o_gp = take(gprog ? sizeof(double2) * nsteps * B * u->gchunks : 16);
+    const size_t o_gp = take(gprog && !gsec ? sizeof(double2) * nsteps * B * u->gchunks : 16);
     const size_t o_ps = take(sizeof(int2) * M);
     const size_t idx_bytes = nqubit <= 32 ? sizeof(uint32_t) : sizeof(uint64_t);
     const size_t o_sec = take(idx_bytes * std::max<size_t>(sector.size(), 1));
@@ -3838,7 +4252,6 @@ static int ucc_create_impl(qfb_prog fprog, qfb_prog gprog, qfb_prog uprog, qfb_s
         u->greal = greal ? 1 : 0;
         u->GL.params = u->params;
         u->GL.nparam = u->nparam;
-        u->g_sgrid = sgrid;
         u->g_hgrid = hgrid;
         u->g_ygrid = (unsigned)((nbatch + spw - 1) / spw);
         u->g_epart = (double2 *)(base + o_epart);
@@ -3940,6 +4353,7 @@ int qfb_ucc_destroy(qfb_ucc u) {
         if (x) cudaEventDestroy(x);
     if (u->hfork) cudaEventDestroy(u->hfork);
     dev_free(u->hblob);
+    dev_free(u->wblob);
     dev_free(u->blob);
     delete u;
     return QFB_OK;
