@@ -290,8 +290,8 @@ QFB_API int qfb_ucc_path(qfb_ucc u, int32_t *path);
  * qfb_ucc_config), else 0.  No counterpart in the reference. */
 QFB_API int qfb_ucc_real_states(qfb_ucc u, int32_t *real);
 /* Parameter sets one CTA of the compact shared-memory forward program holds:
- * 2 with real states (two sets in one 16-byte slot per amplitude), 1
- * otherwise, 0 off the compact shared-memory path.  No counterpart in the
+ * 2 with real states (two sets in one 16-byte slot per amplitude, for
+ * batches of more sets than the SMs take at once), 1 otherwise, 0 off the compact shared-memory path.  No counterpart in the
  * reference. */
 QFB_API int qfb_ucc_sets_per_cta(qfb_ucc u, int32_t *sets);
 /* Entries of the H rows the compact path streams for each parameter set (0

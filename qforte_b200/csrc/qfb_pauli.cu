@@ -2180,6 +2180,7 @@ static std::vector<uint64_t> sector_indices(int n, uint64_t ref) {
 // ---------------------------------------------------------------------------
 
 constexpr size_t kSectorSmemMax = 200 * 1024;  // psi + sigma of one parameter set
+constexpr size_t kStepSmemMax = 226 * 1024;  // the step kernels: states and the records' constants
 constexpr int kSectorThreads = 512;
 constexpr int kSectorHSlicesMax = 64;  // row slices of k_sector_h
 constexpr int kHChains = 4;            // concurrent x-group chains of H without rows
@@ -2268,13 +2269,14 @@ struct SectorPlanDev {
     ~SectorPlanDev() { dev_free(blob); }
 };
 
-// Device copies of a plan's pair-list streams (qfbs::PStream) for one bank
-// slot width, uploaded once and shared by the plan's evaluators.
+// Device copies of a plan's streams of rounds (qfbs::RStream) for one bank slot
+// width, uploaded once and shared by the plan's evaluators.
 struct PairPlanDev {
     void *blob = nullptr;
     size_t bytes = 0;
-    qfbs::PStream fwd{}, sweep{};
-    std::vector<qfbs::PHead> fwd_hd;  // host copy (residual streams run it in reverse)
+    // forward, forward for two real sets per CTA, sweep
+    qfbs::RStream fwd{}, fwd2{}, sweep{};
+    const int2 *prange = nullptr;  // rounds of the sweep of each parameter
     ~PairPlanDev() { dev_free(blob); }
 };
 
@@ -2306,7 +2308,7 @@ struct SectorPlan {
     int na_orb = 0, nb_orb = 0, nalpha = 0, nbeta = 0, nsec = 0, ref_i = 0;
     int ka = 0, kb = 0;  // alpha and beta electrons of the sector
     std::shared_ptr<SectorPlanDev> dev;
-    std::shared_ptr<PairPlanDev> pdev[2];  // pair lists ordered for 8 / 16 bank slots
+    std::shared_ptr<PairPlanDev> pdev[2];  // rounds for complex / real states
     std::vector<uint64_t> adet, bdet;
     std::vector<int32_t> arank, brank;
     std::vector<CStep> fsteps, ksteps, usteps;
@@ -2490,7 +2492,7 @@ static bool build_sector_plan(SectorPlan &sp, const qfb_prog_s *fp, const qfb_pr
         }
     }
     if (!shared) return true;
-    const size_t ang = sizeof(qfbs::PSmem<double2>) * std::max(sp.fwd.span.size(), sp.sweep.span.size());
+    const size_t ang = sizeof(qfbs::PCoef<true, double2>) * std::max(sp.fwd.span.size(), sp.sweep.span.size());
     if (nsec * 2 * sizeof(double2) + ang > kSectorSmemMax) return false;
     return true;
 }
@@ -2607,21 +2609,18 @@ static bool push_pairs(PairHost &P, const SectorPlan &sp, const CStep &cs, int f
 static size_t pair_bytes(const PairHost &P) {
     auto al = [](size_t x) { return (std::max<size_t>(x, 16) + 255) & ~(size_t)255; };
     return al(sizeof(qfbs::PHead) * P.hd.size()) +
-           al(sizeof(uint32_t) * (P.pair.size() + qfbs::kPairPad)) + al(sizeof(double2) * P.coef.size());
+           al(sizeof(uint32_t) * P.pair.size()) + al(sizeof(double2) * P.coef.size());
 }
 static int pair_upload(const PairHost &P, char *base, qfbs::PStream &out) {
     auto al = [](size_t x) { return (std::max<size_t>(x, 16) + 255) & ~(size_t)255; };
     char *hd = base, *pr = hd + al(sizeof(qfbs::PHead) * P.hd.size());
-    char *cf = pr + al(sizeof(uint32_t) * (P.pair.size() + qfbs::kPairPad));
+    char *cf = pr + al(sizeof(uint32_t) * P.pair.size());
     if (!P.hd.empty())
         QFB_CUDA(cudaMemcpyAsync(hd, P.hd.data(), sizeof(qfbs::PHead) * P.hd.size(),
                                  cudaMemcpyHostToDevice, t_stream));
     if (!P.pair.empty())
         QFB_CUDA(cudaMemcpyAsync(pr, P.pair.data(), sizeof(uint32_t) * P.pair.size(),
                                  cudaMemcpyHostToDevice, t_stream));
-    QFB_CUDA(cudaMemsetAsync(pr + sizeof(uint32_t) * P.pair.size(), 0,
-                             sizeof(uint32_t) * qfbs::kPairPad, t_stream));
-
     if (!P.coef.empty())
         QFB_CUDA(cudaMemcpyAsync(cf, P.coef.data(), sizeof(double2) * P.coef.size(),
                                  cudaMemcpyHostToDevice, t_stream));
@@ -2632,30 +2631,159 @@ static int pair_upload(const PairHost &P, char *base, qfbs::PStream &out) {
     return QFB_OK;
 }
 
-// The plan's forward and sweep streams as pair lists ordered for S bank slots.
-static int pair_plan(SectorPlan &sp, int S, std::shared_ptr<PairPlanDev> *out) {
-    std::shared_ptr<PairPlanDev> &slot = sp.pdev[S == 16 ? 1 : 0];
+// A stream of rounds on the host: appended step by step.
+struct RoundHost {
+    std::vector<qfbs::RRec> hd;
+    std::vector<std::vector<uint32_t>> pairs;  // per record, as words without round flags
+    std::vector<int32_t> param;                // per record: parameter of its inner product, or -1
+};
+
+// Append one step: a record per pair of pattern coefficients (gn, hn) that
+// differ by more than a sign (a pattern whose coefficients are another's
+// negated joins it with its pairs' signs flipped), its pairs ordered for S
+// bank slots.
+static bool push_rounds(RoundHost &P, const SectorPlan &sp, const CStep &cs, int flags, int S) {
+    if (sp.nsec + qfbs::kRoundPad > (1 << qfbs::kPairIdxBits)) return false;
+    auto is = [](double2 a, double2 b, double f) { return a.x == f * b.x && a.y == f * b.y; };
+    std::vector<char> done(cs.pats.size(), 0);
+    for (size_t k = 0; k < cs.pats.size(); ++k) {
+        if (done[k]) continue;
+        const auto &p0 = cs.pats[k];
+        std::vector<uint32_t> pr;
+        for (size_t l = k; l < cs.pats.size(); ++l) {
+            const auto &pt = cs.pats[l];
+            const bool same = is(pt.gn, p0.gn, 1.0) && is(pt.hn, p0.hn, 1.0);
+            if (done[l] || !(same || (is(pt.gn, p0.gn, -1.0) && is(pt.hn, p0.hn, -1.0)))) continue;
+            done[l] = 1;
+            for (const qfbs::SEntry &ea : pt.a)
+                for (const qfbs::SEntry &eb : pt.b) {
+                    const uint32_t i0 = (uint32_t)ea.r0 * (uint32_t)sp.nbeta + eb.r0;
+                    const uint32_t i1 = (uint32_t)ea.r1 * (uint32_t)sp.nbeta + eb.r1;
+                    const uint32_t neg = ((ea.s ^ eb.s) & 1u) ^ (same ? 0u : 1u);
+                    pr.push_back(i0 | i1 << qfbs::kPairIdxBits | neg << (2 * qfbs::kPairIdxBits));
+                }
+        }
+        if (pr.empty()) continue;
+        order_pairs(pr.data(), pr.size(), S);
+        P.hd.push_back(qfbs::RRec{cs.gamma, cs.param, flags & (qfbs::R_ROT | qfbs::R_IP), p0.gn, p0.hn});
+        P.pairs.push_back(std::move(pr));
+        P.param.push_back((flags & qfbs::R_IP) ? cs.param : -1);
+    }
+    return true;
+}
+
+// Threads of a block that runs a stream: a round takes a fixed latency and
+// each warp's issue slots on top, about 0.07 of it a warp (one set's sweep, us,
+// at 64 / 128 / 256 / 416 / 512 threads: 12 qubits 15.5 / 15.1 / 20.8 / 29 /
+// 33.9, 16 qubits 366 / 216 / 139 / 116 / 122).
+static int round_threads(const RoundHost &P) {
+    double best = 1e300;
+    int nth = 32;
+    for (int t = 32; t <= qfbs::kStepThreads; t += 32) {
+        int64_t nr = 0;
+        for (const auto &pr : P.pairs) nr += ((int64_t)pr.size() + t - 1) / t;
+        const double cost = (double)nr * (1.0 + 0.07 * (t / 32));
+        if (cost < best) {
+            best = cost;
+            nth = t;
+        }
+    }
+    return nth;
+}
+
+// The stream's words for blocks of nth threads, its rounds made a multiple of
+// four by an empty record; range[mu] = the rounds of parameter mu's inner
+// products (consecutive: the sweep takes the parameters one after another).
+static void lay_rounds(RoundHost &P, int nth, int nsec, int nparam, qfbs::RStream &out,
+                       std::vector<uint32_t> &word, std::vector<int2> &range) {
+    auto pad = [&](int t) {
+        const uint32_t i = (uint32_t)(nsec + (t & (qfbs::kRoundPad - 1)));
+        return i << 3 | i << (3 + qfbs::kPairIdxBits);
+    };
+    word.assign((size_t)4 * nth, 0u);
+    range.assign((size_t)std::max(nparam, 1), make_int2(0, 0));
+    int nr = 0;
+    auto rounds = [&](const std::vector<uint32_t> &pr, int cnt) {
+        for (int r = 0; r < cnt; ++r, ++nr)
+            for (int t = 0; t < nth; ++t) {
+                const size_t k = (size_t)r * nth + t;
+                uint32_t w = pad(t);
+                if (k < pr.size()) w = pair_i0(pr[k]) << 3 | pair_i1(pr[k]) << (3 + qfbs::kPairIdxBits) |
+                                       (pr[k] >> (2 * qfbs::kPairIdxBits) & 1u) << 31;
+                word.push_back(w | (r + 1 == cnt ? 1u : 0u) | (r == 0 ? 2u : 0u));
+            }
+    };
+    for (size_t k = 0; k < P.hd.size(); ++k) {
+        const int r0 = nr;
+        rounds(P.pairs[k], (int)((P.pairs[k].size() + nth - 1) / nth));
+        if (P.param[k] >= 0) {
+            int2 &g = range[(size_t)P.param[k]];
+            if (g.y == 0) g.x = r0;
+            g.y = nr;
+        }
+    }
+    if (nr % 4) {
+        P.hd.push_back(qfbs::RRec{0.0, 0, 0, make_double2(0.0, 0.0), make_double2(0.0, 0.0)});
+        rounds({}, 4 - nr % 4);
+    }
+    word.insert(word.end(), (size_t)4 * nth, 0u);
+    out.n = (int)P.hd.size();
+    out.nr = nr;
+    out.nth = nth;
+}
+
+// The plan's forward and sweep streams as rounds.  Complex amplitudes, pairs
+// of real sets and the real sweep's interleaved states are 16-byte words, read
+// by quarter warps over 8 bank slots; one set's real amplitudes half warps
+// over 16.
+static int pair_plan(SectorPlan &sp, bool real, int nparam, std::shared_ptr<PairPlanDev> *out) {
+    std::shared_ptr<PairPlanDev> &slot = sp.pdev[real ? 1 : 0];
     if (slot) {
         *out = slot;
         return QFB_OK;
     }
-    PairHost F, W;
+    RoundHost F, F2, W;
     for (const CStep &cs : sp.fsteps)
-        if (!push_pairs(F, sp, cs, qfbs::R_ROT, -1, S))
+        if (!push_rounds(F, sp, cs, qfbs::R_ROT, real ? 16 : 8) ||
+            (real && !push_rounds(F2, sp, cs, qfbs::R_ROT, 8)))
             return fail(QFB_ENOSYS, "compact sector: forward step outside the pair-list limits");
     for (const auto &it : sp.sweep_items)
-        if (!push_pairs(W, sp, it.unrot ? sp.usteps[it.step] : sp.ksteps[it.step], it.flags, it.row, S))
+        if (!push_rounds(W, sp, it.unrot ? sp.usteps[it.step] : sp.ksteps[it.step], it.flags, 8))
             return fail(QFB_ENOSYS, "compact sector: sweep step outside the pair-list limits");
     auto d = std::make_shared<PairPlanDev>();
-    const size_t bf = pair_bytes(F), bw = pair_bytes(W);
-    int rc = dev_alloc(&d->blob, bf + bw);
+    std::vector<uint32_t> wf, wf2, ww;
+    std::vector<int2> none, range;
+    lay_rounds(F, round_threads(F), sp.nsec, 0, d->fwd, wf, none);
+    lay_rounds(F2, round_threads(F2), sp.nsec, 0, d->fwd2, wf2, none);
+    lay_rounds(W, round_threads(W), sp.nsec, nparam, d->sweep, ww, range);
+    struct Up {
+        const void *p;
+        size_t n, o;
+    } ups[] = {{F.hd.data(), sizeof(qfbs::RRec) * F.hd.size(), 0},
+               {F2.hd.data(), sizeof(qfbs::RRec) * F2.hd.size(), 0},
+               {W.hd.data(), sizeof(qfbs::RRec) * W.hd.size(), 0},
+               {wf.data(), sizeof(uint32_t) * wf.size(), 0},
+               {wf2.data(), sizeof(uint32_t) * wf2.size(), 0},
+               {ww.data(), sizeof(uint32_t) * ww.size(), 0},
+               {range.data(), sizeof(int2) * range.size(), 0}};
+    size_t off = 0;
+    for (Up &x : ups) {
+        x.o = off;
+        off += (std::max<size_t>(x.n, 16) + 255) & ~(size_t)255;
+    }
+    const int rc = dev_alloc(&d->blob, off);
     if (rc) return rc;
-    d->bytes = bf + bw;
-    rc = pair_upload(F, (char *)d->blob, d->fwd);
-    if (!rc) rc = pair_upload(W, (char *)d->blob + bf, d->sweep);
-    if (!rc) QFB_CUDA(cudaStreamSynchronize(t_stream));
-    if (rc) return rc;
-    d->fwd_hd = F.hd;
+    d->bytes = off;
+    char *base = (char *)d->blob;
+    for (const Up &x : ups)
+        if (x.n) QFB_CUDA(cudaMemcpyAsync(base + x.o, x.p, x.n, cudaMemcpyHostToDevice, t_stream));
+    QFB_CUDA(cudaStreamSynchronize(t_stream));
+    qfbs::RStream *st[] = {&d->fwd, &d->fwd2, &d->sweep};
+    for (int k = 0; k < 3; ++k) {
+        st[k]->hd = (const qfbs::RRec *)(base + ups[k].o);
+        st[k]->word = (const uint32_t *)(base + ups[3 + k].o) + 4 * st[k]->nth;
+    }
+    d->prange = (const int2 *)(base + ups[6].o);
     slot = d;
     *out = d;
     return QFB_OK;
@@ -3057,13 +3185,11 @@ struct qfb_ucc_s {
     double *res = nullptr;            // [B][nres]
     const int64_t *ridx = nullptr;    // full-space index, or compact index (-1: outside)
     const double2 *rphase = nullptr;  // [nres]
-    qfbs::PStream rstream{};          // compact: forward pair lists in reverse order
-    std::shared_ptr<PairPlanDev> pairs;  // compact: the plan's pair lists in use
-    int64_t nprows = 1;                  // rows of the gradient partials (gradient steps)
+    std::shared_ptr<PairPlanDev> pairs;  // compact: the plan's rounds in use
+    void *sblob = nullptr;               // compact: the sweep's warp sums
     // compact, real states: two parameter sets per CTA in the forward kernel
     // (k_sector_forward_pr), with pair lists ordered for 16-byte slots
     int paired = 0;
-    std::shared_ptr<PairPlanDev> pairs16b;
     qfbs::SLaunch SLp{};
 };
 
@@ -3505,6 +3631,13 @@ static int win_smem_attr() {
     return err == cudaSuccess ? QFB_OK : cuda_fail(err, "window shared memory");
 }
 
+// Shared memory of the sweep (and of a packed item): both states and the constants.
+static size_t compact_smem(int real, int nsec, int nfwd, int nsweep) {
+    const int n = std::max(nfwd, nsweep);
+    return real ? qfbs::step_smem<qfbs::PCoef<true, double>>(2, nsec, sizeof(double), n)
+                : qfbs::step_smem<qfbs::PCoef<true, double2>>(2, nsec, sizeof(double2), n);
+}
+
 // Attach a compact plan and its H rows to an evaluator (shared memory or,
 // with `global`, global memory states).
 static int sector_attach(qfb_ucc u, qfb_sum_s *ham, const std::shared_ptr<SectorPlan> &plan,
@@ -3531,19 +3664,15 @@ static int sector_attach(qfb_ucc u, qfb_sum_s *ham, const std::shared_ptr<Sector
     if (!global) {
         if (u->sreal != ((real_steps && rows->vc == nullptr) ? 1 : 0))
             return fail(QFB_EINVAL, "compact sector: H rows' type differs from their groups'");
-        rc = pair_plan(sp, u->sreal ? 16 : 8, &pairs);
+        rc = pair_plan(sp, u->sreal != 0, u->nparam, &pairs);
         if (rc) return rc;
         u->pairs = pairs;
         u->bytes += pairs->bytes;
+        if (compact_smem(u->sreal, sp.nsec, pairs->fwd.n, pairs->sweep.n) > kStepSmemMax)
+            return fail(QFB_EINVAL, "compact sector: %d records outgrow shared memory", pairs->sweep.n);
         // two real sets per CTA in the forward program where its shared memory fits
-        const size_t fwd_b = ((16 * (size_t)sp.nsec + 15) & ~(size_t)15) +
-                             sizeof(qfbs::PSmemPR) * (size_t)pairs->fwd.n;
-        if (u->sreal && g_ucc_compact != 6 && u->nbatch >= 2 && fwd_b <= kSectorSmemMax) {
-            rc = pair_plan(sp, 8, &u->pairs16b);
-            if (rc) return rc;
-            if (u->pairs16b != pairs) u->bytes += u->pairs16b->bytes;
-            u->paired = 1;
-        }
+        u->paired = u->sreal && g_ucc_compact != 6 && u->nbatch >= 2 &&
+                    qfbs::step_smem<qfbs::PCoefPR>(1, sp.nsec, sizeof(double2), pairs->fwd2.n) <= kSectorSmemMax;
     }
     u->splan = plan;
     u->rows = rows;
@@ -3586,6 +3715,10 @@ static int sector_attach(qfb_ucc u, qfb_sum_s *ham, const std::shared_ptr<Sector
         u->g_vc = rows->vc;
         return QFB_OK;
     }
+    const size_t sums = sizeof(double) * (size_t)u->nbatch * pairs->sweep.nr * (pairs->sweep.nth / 32);
+    rc = dev_alloc(&u->sblob, std::max<size_t>(sums, 16));
+    if (rc) return rc;
+    u->bytes += sums;
     qfbs::SLaunch &L = u->SL;
     L.nsec = sp.nsec;
     L.nbeta = sp.nbeta;
@@ -3599,49 +3732,40 @@ static int sector_attach(qfb_ucc u, qfb_sum_s *ham, const std::shared_ptr<Sector
     L.val_c = rows->vc;
     L.params = u->params;
     L.energy = u->energy;
-    L.partial = u->gpart;
+    L.partial = (double *)u->sblob;
+    L.grad = u->gradv;
+    L.prange = pairs->prange;
     if (u->paired) {
         u->SLp = L;
-        u->SLp.fwd = u->pairs16b->fwd;
+        u->SLp.fwd = pairs->fwd2;
     }
     return QFB_OK;
 }
 
 template <class V>
 static cudaError_t sector_smem_attr_v() {
-    const int m = (int)kSectorSmemMax;
-    cudaError_t err = cudaFuncSetAttribute(qfbs::k_sector_forward<V>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, m);
-    auto attr = [&](const void *f) {
-        if (err == cudaSuccess) err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, m);
+    cudaError_t err = cudaSuccess;
+    auto attr = [&](const void *f, size_t m) {
+        if (err == cudaSuccess) err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m);
     };
     if constexpr (sizeof(V) == sizeof(double)) {
-        attr((const void *)qfbs::k_sector_h<true, V, 4, 1024>);
-        attr((const void *)qfbs::k_sector_h<true, V, 2, 512>);
-        attr((const void *)qfbs::k_sector_h<true, V, 1, 512>);
+        attr((const void *)qfbs::k_sector_h<true, V, 4, 1024>, kSectorSmemMax);
+        attr((const void *)qfbs::k_sector_h<true, V, 2, 512>, kSectorSmemMax);
+        attr((const void *)qfbs::k_sector_h<true, V, 1, 512>, kSectorSmemMax);
+        attr((const void *)qfbs::k_sector_forward_pr, kStepSmemMax);
     } else {
-        attr((const void *)qfbs::k_sector_h<true, V, 2, 1024>);
-        attr((const void *)qfbs::k_sector_h<true, V, 1, 512>);
-        attr((const void *)qfbs::k_sector_h<false, V, 2, 1024>);
-        attr((const void *)qfbs::k_sector_h<false, V, 1, 512>);
+        attr((const void *)qfbs::k_sector_h<true, V, 2, 1024>, kSectorSmemMax);
+        attr((const void *)qfbs::k_sector_h<true, V, 1, 512>, kSectorSmemMax);
+        attr((const void *)qfbs::k_sector_h<false, V, 2, 1024>, kSectorSmemMax);
+        attr((const void *)qfbs::k_sector_h<false, V, 1, 512>, kSectorSmemMax);
     }
-    if (err == cudaSuccess)
-        err = cudaFuncSetAttribute(qfbs::k_sector_sweep<V>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, m);
-    if (err == cudaSuccess)
-        err = cudaFuncSetAttribute(qfbs::k_sector_resid<V>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, m);
-    if (err == cudaSuccess)
-        err = cudaFuncSetAttribute(qfbs::k_sector_pool<V>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, m);
-    if (err == cudaSuccess)
-        err = cudaFuncSetAttribute(qfbs::k_sector_pack<V>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, m);
-    if constexpr (sizeof(V) == sizeof(double)) {
-        if (err == cudaSuccess)
-            err = cudaFuncSetAttribute(qfbs::k_sector_forward_pr,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, m);
-    }
+    attr((const void *)qfbs::k_sector_forward<V>, kStepSmemMax);
+    attr((const void *)qfbs::k_sector_sweep<V>, kStepSmemMax);
+    attr((const void *)qfbs::k_sector_resid<V>, kStepSmemMax);
+    attr((const void *)qfbs::k_sector_pool<V>, kSectorSmemMax);
+    attr((const void *)qfbs::k_pack_forward<V>, kStepSmemMax);
+    attr((const void *)qfbs::k_pack_h<V>, kSectorSmemMax);
+    attr((const void *)qfbs::k_pack_sweep<V>, kStepSmemMax);
     return err;
 }
 
@@ -3663,19 +3787,20 @@ static int ucc_stage_compact_v(qfb_ucc u, int stage, int with_grad) {
     switch (stage) {
         case 1:
             if constexpr (sizeof(V) == sizeof(double)) {
-                if (u->paired) {
+                // pairs of sets where single ones would queue (us, single / paired: 16
+                // qubits, 160 sets 106 / 94, 512 sets 213 / 187; 14 qubits 23 / 24
+                // and 41 / 34; 12 qubits 11.6 / 13.1 and 20.4 / 18.1)
+                if (u->paired && u->nbatch > sm_count() * (u->SLp.fwd.nth >= 256 ? 1 : 2)) {
                     const qfbs::SLaunch &LP = u->SLp;
-                    qfbs::k_sector_forward_pr<<<(u->nbatch + 1) / 2, qfbs::kStepThreads,
-                                                ((16 * n + 15) & ~(size_t)15) +
-                                                    sizeof(qfbs::PSmemPR) * (size_t)LP.fwd.n,
+                    qfbs::k_sector_forward_pr<<<(u->nbatch + 1) / 2, LP.fwd.nth,
+                                                qfbs::step_smem<qfbs::PCoefPR>(1, L.nsec, sizeof(double2), LP.fwd.n),
                                                 t_stream>>>(LP, u->nbatch);
                     QFB_LAUNCHED();
                     break;
                 }
             }
-            qfbs::k_sector_forward<V><<<u->nbatch, qfbs::kStepThreads,
-                                        qfbs::sector_smem_states(1, n, real) +
-                                            sizeof(qfbs::PSmem<V>) * (size_t)L.fwd.n,
+            qfbs::k_sector_forward<V><<<u->nbatch, L.fwd.nth,
+                                        qfbs::step_smem<qfbs::PCoef<false, V>>(1, L.nsec, sizeof(V), L.fwd.n),
                                         t_stream>>>(L);
             QFB_LAUNCHED();
             break;
@@ -3702,16 +3827,9 @@ static int ucc_stage_compact_v(qfb_ucc u, int stage, int with_grad) {
         }
         case 3:
             if (!(with_grad && u->grad && u->nparam > 0)) break;
-            qfbs::k_sector_sweep<V><<<u->nbatch, qfbs::kSweepThreads,
-                                      qfbs::sector_smem_states(2, n, real) +
-                                          sizeof(qfbs::PSmem<V>) * (size_t)L.sweep.n,
+            qfbs::k_sector_sweep<V><<<u->nbatch, L.sweep.nth,
+                                      qfbs::step_smem<qfbs::PCoef<true, V>>(2, L.nsec, sizeof(V), L.sweep.n),
                                       t_stream>>>(L);
-            QFB_LAUNCHED();
-            {
-                const int64_t n = (int64_t)u->nparam * u->nbatch;
-                k_grad_final_few<<<(unsigned)((n + 255) / 256), 256, 0, t_stream>>>(
-                    u->gpart, u->psteps, (int)u->gchunks, u->nparam, u->nbatch, u->gradv);
-            }
             QFB_LAUNCHED();
             break;
         default:
@@ -3996,15 +4114,14 @@ static int ucc_pool_stage(qfb_ucc u) {
                                                                     u->pstream.span, u->ppart);
         QFB_LAUNCHED();
     } else if (u->compact) {
-        qfbs::SLaunch L = u->SL;
-        L.partial = u->ppart;
+        const qfbs::SLaunch &L = u->SL;
         const int sm = sm_count();
         const int G = std::max(1, std::min(u->ppairs.n, (2 * sm + B - 1) / B));
         const size_t smem = qfbs::sector_smem_states(2, (size_t)L.nsec, u->sreal);
         if (u->sreal)
-            qfbs::k_sector_pool<double><<<dim3(G, B), kSectorThreads, smem, t_stream>>>(L, u->ppairs);
+            qfbs::k_sector_pool<double><<<dim3(G, B), kSectorThreads, smem, t_stream>>>(L, u->ppairs, u->ppart);
         else
-            qfbs::k_sector_pool<double2><<<dim3(G, B), kSectorThreads, smem, t_stream>>>(L, u->ppairs);
+            qfbs::k_sector_pool<double2><<<dim3(G, B), kSectorThreads, smem, t_stream>>>(L, u->ppairs, u->ppart);
         QFB_LAUNCHED();
         chunks = kSectorThreads / 32;
     } else {
@@ -4030,15 +4147,14 @@ static int ucc_resid_stage(qfb_ucc u) {
     const unsigned gg = (unsigned)(((int64_t)u->nres * B + 255) / 256);
     if (u->compact) {
         const qfbs::SLaunch &L = u->SL;
-        const size_t smem = qfbs::sector_smem_states(1, (size_t)L.nsec, u->sreal) +
-                            (u->sreal ? sizeof(qfbs::PSmem<double>) : sizeof(qfbs::PSmem<double2>)) *
-                                (size_t)u->rstream.n;
         if (u->sreal)
-            qfbs::k_sector_resid<double><<<B, qfbs::kStepThreads, smem, t_stream>>>(
-                L, u->rstream, u->ridx, u->rphase, u->nres, u->res);
+            qfbs::k_sector_resid<double><<<B, L.fwd.nth,
+                                           qfbs::step_smem<qfbs::PCoef<false, double>>(1, L.nsec, 8, L.fwd.n),
+                                           t_stream>>>(L, u->ridx, u->rphase, u->nres, u->res);
         else
-            qfbs::k_sector_resid<double2><<<B, qfbs::kStepThreads, smem, t_stream>>>(
-                L, u->rstream, u->ridx, u->rphase, u->nres, u->res);
+            qfbs::k_sector_resid<double2><<<B, L.fwd.nth,
+                                            qfbs::step_smem<qfbs::PCoef<false, double2>>(1, L.nsec, 16, L.fwd.n),
+                                            t_stream>>>(L, u->ridx, u->rphase, u->nres, u->res);
         QFB_LAUNCHED();
         return QFB_OK;
     }
@@ -4192,8 +4308,7 @@ static int ucc_create_impl(qfb_prog fprog, qfb_prog gprog, qfb_prog uprog, qfb_s
     u->ref = ref_index;
     u->vchunks = grid_for(u->nbasis, 256, 2);
     if (u->vchunks * (unsigned)nbatch > 65535u) u->vchunks = std::max(1u, 65535u / nbatch);
-    u->gchunks = compact ? qfbs::kSweepThreads / 32
-                         : gsec ? 1 : (gprog ? grad_chunks(gprog, nqubit, nbatch) : 1);
+    u->gchunks = compact || gsec ? 1 : (gprog ? grad_chunks(gprog, nqubit, nbatch) : 1);
     const size_t B = nbatch, M = std::max(u->nparam, 1);
     const size_t nsteps = gprog ? std::max<size_t>(gprog->h_steps.size(), 1) : 1;
     const size_t b_state = (compact || gsec) ? 16 : sizeof(double2) * u->nbasis * B;
@@ -4207,7 +4322,7 @@ static int ucc_create_impl(qfb_prog fprog, qfb_prog gprog, qfb_prog uprog, qfb_s
     const size_t o_par = take(sizeof(double) * B * M), o_en = take(sizeof(double) * B);
     const size_t o_gr = take(sizeof(double) * B * M);
     const size_t o_vp = take(sizeof(double2) * B * u->vchunks);
-    const size_t o_gp = take(gprog && !gsec ? sizeof(double2) * nsteps * B * u->gchunks : 16);
+    const size_t o_gp = take(gprog && !gsec && !compact ? sizeof(double2) * nsteps * B * u->gchunks : 16);
     const size_t o_ps = take(sizeof(int2) * M);
     const size_t idx_bytes = nqubit <= 32 ? sizeof(uint32_t) : sizeof(uint64_t);
     const size_t o_sec = take(idx_bytes * std::max<size_t>(sector.size(), 1));
@@ -4236,7 +4351,6 @@ static int ucc_create_impl(qfb_prog fprog, qfb_prog gprog, qfb_prog uprog, qfb_s
     u->vpart = (double2 *)(base + o_vp);
     u->gpart = (double2 *)(base + o_gp);
     u->psteps = (int2 *)(base + o_ps);
-    u->nprows = (int64_t)nsteps;
     u->nsec = compact ? (int64_t)splan.nsec : (int64_t)sector.size();
     u->SL.save = (double2 *)(base + o_save);
     u->h_epart = (double *)(base + o_hep);
@@ -4354,6 +4468,7 @@ int qfb_ucc_destroy(qfb_ucc u) {
     if (u->hfork) cudaEventDestroy(u->hfork);
     dev_free(u->hblob);
     dev_free(u->wblob);
+    dev_free(u->sblob);
     dev_free(u->blob);
     delete u;
     return QFB_OK;
@@ -4479,14 +4594,10 @@ int qfb_ucc_set_residuals(qfb_ucc u, const uint64_t *dets, const qfb_complex *ph
             idx[k] = (int64_t)dets[k];
         }
     }
-    // compact, shared memory: the forward pair-list headers in reverse order
-    std::vector<qfbs::PHead> rhd;
-    if (u->compact) rhd.assign(u->pairs->fwd_hd.rbegin(), u->pairs->fwd_hd.rend());
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const int B = u->nbatch;
     const size_t o_res = 0, o_idx = al(sizeof(double) * (size_t)B * n),
-                 o_ph = o_idx + al(sizeof(int64_t) * n), o_sp = o_ph + al(sizeof(double2) * n),
-                 total = o_sp + sizeof(qfbs::PHead) * std::max<size_t>(1, rhd.size());
+                 o_ph = o_idx + al(sizeof(int64_t) * n), total = o_ph + sizeof(double2) * n;
     void *blob = nullptr;
     int rc = dev_alloc(&blob, total);
     if (rc) return rc;
@@ -4497,9 +4608,6 @@ int qfb_ucc_set_residuals(qfb_ucc u, const uint64_t *dets, const qfb_complex *ph
                              t_stream));
     QFB_CUDA(cudaMemcpyAsync(bp + o_ph, ph.data(), sizeof(double2) * n, cudaMemcpyHostToDevice,
                              t_stream));
-    if (!rhd.empty())
-        QFB_CUDA(cudaMemcpyAsync(bp + o_sp, rhd.data(), sizeof(qfbs::PHead) * rhd.size(),
-                                 cudaMemcpyHostToDevice, t_stream));
     QFB_CUDA(cudaMemsetAsync(bp + o_res, 0, sizeof(double) * (size_t)B * n, t_stream));
     if (u->exec[4]) {  // a captured residual run refers to the old buffers
         cudaGraphExecDestroy(u->exec[4]);
@@ -4516,10 +4624,6 @@ int qfb_ucc_set_residuals(qfb_ucc u, const uint64_t *dets, const qfb_complex *ph
     u->res = (double *)(bp + o_res);
     u->ridx = (const int64_t *)(bp + o_idx);
     u->rphase = (const double2 *)(bp + o_ph);
-    if (u->compact) {
-        u->rstream = u->SL.fwd;
-        u->rstream.hd = (const qfbs::PHead *)(bp + o_sp);
-    }
     return QFB_OK;
 }
 
@@ -4683,14 +4787,23 @@ int qfb_ucc_profile(qfb_ucc u, int with_grad, int reps, double *stage_ms,
 // ===========================================================================
 
 struct qfb_pack_s {
-    int nmem = 0, cap = 0, maxparam = 1, max_rows = 1, sreal = 0;
-    size_t smem = 0, bytes = 0;
+    int nmem = 0, cap = 0, sreal = 1, maxparam = 1, maxsec = 1;
+    int nth = 32;       // threads of an item's block
+    size_t smem = 0;    // psi, sigma and the constants of the largest member
+    size_t smem_h = 0;  // psi alone
+    int chunk = 1;      // items a group of launches takes
+    size_t bytes = 0, maxpart = 0;
     void *blob = nullptr;
     qfbs::PackMember *d_mem = nullptr;
     int2 *items = nullptr;
     double *params = nullptr, *energy = nullptr, *grad = nullptr;
-    double2 *partial = nullptr;
+    double *partial = nullptr, *epart = nullptr;
+    void *save = nullptr;
+    unsigned *count = nullptr;
 };
+
+constexpr int kPackSlices = 16;   // CTAs an item's H rows are split over, at most
+constexpr int kPackChunk = 1024;  // items a group of launches takes (its workspace holds as many)
 
 extern "C" int qfb_pack_create(const qfb_ucc *members, int nmembers, int capacity, qfb_pack *out) {
     if (!out) return fail(QFB_EINVAL, "qfb_pack_create: null output");
@@ -4716,15 +4829,13 @@ extern "C" int qfb_pack_create(const qfb_ucc *members, int nmembers, int capacit
         if (u->sreal != p->sreal)
             return fail(QFB_EINVAL, "qfb_pack_create: members mix real and complex state storage");
         const qfbs::SLaunch &L = u->SL;
-        const size_t es = u->sreal ? sizeof(qfbs::PSmem<double>) : sizeof(qfbs::PSmem<double2>);
-        const size_t need = qfbs::sector_smem_states(2, (size_t)L.nsec, u->sreal) +
-                            es * (size_t)std::max(L.fwd.n, L.sweep.n);
-        if (need > kSectorSmemMax)
-            return fail(QFB_EINVAL, "qfb_pack_create: member %d needs %zu bytes of shared memory",
-                        k, need);
+        const size_t need = compact_smem(u->sreal, L.nsec, L.fwd.n, L.sweep.n);
         p->smem = std::max(p->smem, need);
+        p->smem_h = std::max(p->smem_h, qfbs::sector_smem_states(1, (size_t)L.nsec, u->sreal));
+        p->nth = std::max({p->nth, L.fwd.nth, L.sweep.nth});
+        p->maxsec = std::max(p->maxsec, L.nsec);
         p->maxparam = std::max(p->maxparam, u->nparam);
-        p->max_rows = std::max(p->max_rows, (int)u->nprows);
+        p->maxpart = std::max(p->maxpart, (size_t)L.sweep.nr * (L.sweep.nth / 32));
         qfbs::PackMember &m = hm[(size_t)k];
         m.nsec = L.nsec;
         m.ref_i = L.ref_i;
@@ -4736,10 +4847,11 @@ extern "C" int qfb_pack_create(const qfb_ucc *members, int nmembers, int capacit
         m.col = L.col;
         m.val_r = L.val_r;
         m.val_c = L.val_c;
-        m.psteps = u->psteps;
+        m.prange = L.prange;
     }
     const size_t C = (size_t)capacity, MP = (size_t)p->maxparam;
-    const size_t nw = qfbs::kPackThreads / 32;
+    p->chunk = std::min(capacity, kPackChunk);
+    const size_t NS = (size_t)p->chunk;
     size_t off = 0;
     auto take = [&](size_t bytes) {
         const size_t o = off;
@@ -4749,7 +4861,9 @@ extern "C" int qfb_pack_create(const qfb_ucc *members, int nmembers, int capacit
     const size_t o_mem = take(sizeof(qfbs::PackMember) * (size_t)nmembers);
     const size_t o_it = take(sizeof(int2) * C), o_par = take(sizeof(double) * C * MP);
     const size_t o_en = take(sizeof(double) * C), o_gr = take(sizeof(double) * C * MP);
-    const size_t o_pt = take(sizeof(double2) * C * (size_t)p->max_rows * nw);
+    const size_t o_pt = take(sizeof(double) * NS * p->maxpart);
+    const size_t o_sv = take((p->sreal ? 8 : 16) * NS * 2 * (size_t)p->maxsec);
+    const size_t o_ep = take(sizeof(double) * NS * kPackSlices), o_ct = take(sizeof(unsigned) * NS);
     rc = dev_alloc(&p->blob, off);
     if (rc) return rc;
     p->bytes = off;
@@ -4759,7 +4873,10 @@ extern "C" int qfb_pack_create(const qfb_ucc *members, int nmembers, int capacit
     p->params = (double *)(base + o_par);
     p->energy = (double *)(base + o_en);
     p->grad = (double *)(base + o_gr);
-    p->partial = (double2 *)(base + o_pt);
+    p->partial = (double *)(base + o_pt);
+    p->save = base + o_sv;
+    p->epart = (double *)(base + o_ep);
+    p->count = (unsigned *)(base + o_ct);
     cudaError_t e = cudaMemsetAsync(p->blob, 0, off, t_stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(p->d_mem, hm.data(), sizeof(qfbs::PackMember) * hm.size(),
@@ -4798,20 +4915,32 @@ extern "C" int qfb_pack_buffers(qfb_pack p, int32_t **items, double **params, do
     return QFB_OK;
 }
 
+template <class V>
+static int pack_group(qfb_pack p, const qfbs::PackLaunch &L, int nitems) {
+    qfbs::k_pack_forward<V><<<nitems, p->nth, p->smem, t_stream>>>(L);
+    QFB_LAUNCHED();
+    qfbs::k_pack_h<V><<<dim3(L.Q, nitems), qfbs::kStepThreads, p->smem_h, t_stream>>>(L);
+    QFB_LAUNCHED();
+    qfbs::k_pack_sweep<V><<<nitems, p->nth, p->smem, t_stream>>>(L);
+    QFB_LAUNCHED();
+    return QFB_OK;
+}
+
 extern "C" int qfb_pack_launch(qfb_pack p, int nitems) {
     if (!p) return fail(QFB_EINVAL, "qfb_pack_launch: null pack");
     if (nitems < 0 || nitems > p->cap)
         return fail(QFB_EINVAL, "qfb_pack_launch: %d items for a capacity of %d", nitems, p->cap);
-    if (nitems == 0) return QFB_OK;
-    if (p->sreal)
-        qfbs::k_sector_pack<double><<<nitems, qfbs::kPackThreads, p->smem, t_stream>>>(
-            p->d_mem, p->items, p->maxparam, p->params, p->energy, p->grad, p->partial, p->max_rows,
-            p->nmem);
-    else
-        qfbs::k_sector_pack<double2><<<nitems, qfbs::kPackThreads, p->smem, t_stream>>>(
-            p->d_mem, p->items, p->maxparam, p->params, p->energy, p->grad, p->partial, p->max_rows,
-            p->nmem);
-    QFB_LAUNCHED();
+    for (int i0 = 0; i0 < nitems; i0 += p->chunk) {
+        const int n = std::min(p->chunk, nitems - i0);
+        const size_t at = (size_t)i0 * p->maxparam;
+        // about four CTAs an SM for the H rows
+        const int Q = std::max(1, std::min(kPackSlices, 4 * sm_count() / n));
+        const qfbs::PackLaunch L{p->d_mem, p->items + i0, p->nmem, p->maxparam, p->params + at,
+                                 p->energy + i0, p->grad + at, p->partial, p->maxpart, p->save, p->maxsec, Q,
+                                 p->epart, p->count};
+        const int rc = p->sreal ? pack_group<double>(p, L, n) : pack_group<double2>(p, L, n);
+        if (rc) return rc;
+    }
     return QFB_OK;
 }
 

@@ -28,10 +28,15 @@
 // sigma(j0) = (-1)^popcount(j0 & zbase).  The global-memory path
 // (qfb_csec.cuh) reads those lists (records of RHead / RPat / SEntry); the
 // shared-memory kernels here read the product expanded on the host into one
-// word pair per amplitude pair (PHead / PStream), ordered so that each half
-// warp (quarter warp for complex amplitudes) touches distinct banks.  The
-// arithmetic on each pair is that of the full-space kernels (givens_pair and
-// the gradient inner product).
+// word per amplitude pair, laid out in rounds of a block's threads (RStream)
+// and ordered so that each half warp (quarter warp for 16-byte words) touches
+// distinct banks.  The pool kernel reads pair lists (PHead / PStream).
+//
+// Forward and sweep are bound by one round after another, so the rounds are
+// what was made short.  us, before (a record at a time, tests and look-ups
+// between its barriers) / now: one set, 12 qubits (117 steps) forward 35 / 9.5,
+// sweep 54 / 15; 16 qubits (360 steps) 128 / 56 and 227 / 116; 256 sets of 16
+// qubits 157 / 95 and 320 / 215.
 #pragma once
 
 #include <cstdint>
@@ -67,11 +72,11 @@ struct SStream {          // one kernel's records
     int maxw;             // longest record (words)
 };
 
-// A step record on the pair list, used by the shared-memory kernels: the
-// pairs of the step's patterns as explicit sector index pairs, ordered on the
-// host so that the lanes of a warp reach distinct shared-memory banks, and the
-// step's constants.  A stream's headers, pairs and pattern coefficients are
-// three arrays.
+// A step record on the pair list, used by the pool kernel: the pairs of the
+// step's patterns as explicit sector index pairs, ordered on the host so that
+// the lanes of a warp reach distinct shared-memory banks, and the step's
+// constants.  A stream's headers, pairs and pattern coefficients are three
+// arrays.
 struct PHead {
     int32_t p0;     // first pair
     int32_t np;     // pairs
@@ -86,9 +91,7 @@ static_assert(sizeof(PHead) == 32, "PHead is two 16-byte words");
 // A pair word: i0 (bits 0-13) | i1 << 14 | neg << 28 | pattern << 29 (a
 // Givens-form step has at most 8 active patterns).
 constexpr int kPairIdxBits = 14;  // sector indices below 16384
-constexpr int kSweepRing = 2;     // register sets of pair words in the sweep (2 or 4)
-constexpr int kStepThreads = 512;   // block of the forward and residual kernels
-constexpr int kSweepThreads = 256;  // block of the sweep (more pairs per thread per record)
+constexpr int kStepThreads = 512;  // block of the step kernels, at most
 constexpr int kPairPatterns = 8;
 struct PStream {
     const PHead *hd;
@@ -97,16 +100,41 @@ struct PStream {
     int n;
 };
 
+// A stream as the step kernels run it: rounds of nth pairs, one pair a thread,
+// a barrier after each.  A record takes as many rounds as its pairs need; the
+// lanes left over rotate amplitudes past the sector's end (kRoundPad of them,
+// zero), so no thread tests anything.  A word holds both indices as byte
+// offsets of 8-byte amplitudes: last round of its record (bit 0), first round
+// (bit 1), i0 (bits 3-16), i1 (bits 17-30), neg (bit 31).  The number of rounds
+// is a multiple of 4 (the last ones are an empty record's), with 4 unused
+// rounds of words on either side.
+struct RRec {
+    double gamma;
+    int32_t param;
+    int32_t fl;  // R_ROT | R_IP
+    double2 gn, hn;
+};
+static_assert(sizeof(RRec) == 48, "RRec layout");
+constexpr int kRoundPad = 32;
+constexpr uint32_t kWordIdx = ((1u << kPairIdxBits) - 1u) << 3;
+struct RStream {
+    const RRec *hd;
+    const uint32_t *word;
+    int n, nr, nth, pad;
+};
+
 struct SLaunch {
     int nsec, nbeta, ref_i, nparam;
-    PStream fwd, sweep;
+    RStream fwd, sweep;
     const int32_t *rowptr;     // H rows
     const uint32_t *col;
     const double *val_r;       // real H (val_c == nullptr) ...
     const double2 *val_c;      // ... or complex
     const double *params;      // [B][nparam]
     double *energy;            // [B]
-    double2 *partial;          // [K steps][B][warps]
+    double *grad;              // [B][nparam]
+    const int2 *prange;        // rounds of the sweep of each parameter's inner products
+    double *partial;           // [B][sweep rounds / 4][warps][4]
     void *save;                // V [B][2][nsec]: psi after the forward program, sigma
 };
 
@@ -158,15 +186,6 @@ __device__ __forceinline__ double2 v_shfl_down(double2 v, int o) {
     return make_double2(__shfl_down_sync(0xffffffffu, v.x, o), __shfl_down_sync(0xffffffffu, v.y, o));
 }
 
-// new0 = c v0 + s hn v1, new1 = c v1 + s gn v0 (as givens_pair)
-template <class V, class K>
-__device__ __forceinline__ void s_givens(V &v0, V &v1, double c, double s, K gn, K hn) {
-    const V a = v_mul(hn, v1), b = v_mul(gn, v0);
-    const V n0 = v_lin(c, v0, s, a);
-    v1 = v_lin(c, v1, s, b);
-    v0 = n0;
-}
-
 // A pair's share of <w|K|v>: conj(w0) hn v1 + conj(w1) gn v0
 __device__ __forceinline__ double v_ip(double w0, double w1, double v0, double v1, double gn,
                                        double hn) {
@@ -193,57 +212,6 @@ __device__ __forceinline__ PHead p_head(const PHead *p) {
     return h;
 }
 
-// Pair words of a record held per thread: three for real amplitudes, two
-// for complex ones (whose pairs need twice the registers).
-template <class V>
-__host__ __device__ constexpr int pair_slots() {
-    return sizeof(V) == sizeof(double) ? 3 : 2;
-}
-
-// Words past a stream's last pair (zeros), so that the prefetch below loads
-// without a bound check (a selected value would wait for its load at once).
-constexpr int kPairPad = 4 * 1024;
-
-// This thread's first KP pair words of record h (pairs tid, tid + nth, ...);
-// words past the record are loaded but never used (p_record checks np).
-template <int KP>
-__device__ __forceinline__ void p_words(const PStream &S, const PHead &h, uint32_t (&pw)[KP]) {
-#pragma unroll
-    for (int j = 0; j < KP; ++j) pw[j] = __ldg(S.pair + h.p0 + threadIdx.x + j * blockDim.x);
-}
-
-
-// One pair: the share of <w|K|v> into acc and / or the rotation of v (and w
-// when TWO) by the angle whose cos / sin is (c, s).
-template <bool ROT, bool IP, bool TWO, class V>
-__device__ __forceinline__ void p_pair(uint32_t pw, double c, double s, double gamma, V gn, V hn, V *v,
-                                       V *w, V &acc) {
-    constexpr uint32_t M = (1u << kPairIdxBits) - 1u;
-    const int i0 = (int)(pw & M), i1 = (int)((pw >> kPairIdxBits) & M);
-    const bool neg = (pw >> (2 * kPairIdxBits)) & 1u;
-    V v0 = v[i0], v1 = v[i1];
-    V w0 = v_zero(V()), w1 = w0;
-    if (IP || TWO) {
-        w0 = w[i0];
-        w1 = w[i1];
-    }
-    if (IP) v_acc(acc, neg ? -gamma : gamma, v_ip(w0, w1, v0, v1, gn, hn));
-    if (ROT) {
-        const double ss = neg ? -s : s;
-        s_givens(v0, v1, c, ss, gn, hn);
-        v[i0] = v0;
-        v[i1] = v1;
-        if (TWO) {
-            s_givens(w0, w1, c, ss, gn, hn);
-            w[i0] = w0;
-            w[i1] = w1;
-        }
-    }
-}
-
-// One record on the compact states: this thread's pairs (the prefetched
-// words first, then any beyond KP per thread).  The pairs of one record touch
-// distinct amplitudes, so threads need no ordering within it.
 // The coefficients (gn, hn) of pattern k of a stream: real parts only for
 // real amplitudes.
 __device__ __forceinline__ void p_ldcoef(const PStream &S, int k, double &gn, double &hn) {
@@ -255,56 +223,76 @@ __device__ __forceinline__ void p_ldcoef(const PStream &S, int k, double2 &gn, d
     hn = __ldg(S.coef + 2 * k + 1);
 }
 
-// gn, hn: the coefficients of a single-pattern record (p_coef); records of
-// several patterns load each pair's from its pattern number.
-template <bool ROT, bool IP, bool TWO, class V, int KP>
-__device__ __forceinline__ void p_record(const PStream &S, const PHead &h, const uint32_t (&pw)[KP],
-                                         double2 csn, V gn, V hn, V *v, V *w, V &acc) {
-    const int tid = threadIdx.x, nth = blockDim.x;
-    const bool one = (h.fl >> 8) == 1;
-    auto run = [&](uint32_t p) {
-        if (!one) p_ldcoef(S, h.c0 + (int)(p >> (2 * kPairIdxBits + 1)), gn, hn);
-        p_pair<ROT, IP, TWO, V>(p, csn.x, csn.y, h.gamma, gn, hn, v, w, acc);
-    };
-#pragma unroll
-    for (int j = 0; j < KP; ++j)
-        if (tid + j * nth < h.np) run(pw[j]);
-    for (int k = tid + KP * nth; k < h.np; k += nth) run(__ldg(S.pair + h.p0 + k));
+// Re of conj(w0) h v1 + conj(w1) g v0
+__device__ __forceinline__ double v_ip_re(double w0, double w1, double v0, double v1, double g, double h) {
+    return w0 * (h * v1) + w1 * (g * v0);
+}
+__device__ __forceinline__ double v_ip_re(double2 w0, double2 w1, double2 v0, double2 v1, double2 g, double2 h) {
+    const double2 a = s_cmul(h, v1), b = s_cmul(g, v0);
+    return (w0.x * a.x + w0.y * a.y) + (w1.x * b.x + w1.y * b.y);
+}
+__device__ __forceinline__ double v_of(double, double2 z, double f) { return z.x * f; }
+__device__ __forceinline__ double2 v_of(double2, double2 z, double f) { return make_double2(z.x * f, z.y * f); }
+// a, negated when bit 31 of w is set
+__device__ __forceinline__ double v_flip(double a, uint32_t w) {
+    return __hiloint2double(__double2hiint(a) ^ (int)(w & 0x80000000u), __double2loint(a));
+}
+__device__ __forceinline__ double2 v_flip(double2 a, uint32_t w) {
+    return make_double2(v_flip(a.x, w), v_flip(a.y, w));
+}
+// c x + a y
+__device__ __forceinline__ double v_rot(double c, double x, double a, double y) { return c * x + a * y; }
+__device__ __forceinline__ double2 v_rot(double c, double2 x, double2 a, double2 y) {
+    return make_double2(c * x.x + (a.x * y.x - a.y * y.y), c * x.y + (a.x * y.y + a.y * y.x));
 }
 
-// The coefficients of record h when it has a single pattern (else zeros)
+// What a record's pairs are worked with, for one parameter set: cos, sin times
+// the two coefficients and, in the sweep, gamma times them (zero without an
+// inner product; cos 1 and sin 0 without a rotation).
+template <bool SWEEP, class V>
+struct __align__(16) PCoef;
 template <class V>
-__device__ __forceinline__ void p_coef(const PStream &S, const PHead &h, V &gn, V &hn) {
-    gn = hn = v_zero(V());
-    if ((h.fl >> 8) == 1) p_ldcoef(S, h.c0, gn, hn);
-}
-
-// A record as the kernels keep it in shared memory: its header, the cos / sin
-// of its angle for this CTA's parameter set and, for a single-pattern record,
-// its coefficients.
-template <class V>
-struct PSmem {
-    PHead h;
-    double2 cs;
-    V gn, hn;
+struct __align__(16) PCoef<false, V> {
+    V a, b;  // sin hn, sin gn
+    double c, pad;
 };
-static_assert(sizeof(PSmem<double>) == 64 && sizeof(PSmem<double2>) == 80, "PSmem layout");
-
-// Every record's header, coefficients and cos / sin of sign * gamma * theta
-// into s_pr
 template <class V>
-__device__ __forceinline__ void p_angles(const PStream &S, const double *par, int sign,
-                                         PSmem<V> *s_pr) {
+struct __align__(16) PCoef<true, V> {
+    V a, b, h, g;
+    double c, pad;
+};
+static_assert(sizeof(PCoef<true, double>) == 48 && sizeof(PCoef<true, double2>) == 80, "PCoef layout");
+
+__device__ __forceinline__ RRec r_head(const RRec *p) {
+    RRec h;
+    const int4 a = __ldg(reinterpret_cast<const int4 *>(p));
+    h.gamma = __hiloint2double(a.y, a.x);
+    h.param = a.z;
+    h.fl = a.w;
+    h.gn = __ldg(&p->gn);
+    h.hn = __ldg(&p->hn);
+    return h;
+}
+
+// Every record's PCoef for the angles sign * gamma * theta, record r at cf[r + 1].
+template <bool SWEEP, class V>
+__device__ __forceinline__ void p_angles(const RStream &S, const double *par, int sign,
+                                         PCoef<SWEEP, V> *cf) {
     for (int r = threadIdx.x; r < S.n; r += blockDim.x) {
-        const PHead h = p_head(S.hd + r);
-        double sn, cs;
-        sincos((double)sign * h.gamma * par[h.param], &sn, &cs);
-        V gn, hn;
-        p_coef(S, h, gn, hn);
-        s_pr[r].h = h;
-        s_pr[r].cs = make_double2(cs, sn);
-        s_pr[r].gn = gn;
-        s_pr[r].hn = hn;
+        const RRec h = r_head(S.hd + r);
+        double sn = 0.0, cs = 1.0;
+        if (h.fl & R_ROT) sincos((double)sign * h.gamma * par[h.param], &sn, &cs);
+        PCoef<SWEEP, V> o;
+        o.c = cs;
+        o.pad = 0.0;
+        o.a = v_of(V(), h.hn, sn);
+        o.b = v_of(V(), h.gn, sn);
+        if constexpr (SWEEP) {
+            const double f = (h.fl & R_IP) ? h.gamma : 0.0;
+            o.h = v_of(V(), h.hn, f);
+            o.g = v_of(V(), h.gn, f);
+        }
+        cf[r + 1] = o;
     }
 }
 
@@ -313,16 +301,6 @@ __device__ __forceinline__ double2 v_shfl_xor(double2 v, int o) {
     return make_double2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
 }
 
-// Warp sums of two values at once: a's into lane 0, b's into lane 16 (the
-// first exchange halves the work of two separate reductions).
-template <class V>
-__device__ __forceinline__ V p_sum2(V a, V b) {
-    const bool hi = threadIdx.x & 16;
-    V k = v_add(hi ? b : a, v_shfl_xor(hi ? a : b, 16));
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) k = v_add(k, v_shfl_down(k, o));
-    return k;
-}
 template <class V>
 __device__ __forceinline__ V p_sum1(V a) {
 #pragma unroll
@@ -330,131 +308,204 @@ __device__ __forceinline__ V p_sum1(V a) {
     return a;
 }
 
-// Apply record rec with this thread's prefetched words; returns this
-// thread's share of the record's inner product (SWEEP records carry flags:
-// rotation of both states, inner product or both).
-template <bool SWEEP, class V, int KP>
-__device__ __forceinline__ V p_step(const PStream &S, const PSmem<V> &rec, const uint32_t (&pw)[KP],
-                                    V *v, V *w) {
-    const PHead h = rec.h;
-    const double2 csn = rec.cs;
-    const V gn = rec.gn, hn = rec.hn;
-    const int fl = h.fl & 255;
-    V acc = v_zero(V());
-    if (!SWEEP) {
-        p_record<true, false, false, V, KP>(S, h, pw, csn, gn, hn, v, w, acc);
-    } else if (fl == (R_ROT | R_IP | R_TWO)) {
-        p_record<true, true, true, V, KP>(S, h, pw, csn, gn, hn, v, w, acc);
-    } else if (fl == R_IP) {
-        p_record<false, true, false, V, KP>(S, h, pw, csn, gn, hn, v, w, acc);
-    } else {
-        p_record<true, false, true, V, KP>(S, h, pw, csn, gn, hn, v, w, acc);
+// Warp sums of four rounds' values on the FP64 matrix units: round j's lane
+// values, as a 4 x 8 matrix, are multiplied from the left by ones in row j, so
+// row j of the accumulators holds their 8 column sums (two per lane, lanes
+// 4 j .. 4 j + 3).  One instruction a round instead of three shuffles.
+struct RSum {
+    double d0 = 0.0, d1 = 0.0;
+    __device__ __forceinline__ void add(int j, double x) {
+        const double a = ((threadIdx.x & 31) >> 2) == j ? 1.0 : 0.0;
+        asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+            : "+d"(d0), "+d"(d1)
+            : "d"(a), "d"(x));
     }
-    return acc;
-}
+    // round j's sum in lanes 4 j .. 4 j + 3
+    __device__ __forceinline__ double sum() const {
+        double t = d0 + d1;
+        t += v_shfl_xor(t, 1);
+        return t + v_shfl_xor(t, 2);
+    }
+};
 
-// The warp partials of the inner products of records a and b (b < 0: none):
-// one per warp and record at partial[row][slot][warp] (nslot slots), zero
-// from warps that hold no pair of the record, two records reduced together
-// where both have one.
 template <class V>
-__device__ __forceinline__ void p_partials(const PSmem<V> *s_pr, int a, V acca, int b, V accb,
-                                           double2 *partial, int nslot, int slot) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const PHead ha = s_pr[a].h;
-    const bool ipa = ha.fl & R_IP;
-    bool ipb = false;
-    PHead hb = ha;
-    if (b >= 0) {
-        hb = s_pr[b].h;
-        ipb = hb.fl & R_IP;
-    }
-    if (!ipa && !ipb) return;
-    const bool ida = 32 * warp >= ha.np, idb = 32 * warp >= hb.np;  // warp holds no pair
-    auto put = [&](const PHead &h, V x) {
-        partial[((size_t)h.row * nslot + slot) * nw + warp] = v_as2(x);
-    };
-    if (ipa && ipb && !ida && !idb) {
-        const V k = p_sum2(acca, accb);
-        if (lane == 0) put(ha, k);
-        if (lane == 16) put(hb, k);
-        return;
-    }
-    if (ipa) {
-        const V k = ida ? v_zero(V()) : p_sum1(acca);
-        if (lane == 0) put(ha, k);
-    }
-    if (ipb) {
-        const V k = idb ? v_zero(V()) : p_sum1(accb);
-        if (lane == 0) put(hb, k);
+__device__ __forceinline__ V &r_at0(V *v, uint32_t w) {
+    return *reinterpret_cast<V *>(reinterpret_cast<char *>(v) + (w & kWordIdx) * (uint32_t)(sizeof(V) / 8));
+}
+template <class V>
+__device__ __forceinline__ V &r_at1(V *v, uint32_t w) {
+    return *reinterpret_cast<V *>(reinterpret_cast<char *>(v) +
+                                  ((w >> kPairIdxBits) & kWordIdx) * (uint32_t)(sizeof(V) / 8));
+}
+
+// One round: f rotates (and accumulates) the pair of `word` with the record's
+// constants; the constants of the next round's record are loaded meanwhile.
+template <bool REV, class C, class F>
+__device__ __forceinline__ void r_round(uint32_t word, C &c, const C *&cf, int nth, const F &f) {
+    cf += REV ? -(int)((word >> 1) & 1u) : (int)(word & 1u);
+    const C next = *cf;
+    f(word, c);
+    c = next;
+    asm volatile("bar.sync 1, %0;" ::"r"(nth) : "memory");
+}
+
+// Run a stream's rounds (REV: in reverse order), f(word, constants, j) per
+// pair, j the round's number modulo 4, and done(r) after rounds r .. r + 3.
+// Threads past S.nth do nothing.
+//
+// Bound by the latency of one round after another: a barrier, the amplitudes'
+// way through shared memory, two dependent FP64 operations.  So nothing else
+// lies on that path: no thread tests for its pair or its record's kind, the
+// word was loaded four rounds before (L2), the constants one round before.
+template <bool REV, class C, class F, class G>
+__device__ __forceinline__ void r_run(const RStream &S, const C *cf, const F &f, const G &done) {
+    const int nth = S.nth, tid = threadIdx.x;
+    if (S.nr == 0 || tid >= nth) return;
+    const int step = REV ? -nth : nth;
+    const uint32_t *wp = S.word + (REV ? (size_t)(S.nr - 1) * nth : 0) + tid;
+    cf += REV ? S.n : 1;
+    C c = *cf;
+    uint32_t w0 = __ldg(wp), w1 = __ldg(wp + step), w2 = __ldg(wp + 2 * step), w3 = __ldg(wp + 3 * step);
+    for (int r = 0; r < S.nr; r += 4) {
+        wp += 4 * step;
+        const uint32_t n0 = __ldg(wp);
+        r_round<REV>(w0, c, cf, nth, [&](uint32_t w, const C &k) { f(w, k, 0); });
+        const uint32_t n1 = __ldg(wp + step);
+        r_round<REV>(w1, c, cf, nth, [&](uint32_t w, const C &k) { f(w, k, 1); });
+        const uint32_t n2 = __ldg(wp + 2 * step);
+        r_round<REV>(w2, c, cf, nth, [&](uint32_t w, const C &k) { f(w, k, 2); });
+        const uint32_t n3 = __ldg(wp + 3 * step);
+        r_round<REV>(w3, c, cf, nth, [&](uint32_t w, const C &k) { f(w, k, 3); });
+        done(r);
+        w0 = n0;
+        w1 = n1;
+        w2 = n2;
+        w3 = n3;
     }
 }
 
-// Run a stream, one barrier per record.  RING register sets rotate: while
-// record r is applied from one, the pair words of the next RING - 1 records
-// are in flight in the others (each set is refilled right after its record
-// ran), so a record's words have had RING - 1 records' time to arrive from
-// L2.  SWEEP: the inner products of records (r, r + 1) are reduced together.
-template <bool SWEEP, class V>
-__device__ __forceinline__ void p_run(const PStream &S, const PSmem<V> *s_pr, V *v, V *w,
-                                      double2 *partial, int nslot, int slot) {
-    constexpr int KP = pair_slots<V>();
-    constexpr int RING = SWEEP ? kSweepRing : 4;
-    const int n = S.n;
-    uint32_t w0[KP], w1[KP], w2[KP], w3[KP];
-    if (n > 0) p_words(S, s_pr[0].h, w0);
-    if (n > 1) p_words(S, s_pr[1].h, w1);
-    if (RING == 4 && n > 2) p_words(S, s_pr[2].h, w2);
-    for (int r = 0; r < n; r += RING) {
-        if (RING == 4 && r + 3 < n) p_words(S, s_pr[r + 3].h, w3);
-        const V a0 = p_step<SWEEP, V, KP>(S, s_pr[r], w0, v, w);
-        __syncthreads();
-        if (r + 1 >= n) {
-            if (SWEEP) p_partials(s_pr, r, a0, -1, a0, partial, nslot, slot);
-            break;
-        }
-        if (r + RING < n) p_words(S, s_pr[r + RING].h, w0);
-        const V a1 = p_step<SWEEP, V, KP>(S, s_pr[r + 1], w1, v, w);
-        if (SWEEP) p_partials(s_pr, r, a0, r + 1, a1, partial, nslot, slot);
-        __syncthreads();
-        if (RING == 2) {
-            if (r + 3 < n) p_words(S, s_pr[r + 3].h, w1);
-            continue;
-        }
-        if (r + 2 >= n) break;
-        if (r + 5 < n) p_words(S, s_pr[r + 5].h, w1);
-        const V a2 = p_step<SWEEP, V, KP>(S, s_pr[r + 2], w2, v, w);
-        __syncthreads();
-        if (r + 3 >= n) {
-            if (SWEEP) p_partials(s_pr, r + 2, a2, -1, a2, partial, nslot, slot);
-            break;
-        }
-        if (r + 6 < n) p_words(S, s_pr[r + 6].h, w2);
-        const V a3 = p_step<SWEEP, V, KP>(S, s_pr[r + 3], w3, v, w);
-        if (SWEEP) p_partials(s_pr, r + 2, a2, r + 3, a3, partial, nslot, slot);
-        __syncthreads();
+// The forward program (REV: its inverse, with the angles' sign) on v.
+template <bool REV, class V>
+__device__ __forceinline__ void p_forward(const RStream &S, const PCoef<false, V> *cf, V *v) {
+    r_run<REV>(
+        S, cf,
+        [&](uint32_t w, const PCoef<false, V> &k, int) {
+            V &x0 = r_at0(v, w), &x1 = r_at1(v, w);
+            const V v0 = x0, v1 = x1;
+            x0 = v_rot(k.c, v0, v_flip(k.a, w), v1);
+            x1 = v_rot(k.c, v1, v_flip(k.b, w), v0);
+        },
+        [](int) {});
+}
+
+// psi and sigma of the sweep in shared memory: complex amplitudes as two
+// arrays, real ones interleaved (both states' amplitude in one 16-byte access).
+template <class V>
+struct SweepState;
+template <>
+struct SweepState<double> {
+    double2 *x;
+    __device__ __forceinline__ SweepState(unsigned char *raw, int) : x(reinterpret_cast<double2 *>(raw)) {}
+    __device__ __forceinline__ void set(int i, double p, double s) { x[i] = make_double2(p, s); }
+    __device__ __forceinline__ double round(uint32_t w, const PCoef<true, double> &k) {
+        double2 &r0 = r_at0(x, w), &r1 = r_at1(x, w);
+        const double2 v0 = r0, v1 = r1;
+        const double a = v_flip(k.a, w), b = v_flip(k.b, w);
+        r0 = make_double2(v_rot(k.c, v0.x, a, v1.x), v_rot(k.c, v0.y, a, v1.y));
+        r1 = make_double2(v_rot(k.c, v1.x, b, v0.x), v_rot(k.c, v1.y, b, v0.y));
+        return v_flip(v_ip_re(v0.y, v1.y, v0.x, v1.x, k.g, k.h), w);
     }
+};
+template <>
+struct SweepState<double2> {
+    double2 *v, *w;
+    __device__ __forceinline__ SweepState(unsigned char *raw, int nsec)
+        : v(reinterpret_cast<double2 *>(raw)), w(v + nsec + kRoundPad) {}
+    __device__ __forceinline__ void set(int i, double2 p, double2 s) {
+        v[i] = p;
+        w[i] = s;
+    }
+    __device__ __forceinline__ double round(uint32_t word, const PCoef<true, double2> &k) {
+        double2 &x0 = r_at0(v, word), &x1 = r_at1(v, word), &y0 = r_at0(w, word), &y1 = r_at1(w, word);
+        const double2 v0 = x0, v1 = x1, w0 = y0, w1 = y1;
+        const double2 a = v_flip(k.a, word), b = v_flip(k.b, word);
+        x0 = v_rot(k.c, v0, a, v1);
+        x1 = v_rot(k.c, v1, b, v0);
+        y0 = v_rot(k.c, w0, a, w1);
+        y1 = v_rot(k.c, w1, b, w0);
+        return v_flip(v_ip_re(w0, w1, v0, v1, k.g, k.h), word);
+    }
+};
+// psi and sigma of one slot from the save buffer (sig: its sigma)
+template <class V>
+__device__ __forceinline__ void sweep_load(SweepState<V> &st, const V *psi, const V *sig, int nsec) {
+    for (int i = threadIdx.x; i < nsec + kRoundPad; i += blockDim.x)
+        st.set(i, i < nsec ? psi[i] : v_zero(V()), i < nsec ? sig[i] : v_zero(V()));
+}
+
+// The reverse sweep; partial: this slot's [rounds / 4][warps][4] warp sums of
+// the rounds' inner products.
+template <class V>
+__device__ __forceinline__ void p_sweep(const RStream &S, const PCoef<true, V> *cf, SweepState<V> &st,
+                                        double *partial) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = S.nth >> 5;
+    RSum ip;
+    r_run<false>(
+        S, cf, [&](uint32_t word, const PCoef<true, V> &k, int j) { ip.add(j, st.round(word, k)); },
+        [&](int r) {
+            const double t = ip.sum();
+            if ((lane & 3) == 0 && lane < 16) partial[((size_t)(r >> 2) * nw + warp) * 4 + (lane >> 2)] = t;
+            ip = RSum();
+        });
+}
+
+// grad[mu] = 2 x the sums of parameter mu's rounds, in round and warp order
+// (after a barrier that follows p_sweep).
+__device__ __forceinline__ void p_grad(const int2 *prange, int nparam, int nw, const double *partial,
+                                       double *grad) {
+    for (int mu = threadIdx.x; mu < nparam; mu += blockDim.x) {
+        const int2 pr = prange[mu];
+        double acc = 0.0;
+        for (int r = pr.x; r < pr.y; ++r)
+            for (int k = 0; k < nw; ++k) acc += partial[((size_t)(r >> 2) * nw + k) * 4 + (r & 3)];
+        grad[mu] = 2.0 * acc;
+    }
+}
+
+// Shared memory of the step kernels: nstates states, each with kRoundPad unused
+// amplitudes, then the records' constants (one unused on either side).
+template <class C>
+__host__ __device__ inline size_t step_smem(int nstates, int nsec, size_t elem, int nrec) {
+    return ((nstates * (size_t)(nsec + kRoundPad) * elem + 15) & ~(size_t)15) + sizeof(C) * (size_t)(nrec + 2);
+}
+template <class C>
+__device__ __forceinline__ C *step_coef(unsigned char *raw, int nstates, int nsec, size_t elem) {
+    return reinterpret_cast<C *>(raw + ((nstates * (size_t)(nsec + kRoundPad) * elem + 15) & ~(size_t)15));
+}
+template <class V>
+__device__ __forceinline__ void step_pad(V *v, int nsec) {
+    for (int i = threadIdx.x; i < kRoundPad; i += blockDim.x) v[nsec + i] = v_zero(V());
 }
 
 // The evaluation runs as three kernels: the forward program (one CTA per
 // parameter set, psi in shared memory), sigma = H psi with the energy (a few
 // parameter sets and a slice of the rows per CTA, sigma rows straight to the
 // save buffer), and the reverse sweep (one CTA per parameter set, psi and
-// sigma in shared memory).  Shared memory of the forward and sweep kernels:
-// the states, then every record's header with the cos / sin of its angle
-// (PSmem).
+// sigma in shared memory) with the gradient.
 
 template <class V>
-__global__ void __launch_bounds__(kStepThreads, 1024 / kStepThreads) k_sector_forward(SLaunch L) {
+__global__ void __launch_bounds__(kStepThreads, 2) k_sector_forward(SLaunch L) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     V *psi = reinterpret_cast<V *>(s_raw);
-    PSmem<V> *s_pr = reinterpret_cast<PSmem<V> *>(s_raw + ((sizeof(V) * L.nsec + 15) & ~(size_t)15));
+    PCoef<false, V> *cf = step_coef<PCoef<false, V>>(s_raw, 1, L.nsec, sizeof(V));
     const int b = blockIdx.x, tid = threadIdx.x, nth = blockDim.x;
     const double *par = L.params + (size_t)b * L.nparam;
     for (int i = tid; i < L.nsec; i += nth) psi[i] = i == L.ref_i ? v_one_of<V>() : v_zero(V());
-    p_angles(L.fwd, par, 1, s_pr);
+    step_pad(psi, L.nsec);
+    p_angles<false, V>(L.fwd, par, 1, cf);
     __syncthreads();
-    p_run<false, V>(L.fwd, s_pr, psi, (V *)nullptr, nullptr, 1, 0);
+    p_forward<false, V>(L.fwd, cf, psi);
+    __syncthreads();
     V *sv = reinterpret_cast<V *>(L.save) + (size_t)b * 2 * L.nsec;
     for (int i = tid; i < L.nsec; i += nth) sv[i] = psi[i];
 }
@@ -597,38 +648,41 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_sector_h(
 }
 
 template <class V>
-__global__ void __launch_bounds__(kSweepThreads, 1024 / kSweepThreads) k_sector_sweep(SLaunch L) {
+__global__ void __launch_bounds__(kStepThreads, sizeof(V) == sizeof(double) ? 2 : 1) k_sector_sweep(SLaunch L) {
     extern __shared__ __align__(16) unsigned char s_raw[];
-    V *psi = reinterpret_cast<V *>(s_raw), *sig = psi + L.nsec;
-    PSmem<V> *s_pr = reinterpret_cast<PSmem<V> *>(s_raw + ((sizeof(V) * 2 * L.nsec + 15) & ~(size_t)15));
-    const int b = blockIdx.x, tid = threadIdx.x, nth = blockDim.x;
-    const double *par = L.params + (size_t)b * L.nparam;
+    SweepState<V> st(s_raw, L.nsec);
+    PCoef<true, V> *cf = step_coef<PCoef<true, V>>(s_raw, 2, L.nsec, sizeof(V));
+    const int b = blockIdx.x;
     const V *sv = reinterpret_cast<const V *>(L.save) + (size_t)b * 2 * L.nsec;
-    for (int i = tid; i < 2 * L.nsec; i += nth) psi[i] = sv[i];
-    p_angles(L.sweep, par, -1, s_pr);
+    sweep_load(st, sv, sv + L.nsec, L.nsec);
+    p_angles<true, V>(L.sweep, L.params + (size_t)b * L.nparam, -1, cf);
     __syncthreads();
-    p_run<true, V>(L.sweep, s_pr, psi, sig, L.partial, gridDim.x, blockIdx.x);
+    double *part = L.partial + (size_t)b * L.sweep.nr * (L.sweep.nth >> 5);
+    p_sweep<V>(L.sweep, cf, st, part);
+    __syncthreads();
+    p_grad(L.prange, L.nparam, L.sweep.nth >> 5, part, L.grad + (size_t)b * L.nparam);
 }
 
 // PQE residuals on the compact states: sigma of slot blockIdx.x from the save
-// buffer, U^dagger applied to it in shared memory (stream R: the forward
-// records in reverse order, angles negated), then
+// buffer, U^dagger applied to it in shared memory (the forward rounds in
+// reverse order, angles negated), then
 // res[b][k] = Re(sigma[idx[k]] * phase[k]) (0 where idx[k] < 0).
 template <class V>
-__global__ void __launch_bounds__(kStepThreads, 1024 / kStepThreads) k_sector_resid(SLaunch L, PStream R,
-                                                         const int64_t *__restrict__ idx,
-                                                         const double2 *__restrict__ phase,
-                                                         int nres, double *__restrict__ res) {
+__global__ void __launch_bounds__(kStepThreads, 2) k_sector_resid(SLaunch L, const int64_t *__restrict__ idx,
+                                                                  const double2 *__restrict__ phase,
+                                                                  int nres, double *__restrict__ res) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     V *sig = reinterpret_cast<V *>(s_raw);
-    PSmem<V> *s_pr = reinterpret_cast<PSmem<V> *>(s_raw + ((sizeof(V) * L.nsec + 15) & ~(size_t)15));
+    PCoef<false, V> *cf = step_coef<PCoef<false, V>>(s_raw, 1, L.nsec, sizeof(V));
     const int b = blockIdx.x, tid = threadIdx.x, nth = blockDim.x;
     const double *par = L.params + (size_t)b * L.nparam;
     const V *sv = reinterpret_cast<const V *>(L.save) + (size_t)b * 2 * L.nsec + L.nsec;
     for (int i = tid; i < L.nsec; i += nth) sig[i] = sv[i];
-    p_angles(R, par, -1, s_pr);
+    step_pad(sig, L.nsec);
+    p_angles<false, V>(L.fwd, par, -1, cf);
     __syncthreads();
-    p_run<false, V>(R, s_pr, sig, (V *)nullptr, nullptr, 1, 0);
+    p_forward<true, V>(L.fwd, cf, sig);
+    __syncthreads();
     for (int k = tid; k < nres; k += nth) {
         const int64_t i = idx[k];
         double r = 0.0;
@@ -645,7 +699,7 @@ __global__ void __launch_bounds__(kStepThreads, 1024 / kStepThreads) k_sector_re
 // blockIdx.x + gridDim.x, ... of the pool stream.  The records leave the
 // states unchanged, so they need no barrier between them.
 template <class V>
-__global__ void __launch_bounds__(512, 2) k_sector_pool(SLaunch L, PStream P) {
+__global__ void __launch_bounds__(512, 2) k_sector_pool(SLaunch L, PStream P, double2 *__restrict__ partial) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     V *psi = reinterpret_cast<V *>(s_raw), *sig = psi + L.nsec;
     const int b = blockIdx.y, tid = threadIdx.x, nth = blockDim.x, nw = nth >> 5;
@@ -653,17 +707,22 @@ __global__ void __launch_bounds__(512, 2) k_sector_pool(SLaunch L, PStream P) {
     for (int i = tid; i < 2 * L.nsec; i += nth) psi[i] = sv[i];
     __syncthreads();
     for (int r = blockIdx.x; r < P.n; r += gridDim.x) {
-        constexpr int KP = pair_slots<V>();
         const PHead h = p_head(P.hd + r);
-        uint32_t pw[KP];
-        p_words(P, h, pw);
-        V gn, hn;
-        p_coef(P, h, gn, hn);
+        const bool one = (h.fl >> 8) == 1;
+        V gn = v_zero(V()), hn = gn;
+        if (one) p_ldcoef(P, h.c0, gn, hn);
         V acc = v_zero(V());
-        p_record<false, true, false, V, KP>(P, h, pw, make_double2(1.0, 0.0), gn, hn, psi, sig, acc);
+        for (int k = tid; k < h.np; k += nth) {
+            const uint32_t word = __ldg(P.pair + h.p0 + k);
+            constexpr uint32_t M = (1u << kPairIdxBits) - 1u;
+            const uint32_t i0 = word & M, i1 = (word >> kPairIdxBits) & M;
+            if (!one) p_ldcoef(P, h.c0 + (int)(word >> (2 * kPairIdxBits + 1)), gn, hn);
+            const double f = (word >> (2 * kPairIdxBits)) & 1u ? -h.gamma : h.gamma;
+            v_acc(acc, f, v_ip(sig[i0], sig[i1], psi[i0], psi[i1], gn, hn));
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc = v_add(acc, v_shfl_down(acc, o));
-        if ((tid & 31) == 0) L.partial[((size_t)h.row * gridDim.y + b) * nw + (tid >> 5)] = v_as2(acc);
+        if ((tid & 31) == 0) partial[((size_t)h.row * gridDim.y + b) * nw + (tid >> 5)] = v_as2(acc);
     }
 }
 
@@ -675,89 +734,38 @@ __global__ void __launch_bounds__(512, 2) k_sector_pool(SLaunch L, PStream P) {
 // 2g + 1), so every pair word, record header, shared-memory load / store and
 // barrier serves both sets, while each set keeps its own angle (cos / sin per
 // set in the record).  The arithmetic on each set is that of k_sector_forward.
-// (The reverse sweep stays one set per CTA: paired, its shared memory of two
-// states for two sets leaves half the warps per set to hide latency, and it
-// ran slower at 256 sets on 148 SMs.)
+// (The reverse sweep stays one set per CTA: its 16-byte slot holds the set's
+// psi and sigma.)
 
-struct PSmemPR {
-    PHead h;
-    double2 c, s;   // cos / sin of the record's angle: .x first set, .y second
-    double gn, hn;  // single-pattern records: the coefficients
+struct __align__(16) PCoefPR {
+    double2 c, a, b;  // cos, sin hn, sin gn: .x first set, .y second
 };
-static_assert(sizeof(PSmemPR) == 80, "PSmemPR layout");
 
-__device__ __forceinline__ void p_angles_pr(const PStream &S, const double *parA, const double *parB,
-                                            int sign, PSmemPR *s_pr) {
+__device__ __forceinline__ void p_angles_pr(const RStream &S, const double *parA, const double *parB,
+                                            PCoefPR *cf) {
     for (int r = threadIdx.x; r < S.n; r += blockDim.x) {
-        const PHead h = p_head(S.hd + r);
-        double sa, ca, sb, cb;
-        sincos((double)sign * h.gamma * parA[h.param], &sa, &ca);
-        sincos((double)sign * h.gamma * parB[h.param], &sb, &cb);
-        double gn, hn;
-        p_coef(S, h, gn, hn);
-        s_pr[r].h = h;
-        s_pr[r].c = make_double2(ca, cb);
-        s_pr[r].s = make_double2(sa, sb);
-        s_pr[r].gn = gn;
-        s_pr[r].hn = hn;
+        const RRec h = r_head(S.hd + r);
+        double sa = 0.0, ca = 1.0, sb = 0.0, cb = 1.0;
+        if (h.fl & R_ROT) {
+            sincos(h.gamma * parA[h.param], &sa, &ca);
+            sincos(h.gamma * parB[h.param], &sb, &cb);
+        }
+        cf[r + 1] = PCoefPR{make_double2(ca, cb), make_double2(sa * h.hn.x, sb * h.hn.x),
+                            make_double2(sa * h.gn.x, sb * h.gn.x)};
     }
 }
 
-// One pair of a forward record on both sets (p_pair's rotation per set).
-__device__ __forceinline__ void pr_pair(uint32_t pw, double2 c, double2 s, double gn, double hn,
-                                        double2 *v) {
-    constexpr uint32_t M = (1u << kPairIdxBits) - 1u;
-    const int i0 = (int)(pw & M), i1 = (int)((pw >> kPairIdxBits) & M);
-    const bool neg = (pw >> (2 * kPairIdxBits)) & 1u;
-    const double2 a0 = v[i0], a1 = v[i1];
-    const double sx = neg ? -s.x : s.x, sy = neg ? -s.y : s.y;
-    v[i0] = make_double2(c.x * a0.x + sx * (hn * a1.x), c.y * a0.y + sy * (hn * a1.y));
-    v[i1] = make_double2(c.x * a1.x + sx * (gn * a0.x), c.y * a1.y + sy * (gn * a0.y));
-}
-
-template <int KP>
-__device__ __forceinline__ void pr_record(const PStream &S, const PSmemPR &rec, const uint32_t (&pw)[KP],
-                                          double2 *v) {
-    const int tid = threadIdx.x, nth = blockDim.x;
-    const PHead &h = rec.h;
-    const bool one = (h.fl >> 8) == 1;
-    double gn = rec.gn, hn = rec.hn;
-    auto run = [&](uint32_t p) {
-        if (!one) p_ldcoef(S, h.c0 + (int)(p >> (2 * kPairIdxBits + 1)), gn, hn);
-        pr_pair(p, rec.c, rec.s, gn, hn, v);
-    };
-#pragma unroll
-    for (int j = 0; j < KP; ++j)
-        if (tid + j * nth < h.np) run(pw[j]);
-    for (int k = tid + KP * nth; k < h.np; k += nth) run(__ldg(S.pair + h.p0 + k));
-}
-
-// p_run's forward program for two real sets: the same ring of four
-// prefetched sets of pair words, one barrier per record.
-__device__ __forceinline__ void pr_run(const PStream &S, const PSmemPR *s_pr, double2 *v) {
-    constexpr int KP = 2;
-    const int n = S.n;
-    uint32_t w0[KP], w1[KP], w2[KP], w3[KP];
-    if (n > 0) p_words(S, s_pr[0].h, w0);
-    if (n > 1) p_words(S, s_pr[1].h, w1);
-    if (n > 2) p_words(S, s_pr[2].h, w2);
-    for (int r = 0; r < n; r += 4) {
-        if (r + 3 < n) p_words(S, s_pr[r + 3].h, w3);
-        pr_record<KP>(S, s_pr[r], w0, v);
-        __syncthreads();
-        if (r + 1 >= n) break;
-        if (r + 4 < n) p_words(S, s_pr[r + 4].h, w0);
-        pr_record<KP>(S, s_pr[r + 1], w1, v);
-        __syncthreads();
-        if (r + 2 >= n) break;
-        if (r + 5 < n) p_words(S, s_pr[r + 5].h, w1);
-        pr_record<KP>(S, s_pr[r + 2], w2, v);
-        __syncthreads();
-        if (r + 3 >= n) break;
-        if (r + 6 < n) p_words(S, s_pr[r + 6].h, w2);
-        pr_record<KP>(S, s_pr[r + 3], w3, v);
-        __syncthreads();
-    }
+__device__ __forceinline__ void pr_forward(const RStream &S, const PCoefPR *cf, double2 *v) {
+    r_run<false>(
+        S, cf,
+        [&](uint32_t w, const PCoefPR &k, int) {
+            double2 &x0 = r_at0(v, w), &x1 = r_at1(v, w);
+            const double2 v0 = x0, v1 = x1;
+            const double2 a = v_flip(k.a, w), b = v_flip(k.b, w);
+            x0 = make_double2(v_rot(k.c.x, v0.x, a.x, v1.x), v_rot(k.c.y, v0.y, a.y, v1.y));
+            x1 = make_double2(v_rot(k.c.x, v1.x, b.x, v0.x), v_rot(k.c.y, v1.y, b.y, v0.y));
+        },
+        [](int) {});
 }
 
 // Forward program of sets 2g, 2g + 1 (g = blockIdx.x; a last odd set runs
@@ -765,16 +773,18 @@ __device__ __forceinline__ void pr_run(const PStream &S, const PSmemPR *s_pr, do
 __global__ void __launch_bounds__(kStepThreads, 1) k_sector_forward_pr(SLaunch L, int nbatch) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     double2 *psi = reinterpret_cast<double2 *>(s_raw);
-    PSmemPR *s_pr = reinterpret_cast<PSmemPR *>(s_raw + ((16 * (size_t)L.nsec + 15) & ~(size_t)15));
+    PCoefPR *cf = step_coef<PCoefPR>(s_raw, 1, L.nsec, sizeof(double2));
     const int b0 = 2 * blockIdx.x, tid = threadIdx.x, nth = blockDim.x;
     const bool two = b0 + 1 < nbatch;
     const double *parA = L.params + (size_t)b0 * L.nparam;
     const double *parB = two ? parA + L.nparam : parA;
     for (int i = tid; i < L.nsec; i += nth)
         psi[i] = i == L.ref_i ? make_double2(1.0, 1.0) : make_double2(0.0, 0.0);
-    p_angles_pr(L.fwd, parA, parB, 1, s_pr);
+    step_pad(psi, L.nsec);
+    p_angles_pr(L.fwd, parA, parB, cf);
     __syncthreads();
-    pr_run(L.fwd, s_pr, psi);
+    pr_forward(L.fwd, cf, psi);
+    __syncthreads();
     double *sv = reinterpret_cast<double *>(L.save) + (size_t)b0 * 2 * L.nsec;
     for (int i = tid; i < L.nsec; i += nth) {
         const double2 x = psi[i];
@@ -788,28 +798,42 @@ __global__ void __launch_bounds__(kStepThreads, 1) k_sector_forward_pr(SLaunch L
 // ---------------------------------------------------------------------------
 
 // One problem of a packed launch: the compact evaluator data of one dUCC
-// problem (its sector, forward and sweep pair lists, H rows on the sector and
-// the sweep record rows of each parameter).
+// problem (its sector, forward and sweep rounds, H rows on the sector and the
+// sweep rounds of each parameter).
 struct PackMember {
     int nsec, ref_i, nparam, pad;
-    PStream fwd, sweep;
+    RStream fwd, sweep;
     const int32_t *rowptr;
     const uint32_t *col;
     const double *val_r;   // real H (val_c == nullptr) ...
     const double2 *val_c;  // ... or complex
-    const int2 *psteps;    // per parameter: its rows of the sweep partials
+    const int2 *prange;    // rounds of the sweep of each parameter
 };
 
-constexpr int kPackThreads = 256;
+// A packed launch's buffers.
+struct PackLaunch {
+    const PackMember *members;
+    const int2 *items;  // (problem, with gradient)
+    int nmem, maxparam;
+    const double *params;  // [items][maxparam]
+    double *energy, *grad;
+    double *partial;       // [items][maxpart]: the sweeps' warp sums
+    size_t maxpart;
+    void *save;            // V [items][2][maxsec]: psi, sigma
+    int maxsec, Q;         // Q: CTAs an item's H rows are split over
+    double *epart;         // [items][Q]
+    unsigned *count;       // [items]: CTAs done
+};
 
-// sigma = H psi on one CTA's state (a warp per row, the lanes over the row's
-// entries) and this CTA's energy <psi|H|psi>, summed in a fixed order.
+// Rows r0 .. r1 of sigma = H psi (a warp per row, the lanes over the row's
+// entries) and this CTA's share of <psi|H|psi>, summed in a fixed order.
 template <class V>
-__device__ __forceinline__ double p_hpsi(const PackMember &m, const V *psi, V *sig, double *s_red) {
+__device__ __forceinline__ double p_hpsi(const PackMember &m, int r0, int r1, const V *psi, V *sig,
+                                         double *s_red) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     constexpr int U = 4;  // row entries in flight per lane
     double en = 0.0;
-    for (int i = warp; i < m.nsec; i += nw) {
+    for (int i = r0 + warp; i < r1; i += nw) {
         V acc = v_zero(V());
         const int e1 = m.rowptr[i + 1];
         for (int e0 = m.rowptr[i] + lane; e0 < e1; e0 += 32 * U) {
@@ -853,56 +877,104 @@ __device__ __forceinline__ double p_hpsi(const PackMember &m, const V *psi, V *s
     return t;
 }
 
-// CTA x evaluates item x: parameter set params[x][0 .. nparam) of problem
-// items[x].x, with its gradient when items[x].y != 0.  Energy into energy[x],
-// gradient into grad[x][0 .. nparam); partial[x] holds the sweep's warp
-// partials ([max_rows][warps] per item).  The whole evaluation stays in
-// this CTA's shared memory: psi = U(t)|ref> (forward pair lists), sigma = H psi
-// from the H rows, the energy, the reverse sweep and the per-parameter sums,
-// so one launch serves parameter sets of different problems side by side.
+// One item's forward program: psi = U(t)|ref> in shared memory.
 template <class V>
-__global__ void __launch_bounds__(kPackThreads, 2) k_sector_pack(
-    const PackMember *__restrict__ members, const int2 *__restrict__ items, int maxparam,
-    const double *__restrict__ params, double *__restrict__ energy, double *__restrict__ grad,
-    double2 *__restrict__ partial, int max_rows, int nmem) {
-    extern __shared__ __align__(16) unsigned char s_raw[];
-    __shared__ double s_red[kPackThreads / 32];
-    const int2 it = items[blockIdx.x];
-    if ((unsigned)it.x >= (unsigned)nmem) {  // no such problem: NaN energy, nothing else
-        if (threadIdx.x == 0) energy[blockIdx.x] = __longlong_as_double(0x7ff8000000000000ll);
-        return;
-    }
-    const PackMember m = members[it.x];
-    const int tid = threadIdx.x, nth = blockDim.x, nw = nth >> 5;
-    V *psi = reinterpret_cast<V *>(s_raw), *sig = psi + m.nsec;
-    PSmem<V> *s_pr = reinterpret_cast<PSmem<V> *>(s_raw + ((sizeof(V) * 2 * m.nsec + 15) & ~(size_t)15));
-    const double *par = params + (size_t)blockIdx.x * maxparam;
+__device__ __forceinline__ void pack_forward(const PackMember &m, const double *par, V *psi,
+                                             PCoef<false, V> *cf) {
+    const int tid = threadIdx.x, nth = blockDim.x;
     for (int i = tid; i < m.nsec; i += nth) psi[i] = i == m.ref_i ? v_one_of<V>() : v_zero(V());
-    p_angles(m.fwd, par, 1, s_pr);
+    step_pad(psi, m.nsec);
+    p_angles<false, V>(m.fwd, par, 1, cf);
     __syncthreads();
-    p_run<false, V>(m.fwd, s_pr, psi, (V *)nullptr, nullptr, 1, 0);
+    p_forward<false, V>(m.fwd, cf, psi);
     __syncthreads();
-    const double e = p_hpsi<V>(m, psi, sig, s_red);
-    if (tid == 0) energy[blockIdx.x] = e;
-    if (!it.y || m.nparam == 0) return;
-    __syncthreads();  // every thread is done with the forward angles and sigma
-    p_angles(m.sweep, par, -1, s_pr);
+}
+
+// One item's reverse sweep on psi and sig (save buffer) and its gradient.
+template <class V>
+__device__ __forceinline__ void pack_sweep(const PackLaunch &P, const PackMember &m, const double *par,
+                                           const V *psi, const V *sig, unsigned char *raw) {
+    SweepState<V> st(raw, m.nsec);
+    PCoef<true, V> *cf = step_coef<PCoef<true, V>>(raw, 2, m.nsec, sizeof(V));
+    sweep_load(st, psi, sig, m.nsec);
+    p_angles<true, V>(m.sweep, par, -1, cf);
     __syncthreads();
-    double2 *pp = partial + (size_t)blockIdx.x * max_rows * nw;
-    p_run<true, V>(m.sweep, s_pr, psi, sig, pp, 1, 0);
+    double *pp = P.partial + (size_t)blockIdx.x * P.maxpart;
+    p_sweep<V>(m.sweep, cf, st, pp);
     __syncthreads();  // this CTA's partials are visible to all its threads
-    double *g = grad + (size_t)blockIdx.x * maxparam;
-    for (int mu = tid; mu < m.nparam; mu += nth) {
-        const int2 r = m.psteps[mu];
-        double acc = 0.0;
-        for (int s = r.x; s < r.y; ++s)
-            for (int c = 0; c < nw; ++c) acc += pp[(size_t)s * nw + c].x;
-        g[mu] = 2.0 * acc;
+    p_grad(m.prange, m.nparam, m.sweep.nth >> 5, pp, P.grad + (size_t)blockIdx.x * P.maxparam);
+}
+
+// The item of CTA x, or nothing for a number that is no problem's (its energy
+// is NaN).
+__device__ __forceinline__ bool pack_item(const PackLaunch &P, int x, int2 &it) {
+    it = P.items[x];
+    if ((unsigned)it.x < (unsigned)P.nmem) return true;
+    if (threadIdx.x == 0) P.energy[x] = __longlong_as_double(0x7ff8000000000000ll);
+    return false;
+}
+
+// Item x is parameter set params[x][0 .. nparam) of problem items[x].x, with its
+// gradient when items[x].y != 0; energy into energy[x], gradient into
+// grad[x][0 .. nparam).  Three launches serve parameter sets of different
+// problems side by side: the forward programs (a CTA per item), sigma = H psi
+// and the energies (Q CTAs per item: one alone takes ~400 us for the 1.8 M row
+// entries of a 16-qubit problem), the reverse sweeps (a CTA per item).
+template <class V>
+__global__ void __launch_bounds__(kStepThreads, 2) k_pack_forward(PackLaunch P) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    int2 it;
+    if (!pack_item(P, blockIdx.x, it)) return;
+    const PackMember m = P.members[it.x];
+    V *psi = reinterpret_cast<V *>(s_raw);
+    pack_forward<V>(m, P.params + (size_t)blockIdx.x * P.maxparam, psi,
+                    step_coef<PCoef<false, V>>(s_raw, 1, m.nsec, sizeof(V)));
+    V *sv = reinterpret_cast<V *>(P.save) + (size_t)blockIdx.x * 2 * P.maxsec;
+    for (int i = threadIdx.x; i < m.nsec; i += blockDim.x) sv[i] = psi[i];
+}
+
+// CTA (q, x): row slice q of item x's sigma and its share of the energy; the
+// CTA that finishes an item last (a ticket, which it resets) adds the shares
+// in order.
+template <class V>
+__global__ void __launch_bounds__(kStepThreads, 2) k_pack_h(PackLaunch P) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    __shared__ double s_red[kStepThreads / 32];
+    const int x = blockIdx.y, q = blockIdx.x, tid = threadIdx.x;
+    const int2 it = P.items[x];
+    if ((unsigned)it.x >= (unsigned)P.nmem) return;
+    const PackMember m = P.members[it.x];
+    V *psi = reinterpret_cast<V *>(s_raw);
+    V *sv = reinterpret_cast<V *>(P.save) + (size_t)x * 2 * P.maxsec;
+    for (int i = tid; i < m.nsec; i += blockDim.x) psi[i] = sv[i];
+    __syncthreads();
+    const int r0 = (int)((int64_t)q * m.nsec / P.Q), r1 = (int)((int64_t)(q + 1) * m.nsec / P.Q);
+    const double e = p_hpsi<V>(m, r0, r1, psi, sv + P.maxsec, s_red);
+    if (tid == 0) {
+        P.epart[(size_t)x * P.Q + q] = e;
+        __threadfence();
+        if (atomicAdd(&P.count[x], 1u) == (unsigned)P.Q - 1u) {
+            __threadfence();
+            double t = 0.0;
+            for (int k = 0; k < P.Q; ++k) t += __ldcg(&P.epart[(size_t)x * P.Q + k]);
+            P.energy[x] = t;
+            P.count[x] = 0u;
+        }
     }
 }
 
-// Shared-memory bytes of the kernels for a sector of nsec amplitudes:
-// states, then the record angles, then the record ring.
+template <class V>
+__global__ void __launch_bounds__(kStepThreads, sizeof(V) == sizeof(double) ? 2 : 1) k_pack_sweep(PackLaunch P) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    const int2 it = P.items[blockIdx.x];
+    if ((unsigned)it.x >= (unsigned)P.nmem || !it.y) return;
+    const PackMember m = P.members[it.x];
+    if (m.nparam == 0) return;
+    const V *sv = reinterpret_cast<const V *>(P.save) + (size_t)blockIdx.x * 2 * P.maxsec;
+    pack_sweep<V>(P, m, P.params + (size_t)blockIdx.x * P.maxparam, sv, sv + P.maxsec, s_raw);
+}
+
+// Shared-memory bytes of nstates states of nsec amplitudes.
 inline size_t sector_smem_states(size_t nstates, size_t nsec, bool real) {
     return ((nstates * nsec * (real ? 8 : 16)) + 15) & ~(size_t)15;
 }

@@ -28,6 +28,10 @@
 namespace qfbv {
 
 using qfbg::GLaunch;
+using qfbs::v_flip;
+using qfbs::v_ip_re;
+using qfbs::v_of;
+using qfbs::v_rot;
 
 constexpr int kWinItems = 192;    // items of a window
 constexpr int kWinIdx = 12;       // bits of a local string or amplitude index
@@ -109,28 +113,6 @@ __global__ void __launch_bounds__(256) k_win_angles(const double *__restrict__ g
     double sn, cs;
     sincos(gamma[i] * params[(size_t)s * nparam + param[i]], &sn, &cs);
     ang[t] = make_double2(cs, sn);
-}
-
-// Re of conj(w0) h v1 + conj(w1) g v0
-__device__ __forceinline__ double v_ip_re(double w0, double w1, double v0, double v1, double g, double h) {
-    return w0 * (h * v1) + w1 * (g * v0);
-}
-__device__ __forceinline__ double v_ip_re(double2 w0, double2 w1, double2 v0, double2 v1, double2 g, double2 h) {
-    const double2 a = qfbs::s_cmul(h, v1), b = qfbs::s_cmul(g, v0);
-    return (w0.x * a.x + w0.y * a.y) + (w1.x * b.x + w1.y * b.y);
-}
-__device__ __forceinline__ double v_of(double, double2 z, double f) { return z.x * f; }
-__device__ __forceinline__ double2 v_of(double2, double2 z, double f) { return make_double2(z.x * f, z.y * f); }
-// c x + a y, the product negated when bit 31 of w is set
-__device__ __forceinline__ double v_flip(double a, uint32_t w) {
-    return __hiloint2double(__double2hiint(a) ^ (int)(w & 0x80000000u), __double2loint(a));
-}
-__device__ __forceinline__ double2 v_flip(double2 a, uint32_t w) {
-    return make_double2(v_flip(a.x, w), v_flip(a.y, w));
-}
-__device__ __forceinline__ double v_rot(double c, double x, double a, double y) { return c * x + a * y; }
-__device__ __forceinline__ double2 v_rot(double c, double2 x, double2 a, double2 y) {
-    return make_double2(c * x.x + (a.x * y.x - a.y * y.y), c * x.y + (a.x * y.y + a.y * y.x));
 }
 
 // Apply window W to every block and slot.  grid = (blocks, slot groups);
