@@ -291,86 +291,134 @@ __global__ void __launch_bounds__(256) k_sum_apply4(
     }
 }
 
-// dst = O src over output tiles in shared memory, several states per block.
-// Block (t, c) owns outputs k = t * 2^m + tid (one per thread) of states
-// c * NB .. c * NB + NB - 1.  Groups are visited ordered by their high part
-// x >> m: for each distinct high part the block stages the partner tile
-// (the 2^m inputs k ^ x of its outputs for every x with that high part) of
-// its NB states once, then every group of that high part reads its inputs
-// from shared memory.  f_x(k ^ x) depends on k and x only, so it is computed
-// once and applied to all NB states.
-constexpr int kApplyTileBits = 8;
-constexpr int kApplyStates = 16;
-
-// IDX = uint32_t when the state has at most 32 qubits (one popcount per term).
-template <typename IDX>
-__global__ void __launch_bounds__(1 << kApplyTileBits, 2) k_sum_apply_tiled(
-    double2 *__restrict__ dst, const double2 *__restrict__ src, uint64_t nbasis, int nbatch,
-    int m, const GroupDev *__restrict__ groups, const int32_t *__restrict__ hi_g0,
-    const uint64_t *__restrict__ hi_val, int nhi, const TermDev *__restrict__ terms,
-    const double2 *__restrict__ rterms) {
-    extern __shared__ double2 apply_smem[];
-    double2(*tile)[1 << kApplyTileBits] = reinterpret_cast<double2(*)[1 << kApplyTileBits]>(apply_smem);
-    const int T = 1 << m;
-    const int tid = threadIdx.x;
-    const uint64_t kbase = (uint64_t)blockIdx.x << m;
-    const int s0 = blockIdx.y * kApplyStates;
-    const int ns = min(kApplyStates, nbatch - s0);
-    const IDX k = (IDX)(kbase + tid);
-    double2 acc[kApplyStates];
+// dst = O src (DOT: <bra|O|src> instead), states of 8 qubits and more: 2^8
+// outputs a block, the groups dealt to its 8 warps.  A group's coefficient on output k, d its bits
+// 2-4, is the sum over its terms of
+//     (-1)^popcount(d & z's bits 2-4)  c (-1)^popcount(((k with d = 0) ^ x) & z):
+// an 8 x terms matrix of signs times a terms x 32 matrix of signed coefficients,
+// done on the FP64 matrix units four terms at a time.  So a warp takes one parity
+// per term and 8 outputs, and branches only where a group ends.  The columns are
+// numbered so that a lane's accumulators belong to outputs lane + 32 q: whole
+// 512-byte runs, L1-resident while the groups' high part x >> 8 stays.  Groups
+// are padded to blocks of four terms; a warp stages eight blocks at a time, the
+// next eight on their way from L2 meanwhile, and loads a group's amplitudes while
+// its coefficients are formed.
+//
+// A molecular H, us, one parity per output and term / this kernel: 16 qubits
+// (981 groups, 5,793 terms) 1 state 762 / 88, 64 states 6,033 / 4,496; 12 qubits
+// 206 / 20 and 314 / 98; <psi|H|psi> group by group (k_sum_expval) / this kernel:
+// 16 qubits 1 state 492 / 84; 12 qubits 20.4 / 18.0; 8 qubits 3.7 / 5.4.
+constexpr int kSumTileBits = 8;
+constexpr int kSumWarps = 8;
+constexpr int kSumAhead = 8;  // blocks a warp stages (four terms each: one a lane)
+struct SumBlock {  // of four terms
+    uint64_t x;
+    uint32_t fl;  // bit 0: first of its group, 1: last, 2: the coefficients are imaginary parts
+    uint32_t pad;
+};
+template <bool DOT, typename IDX>
+__global__ void __launch_bounds__(32 * kSumWarps, 2) k_sum_tile(
+    double2 *__restrict__ dst, const double2 *__restrict__ bra, const double2 *__restrict__ src,
+    uint64_t nbasis, const SumBlock *__restrict__ blocks, const double2 *__restrict__ terms,
+    const int32_t *__restrict__ slice, double2 *__restrict__ partial) {
+    __shared__ double2 s_acc[kSumWarps][256];
+    __shared__ double2 s_term[kSumWarps][4 * kSumAhead];
+    __shared__ uint4 s_block[kSumWarps][kSumAhead];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = lane >> 2, col = lane & 3;
+    const uint64_t off = (uint64_t)blockIdx.y * nbasis;
+    const int b0 = slice[warp], b1 = slice[warp + 1];
+    double2 dot = make_double2(0.0, 0.0);
+    for (uint64_t tile = blockIdx.x; tile < nbasis >> 8; tile += gridDim.x) {
+        const IDX kb = (IDX)(tile << 8);
+        double2 acc[8], a[8];
+        double f[8];
 #pragma unroll
-    for (int s = 0; s < kApplyStates; ++s) acc[s] = make_double2(0.0, 0.0);
-    for (int r = 0; r < nhi; ++r) {
-        const uint64_t jbase = kbase ^ (hi_val[r] << m);
-        __syncthreads();
-        for (int s = 0; s < ns; ++s)
-            for (int l = tid; l < T; l += blockDim.x)
-                tile[s][l] = src[(uint64_t)(s0 + s) * nbasis + jbase + l];
-        __syncthreads();
-        if (tid >= T) continue;
-        for (int g = hi_g0[r]; g < hi_g0[r + 1]; ++g) {
-            const GroupDev gr = groups[g];
-            const IDX j = k ^ (IDX)gr.x;
-            const int lj = (int)(j & (IDX)(T - 1));
-            if (gr.real) {
-                double f = 0.0;
-#pragma unroll 4
-                for (int t = gr.begin; t < gr.end; ++t) {
-                    const double2 zc = __ldg(&rterms[t]);
-                    const IDX z = (IDX)__double_as_longlong(zc.x);
-                    const int odd = (sizeof(IDX) == 4) ? (__popc((uint32_t)(j & z)) & 1)
-                                                       : parity64((uint64_t)(j & z));
-                    f += odd ? -zc.y : zc.y;
+        for (int q = 0; q < 8; ++q) acc[q] = a[q] = make_double2(0.0, 0.0), f[q] = 0.0;
+        // (the arrays hold 2 kSumAhead unused blocks at their end)
+        uint4 nb = __ldg(reinterpret_cast<const uint4 *>(blocks + b0) + (lane & (kSumAhead - 1)));
+        double2 nt = __ldg(terms + 4 * (size_t)b0 + lane);
+        for (int b = b0; b < b1; ++b) {
+            const int at = (b - b0) & (kSumAhead - 1);
+            if (at == 0) {
+                __syncwarp();
+                s_block[warp][lane & (kSumAhead - 1)] = nb;
+                s_term[warp][lane] = nt;
+                __syncwarp();
+                nb = __ldg(reinterpret_cast<const uint4 *>(blocks + b) + kSumAhead + (lane & (kSumAhead - 1)));
+                nt = __ldg(terms + 4 * (size_t)(b + kSumAhead) + lane);
+            }
+            const uint4 bl = s_block[warp][at];
+            const double2 zc = s_term[warp][4 * at + col];
+            const IDX x = sizeof(IDX) == 4 ? (IDX)bl.x : (IDX)((uint64_t)bl.y << 32 | bl.x);
+            if (bl.z & 1u) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    a[q] = __ldg(&src[off + (uint64_t)((kb | (IDX)(q << 5 | lane)) ^ x)]);
                 }
+            }
+            const IDX z = (IDX)__double_as_longlong(zc.x);
+            // column c of matrix product n is output bits 0-1 = c / 2, bit 5 = c % 2,
+            // bits 6-7 = n
+            const IDX in = (kb ^ x ^ (IDX)(row >> 1 | (row & 1) << 5)) & z;
+            const uint32_t zl = (uint32_t)z;
+            const uint32_t s0 = sizeof(IDX) == 4 ? (uint32_t)__popc((uint32_t)in) : (uint32_t)__popcll((uint64_t)in);
+            const uint32_t s1 = s0 ^ zl >> 6, s2 = s0 ^ zl >> 7, s3 = s1 ^ zl >> 7;
+            const double sa = __hiloint2double(0x3ff00000 | (int)((uint32_t)__popc((zl >> 2) & row) << 31), 0);
+            const int hi = __double2hiint(zc.y), lo = __double2loint(zc.y);
+            auto mma = [&](int n, uint32_t sg) {
+                const double c = __hiloint2double(hi ^ (int)(sg << 31), lo);
+                asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                    : "+d"(f[2 * n]), "+d"(f[2 * n + 1])
+                    : "d"(sa), "d"(c));
+            };
+            mma(0, s0);
+            mma(1, s1);
+            mma(2, s2);
+            mma(3, s3);
+            if (bl.z & 2u) {
+                if (bl.z & 4u) {
 #pragma unroll
-                for (int s = 0; s < kApplyStates; ++s) {
-                    if (s < ns) {
-                        const double2 a = tile[s][lj];
-                        acc[s].x += f * a.x;
-                        acc[s].y += f * a.y;
+                    for (int q = 0; q < 8; ++q) {
+                        acc[q].x -= f[q] * a[q].y;
+                        acc[q].y += f[q] * a[q].x;
+                        f[q] = 0.0;
+                    }
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        acc[q].x += f[q] * a[q].x;
+                        acc[q].y += f[q] * a[q].y;
+                        f[q] = 0.0;
                     }
                 }
-            } else {
-                double2 f = make_double2(0.0, 0.0);
-                for (int t = gr.begin; t < gr.end; ++t) {
-                    const double2 c = terms[t].c;
-                    if (parity64((uint64_t)j & __ldg(&terms[t].z))) { f.x -= c.x; f.y -= c.y; }
-                    else { f.x += c.x; f.y += c.y; }
-                }
-#pragma unroll
-                for (int s = 0; s < kApplyStates; ++s)
-                    if (s < ns) acc[s] = c_add(acc[s], c_mul(f, tile[s][lj]));
             }
         }
-    }
-    if (tid < T) {
+        __syncthreads();  // the tile before has been summed
 #pragma unroll
-        for (int s = 0; s < kApplyStates; ++s)
-            if (s < ns) dst[(uint64_t)(s0 + s) * nbasis + (uint64_t)k] = acc[s];
+        for (int q = 0; q < 8; ++q) s_acc[warp][q << 5 | lane] = acc[q];
+        __syncthreads();
+        double2 t = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int w = 0; w < kSumWarps; ++w) t = c_add(t, s_acc[w][threadIdx.x]);
+        const uint64_t k = off + (tile << 8) + threadIdx.x;
+        if (DOT)
+            dot = c_add(dot, c_cjmul(bra[k], t));
+        else
+            dst[k] = t;
+    }
+    if (DOT) {
+        dot = block_sum(dot);
+        if (threadIdx.x == 0) partial[(uint64_t)blockIdx.y * gridDim.x + blockIdx.x] = dot;
     }
 }
 
-constexpr size_t kApplySmem = sizeof(double2) * kApplyStates * (1 << kApplyTileBits);
+// out[b] = sum of n partials of slot b
+__global__ void k_part_sum(const double2 *__restrict__ partial, int n, double2 *__restrict__ out) {
+    double2 acc = make_double2(0.0, 0.0);
+    for (int k = threadIdx.x; k < n; k += blockDim.x) acc = c_add(acc, partial[(size_t)blockIdx.x * n + k]);
+    acc = block_sum(acc);
+    if (threadIdx.x == 0) out[blockIdx.x] = acc;
+}
 
 // One x-group of a Hamiltonian restricted to a particle-number sector: an
 // output index k of the sector reaches k ^ x inside the sector exactly when k
@@ -868,13 +916,13 @@ __global__ void k_set_ref(double2 *__restrict__ psi, uint64_t nbasis, uint64_t r
 // host objects
 // ===========================================================================
 
-// Groups ordered by their high part x >> m, for k_sum_apply_tiled.
-struct TiledView {
-    int m = 0, nhi = 0;
+// A sum as k_sum_tile reads it: its groups ordered by their high part x >> 8,
+// their terms in blocks of four, the warps' blocks.
+struct SumTiles {
     void *blob = nullptr;
-    GroupDev *d_groups = nullptr;
-    int32_t *d_hi0 = nullptr;
-    uint64_t *d_hival = nullptr;
+    SumBlock *blocks = nullptr;
+    double2 *terms = nullptr;
+    int32_t *slice = nullptr;
 };
 
 // H rows on a particle-number sector and compact plans (defined with the
@@ -888,13 +936,10 @@ struct qfb_sum_s {
     int64_t nterms = 0;
     int32_t ngroups = 0;
     int32_t nsegment = 0;
-    TiledView *tiled[kApplyTileBits + 1] = {nullptr};
+    SumTiles *tiles = nullptr;  // ensure_tiles
     ~qfb_sum_s() {
-        for (auto *t : tiled)
-            if (t) {
-                dev_free(t->blob);
-                delete t;
-            }
+        if (tiles) dev_free(tiles->blob);
+        delete tiles;
     }
     void *blob = nullptr;  // device: groups, terms, segment starts
     GroupDev *d_groups = nullptr;
@@ -1462,11 +1507,35 @@ static void make_table(qfb_prog_s *p, StepDev &st) {
     }
 }
 
+// Blocks of k_sum_tile per state.
+static unsigned tile_grid(uint64_t nbasis) {
+    return (unsigned)std::min<uint64_t>(nbasis >> kSumTileBits, 16 * (uint64_t)sm_count());
+}
+
+template <bool DOT>
+static int launch_tiles(const qfb_sum_s *h, double2 *dst, const double2 *bra, const double2 *src,
+                        uint64_t nbasis, int B, double2 *partial) {
+    const SumTiles &tv = *h->tiles;
+    for (int b = 0; b < B; b += 65535) {  // grid.y's limit
+        const dim3 grid(tile_grid(nbasis), (unsigned)std::min(65535, B - b));
+        const uint64_t at = (uint64_t)b * nbasis;
+        double2 *part = DOT ? partial + (size_t)b * grid.x : nullptr;
+        if (nbasis <= 1ull << 32)
+            k_sum_tile<DOT, uint32_t><<<grid, 32 * kSumWarps, 0, t_stream>>>(
+                DOT ? nullptr : dst + at, DOT ? bra + at : nullptr, src + at, nbasis, tv.blocks, tv.terms, tv.slice, part);
+        else
+            k_sum_tile<DOT, uint64_t><<<grid, 32 * kSumWarps, 0, t_stream>>>(
+                DOT ? nullptr : dst + at, DOT ? bra + at : nullptr, src + at, nbasis, tv.blocks, tv.terms, tv.slice, part);
+        QFB_LAUNCHED();
+    }
+    return QFB_OK;
+}
+
 extern "C" {
 
 static int enqueue_sum_apply(const qfb_sum_s *h, double2 *dst, const double2 *src,
                              uint64_t nbasis, int B);
-static int ensure_tiled(qfb_sum_s *h, int nqubit);
+static int ensure_tiles(qfb_sum_s *h, int nqubit);
 
 int qfb_sum_create(const qfb_pauli *paulis, const qfb_complex *coeffs, const int32_t *segment,
                    int64_t nterms, int32_t nsegment, qfb_sum *out) {
@@ -1608,15 +1677,29 @@ int qfb_sum_expval(qfb_sum h, qfb_state bra, qfb_state ket, qfb_complex *out) {
         for (size_t i = 0; i < nout; ++i) out[i] = qfb_complex{0.0, 0.0};
         return QFB_OK;
     }
+    // one sum over all groups: by outputs, where there are enough of them
+    const bool tv = h->nsegment == 1 && h->ngroups <= 65535 && bra->nqubit >= kSumTileBits &&
+                    bra->nbasis * (uint64_t)B >= 4096;
+    int rc = tv ? ensure_tiles(h, bra->nqubit) : QFB_OK;
+    if (rc) return rc;
     const uint64_t npair = bra->nbasis >> 1;
-    const unsigned chunks = chunks_for(npair, B, h->ngroups);
-    const size_t nparts = (size_t)B * h->ngroups * chunks;
+    const unsigned chunks = tv ? tile_grid(bra->nbasis) : chunks_for(npair, B, h->ngroups);
+    const size_t nparts = (size_t)B * (tv ? 1 : h->ngroups) * chunks;
     void *buf = nullptr;
-    int rc = dev_alloc(&buf, sizeof(double2) * (nparts + nout));
+    rc = dev_alloc(&buf, sizeof(double2) * (nparts + nout));
     if (rc) return rc;
     double2 *partial = (double2 *)buf;
     double2 *res = partial + nparts;
-    for (int32_t g0 = 0; g0 < h->ngroups; g0 += 65535) {
+    if (tv) {
+        rc = launch_tiles<true>(h, nullptr, bra->d, ket->d, bra->nbasis, B, partial);
+        if (rc) {
+            dev_free(buf);
+            return rc;
+        }
+        k_part_sum<<<B, 256, 0, t_stream>>>(partial, (int)chunks, res);
+        QFB_LAUNCHED();
+    }
+    for (int32_t g0 = 0; !tv && g0 < h->ngroups; g0 += 65535) {
         // grid.y is limited to 65535 groups per launch
         const int32_t ng = std::min<int32_t>(65535, h->ngroups - g0);
         if (g0 == 0 && ng == h->ngroups) {
@@ -1628,9 +1711,11 @@ int qfb_sum_expval(qfb_sum h, qfb_state bra, qfb_state ket, qfb_complex *out) {
             return fail(QFB_ENOSYS, "qfb_sum_expval: more than 65535 x-groups");
         }
     }
-    k_seg_sum<<<dim3(h->nsegment, B), 256, 0, t_stream>>>(partial, h->d_seg_g0, h->ngroups,
-                                                          chunks, res);
-    QFB_LAUNCHED();
+    if (!tv) {
+        k_seg_sum<<<dim3(h->nsegment, B), 256, 0, t_stream>>>(partial, h->d_seg_g0, h->ngroups,
+                                                              chunks, res);
+        QFB_LAUNCHED();
+    }
     QFB_CUDA(cudaMemcpyAsync(out, res, sizeof(double2) * nout, cudaMemcpyDeviceToHost, t_stream));
     dev_free(buf);
     QFB_CUDA(cudaStreamSynchronize(t_stream));
@@ -1646,7 +1731,7 @@ int qfb_sum_apply(qfb_sum h, qfb_state dst, qfb_state src) {
         if (g.h >= src->nqubit)
             return fail(QFB_EINVAL, "qfb_sum_apply: operator acts on qubit %d of a %d-qubit state",
                         g.h, src->nqubit);
-    int rc = ensure_tiled(h, src->nqubit);
+    int rc = ensure_tiles(h, src->nqubit);
     if (rc) return rc;
     return enqueue_sum_apply(h, dst->d, src->d, src->nbasis, src->nbatch);
 }
@@ -1804,92 +1889,76 @@ static int enqueue_prog(const qfb_prog_s *p, double2 *psi, int nqubit, int B,
     return QFB_OK;
 }
 
-static int tile_bits_for(int nqubit) { return std::min(kApplyTileBits, nqubit); }
 
-static int ensure_tiled(qfb_sum_s *h, int nqubit) {
-    const int m = tile_bits_for(nqubit);
-    if (h->tiled[m]) return QFB_OK;
-    static std::once_flag smem_once;
-    static cudaError_t smem_err = cudaSuccess;
-    std::call_once(smem_once, [] {
-        smem_err = cudaFuncSetAttribute(k_sum_apply_tiled<uint32_t>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kApplySmem);
-        if (smem_err == cudaSuccess)
-            smem_err = cudaFuncSetAttribute(k_sum_apply_tiled<uint64_t>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)kApplySmem);
+static int ensure_tiles(qfb_sum_s *h, int nqubit) {
+    if (nqubit < kSumTileBits) return QFB_OK;
+    // sums are shared between threads
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    if (h->tiles) return QFB_OK;
+    std::vector<GroupDev> gs = h->h_groups;
+    std::stable_sort(gs.begin(), gs.end(), [](const GroupDev &a, const GroupDev &b) {
+        return (a.x >> kSumTileBits) < (b.x >> kSumTileBits);
     });
-    if (smem_err != cudaSuccess) return cuda_fail(smem_err, "tiled apply shared memory");
-    std::vector<int32_t> order(h->h_groups.size());
-    for (size_t g = 0; g < order.size(); ++g) order[g] = (int32_t)g;
-    std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) {
-        return (h->h_groups[a].x >> m) < (h->h_groups[b].x >> m);
-    });
-    std::vector<GroupDev> gs;
-    std::vector<int32_t> hi0;
-    std::vector<uint64_t> hiv;
-    for (size_t i = 0; i < order.size(); ++i) {
-        const GroupDev &g = h->h_groups[order[i]];
-        const uint64_t hi = g.x >> m;
-        if (hiv.empty() || hiv.back() != hi) {
-            hiv.push_back(hi);
-            hi0.push_back((int32_t)i);
+    // real and imaginary parts apart
+    std::vector<SumBlock> fb;
+    std::vector<double2> ft;
+    for (const GroupDev &g : gs)
+        for (int part = 0; part < (g.real ? 1 : 2); ++part)
+            for (int t = g.begin; t < g.end; t += 4) {
+                fb.push_back(SumBlock{g.x, (t == g.begin ? 1u : 0u) | (t + 4 >= g.end ? 2u : 0u) | (part ? 4u : 0u), 0});
+                for (int k = t; k < t + 4; ++k) {
+                    double2 zc = make_double2(0.0, 0.0);
+                    if (k < g.end) {
+                        std::memcpy(&zc.x, &h->h_terms[(size_t)k].z, sizeof(double));
+                        zc.y = part ? h->h_terms[(size_t)k].c.y : h->h_terms[(size_t)k].c.x;
+                    }
+                    ft.push_back(zc);
+                }
+            }
+    // the warps take consecutive groups of about equal work: a block about 30
+    // instructions, a group's amplitudes about 45
+    std::vector<int32_t> slice(kSumWarps + 1, (int32_t)fb.size());
+    {
+        auto cost = [](const SumBlock &b) { return (int64_t)(30 + (b.fl & 1u ? 45 : 0)); };
+        int64_t all = 0, at = 0;
+        for (const SumBlock &b : fb) all += cost(b);
+        slice[0] = 0;
+        int w = 1;
+        for (size_t i = 0; i < fb.size(); ++i) {
+            at += cost(fb[i]);
+            if (fb[i].fl & 2u)
+                while (w < kSumWarps && at * kSumWarps >= all * w) slice[(size_t)w++] = (int32_t)i + 1;
         }
-        gs.push_back(g);
     }
-    hi0.push_back((int32_t)gs.size());
+    fb.resize(fb.size() + 2 * kSumAhead, SumBlock{0, 0, 0});
+    ft.resize(ft.size() + 8 * kSumAhead, make_double2(0.0, 0.0));
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-    const size_t gb = al(sizeof(GroupDev) * std::max<size_t>(1, gs.size()));
-    const size_t hb = al(sizeof(int32_t) * hi0.size());
-    const size_t vb = sizeof(uint64_t) * std::max<size_t>(1, hiv.size());
-    TiledView *tv = new TiledView;
-    tv->m = m;
-    tv->nhi = (int)hiv.size();
-    int rc = dev_alloc(&tv->blob, gb + hb + vb);
-    if (rc) {
-        delete tv;
-        return rc;
-    }
-    tv->d_groups = (GroupDev *)tv->blob;
-    tv->d_hi0 = (int32_t *)((char *)tv->blob + gb);
-    tv->d_hival = (uint64_t *)((char *)tv->blob + gb + hb);
-    cudaError_t e = cudaSuccess;
-    if (!gs.empty())
-        e = cudaMemcpyAsync(tv->d_groups, gs.data(), sizeof(GroupDev) * gs.size(),
-                            cudaMemcpyHostToDevice, t_stream);
+    const size_t bb = al(sizeof(SumBlock) * fb.size()), bt = al(sizeof(double2) * ft.size());
+    const size_t bs = sizeof(int32_t) * slice.size();
+    auto tv = std::make_unique<SumTiles>();
+    int rc = dev_alloc(&tv->blob, bb + bt + bs);
+    if (rc) return rc;
+    tv->blocks = (SumBlock *)tv->blob;
+    tv->terms = (double2 *)((char *)tv->blob + bb);
+    tv->slice = (int32_t *)((char *)tv->blob + bb + bt);
+    cudaError_t e = cudaMemcpyAsync(tv->blocks, fb.data(), sizeof(SumBlock) * fb.size(), cudaMemcpyHostToDevice, t_stream);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(tv->d_hi0, hi0.data(), sizeof(int32_t) * hi0.size(),
-                            cudaMemcpyHostToDevice, t_stream);
-    if (e == cudaSuccess && !hiv.empty())
-        e = cudaMemcpyAsync(tv->d_hival, hiv.data(), sizeof(uint64_t) * hiv.size(),
-                            cudaMemcpyHostToDevice, t_stream);
+        e = cudaMemcpyAsync(tv->terms, ft.data(), sizeof(double2) * ft.size(), cudaMemcpyHostToDevice, t_stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(tv->slice, slice.data(), bs, cudaMemcpyHostToDevice, t_stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(t_stream);
     if (e != cudaSuccess) {
         dev_free(tv->blob);
-        delete tv;
-        return cuda_fail(e, "tiled group view upload");
+        return cuda_fail(e, "sum tiles upload");
     }
-    h->tiled[m] = tv;
+    h->tiles = tv.release();
     return QFB_OK;
 }
 
 static int enqueue_sum_apply(const qfb_sum_s *h, double2 *dst, const double2 *src,
                              uint64_t nbasis, int B) {
-    const int nq = 63 - __builtin_clzll(nbasis);
-    const TiledView *tv = h->tiled[tile_bits_for(nq)];
-    if (tv && h->ngroups > 0) {
-        const dim3 grid((unsigned)(nbasis >> tv->m), (unsigned)((B + kApplyStates - 1) / kApplyStates));
-        if (nq <= 32)
-            k_sum_apply_tiled<uint32_t><<<grid, 1 << kApplyTileBits, kApplySmem, t_stream>>>(
-                dst, src, nbasis, B, tv->m, tv->d_groups, tv->d_hi0, tv->d_hival, tv->nhi,
-                h->d_terms, h->d_rterms);
-        else
-            k_sum_apply_tiled<uint64_t><<<grid, 1 << kApplyTileBits, kApplySmem, t_stream>>>(
-                dst, src, nbasis, B, tv->m, tv->d_groups, tv->d_hi0, tv->d_hival, tv->nhi,
-                h->d_terms, h->d_rterms);
-        QFB_LAUNCHED();
-        return QFB_OK;
-    }
+    if (h->tiles && nbasis >> kSumTileBits)
+        return launch_tiles<false>(h, dst, nullptr, src, nbasis, B, nullptr);
     if (nbasis >= 4) {
         const dim3 grid(grid_for(nbasis >> 2, 256), B);
         k_sum_apply4<<<grid, 256, 0, t_stream>>>(dst, src, nbasis, h->d_groups, h->d_terms,
@@ -4243,7 +4312,7 @@ static int ucc_create_impl(qfb_prog fprog, qfb_prog gprog, qfb_prog uprog, qfb_s
         for (const auto &sd : p->h_strs)
             if (sd.z >> nqubit) return fail(QFB_EINVAL, "qfb_ucc_create: program beyond qubit");
     }
-    int prc = ensure_tiled(ham, nqubit);
+    int prc = ensure_tiles(ham, nqubit);
     if (prc == QFB_OK) prc = ensure_plans(fprog, nqubit, true);
     if (prc == QFB_OK && gprog) prc = ensure_plans(gprog, nqubit, false, uprog);
     if (prc) return prc;
