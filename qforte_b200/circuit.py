@@ -29,6 +29,12 @@ def _pauli_gate(letter, q):
     return g
 
 
+# Changes so far to circuits held as Pauli masks: while it stands still, every
+# circuit that holds masks holds the same ones (operators compiled from such
+# circuits compare it).
+_MASKS_DROPPED = [0]
+
+
 class Circuit:
     __slots__ = ("_g", "_pauli", "_pexp", "_plan")
 
@@ -56,6 +62,11 @@ class Circuit:
         return c
 
     # -- internal ---------------------------------------------------------
+    def _drop_masks(self):
+        if self._pauli is not None:
+            self._pauli = None
+            _MASKS_DROPPED[0] += 1
+
     def _gates(self):
         if self._g is None:
             x, z = self._pauli
@@ -64,7 +75,7 @@ class Circuit:
 
     def _edit(self):
         g = self._gates()
-        self._pauli = None
+        self._drop_masks()
         self._pexp = None
         self._plan = None
         return g
@@ -106,7 +117,7 @@ class Circuit:
 
     def add_gate(self, gate):
         g = self._gates()
-        self._pauli = None
+        self._drop_masks()
         self._plan = None
         g.append(gate)
 
@@ -118,7 +129,7 @@ class Circuit:
             segs = segs + [(s + n0, e + n0, x, z, th) for (s, e, x, z, th) in circ._pexp]
             self._pexp = segs
         g.extend(circ._gates())
-        self._pauli = None
+        self._drop_masks()
         self._plan = None
 
     def insert_gate(self, pos, gate):
@@ -210,7 +221,7 @@ class Circuit:
             raise RuntimeError("Circuit::set_parameters: number of parameters does not match "
                                "number of gates with parameters")
         self._g = out
-        self._pauli = None
+        self._drop_masks()
         self._pexp = None
         self._plan = None
 

@@ -287,9 +287,8 @@ class Computer:
     # ---- operators (computer.cc:80-91, :753-848) ---------------------------
     def apply_operator(self, qo):
         qo = _as_operator(qo)
-        pt = qo._pauli_terms(applied=True)
-        if pt is not None:
-            ds = sum_from_terms(pt)
+        ds = qo._device_sum()
+        if ds is not None:
             self._check_qubits(ds.maxbit)
             h = _new_state(self._n)
             try:
@@ -319,7 +318,9 @@ class Computer:
         self._swap_in(acc)
 
     def _expval_terms(self, terms, segments=None, nsegment=1):
-        ds = sum_from_terms(terms, segments, nsegment)
+        return self._expvals(sum_from_terms(terms, segments, nsegment), nsegment)
+
+    def _expvals(self, ds, nsegment=1):
         self._check_qubits(ds.maxbit)
         out = np.zeros(nsegment, dtype=np.complex128)
         check(lib().qfb_sum_expval(ds.h, self._h, self._h, ptr(out)), "expectation value")
@@ -327,9 +328,9 @@ class Computer:
 
     def direct_op_exp_val(self, qo):
         qo = _as_operator(qo)
-        pt = qo._pauli_terms(applied=True)
-        if pt is not None:
-            return complex(self._expval_terms(pt)[0])
+        ds = qo._device_sum()
+        if ds is not None:
+            return complex(self._expvals(ds)[0])
         tmp = Computer(self)
         tmp.apply_operator(qo)
         return inner_product(self, tmp)

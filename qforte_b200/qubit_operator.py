@@ -20,7 +20,7 @@ Circuits that are canonical Pauli strings are held in mask form throughout.
 
 import functools
 
-from .circuit import Circuit, _product_masks
+from .circuit import _MASKS_DROPPED, Circuit, _product_masks
 from .pauli import canonical_key, ipow_mul
 
 __all__ = ["QubitOperator", "to_string"]
@@ -37,11 +37,26 @@ def to_string(c):
     return f"{re:+.6f} {im:+.6f}i"
 
 
+class _Terms(list):
+    """An operator's [coeff, Circuit] entries, with what ``_device_sum`` made of
+    them (whoever shares the list shares that; copies and pickles start
+    without)."""
+
+    __slots__ = ("compiled",)
+
+    def __init__(self, *args):
+        super().__init__(*args)
+        self.compiled = None
+
+    def __reduce_ex__(self, protocol):
+        return _Terms, (list(self),)
+
+
 class QubitOperator:
     __slots__ = ("_t",)
 
     def __init__(self):
-        self._t = []  # [coeff, Circuit]
+        self._t = _Terms()  # [coeff, Circuit]
 
     # -- building (bindings.cc:95-116) ----------------------------------------
     def add(self, *args):
@@ -53,20 +68,24 @@ class QubitOperator:
     def add_term(self, coeff, circuit):
         if not isinstance(circuit, Circuit):
             raise TypeError("QubitOperator.add_term expects (complex, Circuit)")
+        self._t.compiled = None
         self._t.append([complex(coeff), circuit])
 
     def add_op(self, qo):
+        self._t.compiled = None
         for c, circ in qo._t:
             self._t.append([c, circ])
 
     def set_coeffs(self, new_coeffs):
         if len(new_coeffs) != len(self._t):
             raise ValueError("number of new coefficients for quantum operator must equal ")
+        self._t.compiled = None
         for t, c in zip(self._t, new_coeffs):
             t[0] = complex(c)
 
     def mult_coeffs(self, multiplier):
         m = complex(multiplier)
+        self._t.compiled = None
         for t in self._t:
             t[0] = t[0] * m
 
@@ -81,6 +100,7 @@ class QubitOperator:
 
     # -- algebra -----------------------------------------------------------------
     def canonical_order(self):
+        self._t.compiled = None
         for t in self._t:
             t[0] = t[0] * t[1].canonicalize_pauli_circuit()
 
@@ -95,9 +115,9 @@ class QubitOperator:
                 acc[key] = [c, circ]
         items = sorted(acc.items(), key=lambda kv: canonical_key(*kv[0]))
         if combine_like_terms:
-            self._t = [[v[0], v[1]] for _, v in items if abs(v[0]) > 1.0e-12]
+            self._t = _Terms([v[0], v[1]] for _, v in items if abs(v[0]) > 1.0e-12)
         else:
-            self._t = [[v[0], v[1]] for _, v in items]
+            self._t = _Terms([v[0], v[1]] for _, v in items)
 
     def operator_product(self, rqo, pre_simplify=True, post_simplify=True):
         if pre_simplify:
@@ -115,7 +135,7 @@ class QubitOperator:
                     # the reference multiplies the canonicalisation phase in
                     # afterwards (canonical_order); i^e products are exact
                     out.append([ipow_mul(cl * cr, e), Circuit._from_masks(x, z)])
-        self._t = out
+        self._t = _Terms(out)
         if post_simplify:
             self.simplify()
         else:
@@ -135,11 +155,12 @@ class QubitOperator:
                     return -1 if ga[k].gate_id() < gb[k].gate_id() else 1
             return 0
 
+        self._t.compiled = None
         self._t.sort(key=functools.cmp_to_key(cmp))
 
     def check_op_equivalence(self, qo, reorder):
         other = QubitOperator()
-        other._t = [[c, Circuit(circ)] for c, circ in qo._t]
+        other._t = _Terms([c, Circuit(circ)] for c, circ in qo._t)
         if reorder:
             self.order_terms()
             other.order_terms()
@@ -175,3 +196,23 @@ class QubitOperator:
             x, z, e = m
             out.append((ipow_mul(c, e), x, z))
         return out
+
+    def _device_sum(self):
+        """The operator each circuit applies in list order as a DeviceSum, or
+        None if a term holds a non-Pauli gate.  A molecular operator's thousands
+        of terms take milliseconds to gather, so the sum is kept until a method
+        changes the terms, or a circuit held as Pauli masks is changed (gate
+        lists are gathered on each call)."""
+        from .device import sum_from_terms
+
+        terms = self._t
+        kept, drops = terms.compiled, _MASKS_DROPPED[0]
+        if kept is not None and kept[1] == drops:
+            return kept[0]
+        pt = self._pauli_terms(applied=True)
+        if pt is None:
+            return None
+        ds = sum_from_terms(pt)
+        if all(circ._pauli is not None for _, circ in terms):
+            terms.compiled = (ds, drops)
+        return ds

@@ -17,7 +17,7 @@ in one pass over their terms.
 import functools
 
 from .circuit import Circuit
-from .qubit_operator import QubitOperator, to_string
+from .qubit_operator import QubitOperator, _Terms, to_string
 from .pauli import canonical_key, ipow_mul, pauli_mul
 
 __all__ = ["SQOperator"]
@@ -151,7 +151,7 @@ class SQOperator:
 
     def jw_transform(self, qubit_excitation=False):
         qo = QubitOperator()
-        qo._t = [[c, Circuit._from_masks(x, z)] for c, x, z in self._jw_masks(qubit_excitation)]
+        qo._t = _Terms([c, Circuit._from_masks(x, z)] for c, x, z in self._jw_masks(qubit_excitation))
         return qo
 
     def str(self):
