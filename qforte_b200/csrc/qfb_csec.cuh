@@ -177,6 +177,113 @@ __global__ void __launch_bounds__(256) k_cg_ip_many(GLaunch L, const uint4 *__re
     }
 }
 
+// Inner products of many independent records on one state.  A record's pattern
+// is an alpha list times a beta list; patterns whose alpha lists move the same strings
+// (their signs may differ) share rows: a CTA stages the two rows (psi and sigma
+// interleaved) of a few entries of one alpha list and works all the beta lists
+// that meet it against them, a warp per list, each list word read once for all
+// staged entries.  So the gathers of 8 bytes each from L2, one
+// per pair and amplitude, become 16-byte gathers from shared memory.
+//
+// Bound by those (two 16-byte loads a pair).  Generalised singles and doubles
+// of 10 orbitals on 63,504 amplitudes (about 2e7 pairs): k_cg_ip_many 634 us,
+// this kernel 116 us (9
+// orbitals, 8 electrons, 15,876 amplitudes: 31 us).
+struct GPoolTask {
+    int32_t e0, ne;  // alpha entries
+    int32_t k0, nk;  // beta lists
+    int32_t part0;   // first partial
+    int32_t er;      // first entry's number in its list
+    int32_t lw;      // log2 of the warps a beta list is dealt to (tasks of few lists)
+    int32_t pad;
+};
+struct GPoolList {
+    int32_t b0, nb;  // words: r0 | r1 << 15 | sign << 31
+    int32_t s0, pad;  // signs of the alpha entries, a bit each
+    double2 h, g;    // gamma times the pattern's coefficients
+};
+constexpr int kPoolIdx = 15;  // bits of a beta rank
+
+template <class V>
+struct PoolAmp {  // psi and sigma of one amplitude
+    V v, w;
+};
+__device__ __forceinline__ void pool_acc(double &t, double a, double b) { t += a * b; }
+__device__ __forceinline__ void pool_acc(double2 &t, double2 a, double2 b) { t = g_cadd(t, g_cjmul(a, b)); }
+__device__ __forceinline__ double pool_re(double2 c, double t) { return c.x * t; }
+__device__ __forceinline__ double pool_re(double2 c, double2 t) { return c.x * t.x - c.y * t.y; }
+__device__ __forceinline__ PoolAmp<double> pool_ld(const PoolAmp<double> *p) {
+    const double2 x = *reinterpret_cast<const double2 *>(p);
+    return {x.x, x.y};
+}
+__device__ __forceinline__ PoolAmp<double2> pool_ld(const PoolAmp<double2> *p) {
+    const double2 *q = reinterpret_cast<const double2 *>(p);
+    return {q[0], q[1]};
+}
+
+template <class V>
+__global__ void __launch_bounds__(256) k_cg_pool(GLaunch L, const GPoolTask *__restrict__ tasks,
+                                                 const uint32_t *__restrict__ ents,
+                                                 const GPoolList *__restrict__ lists,
+                                                 const uint32_t *__restrict__ words,
+                                                 const uint32_t *__restrict__ signs,
+                                                 double *__restrict__ partial) {
+    extern __shared__ __align__(16) unsigned char p_raw[];
+    PoolAmp<V> *row = reinterpret_cast<PoolAmp<V> *>(p_raw);  // [entry][2][nbeta]
+    const V *psi = reinterpret_cast<const V *>(L.psi), *sig = reinterpret_cast<const V *>(L.sig);
+    const GPoolTask t = tasks[blockIdx.x];
+    const int nb = L.nbeta, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int e = 0; e < t.ne; ++e) {
+        const uint32_t a = ents[t.e0 + e];  // r0 | r1 << 16
+        const size_t g0 = (size_t)(a & 0xffffu) * nb, g1 = (size_t)(a >> 16) * nb;
+        PoolAmp<V> *r = row + (size_t)2 * e * nb;
+        for (int b = threadIdx.x; b < nb; b += blockDim.x) {
+            r[b] = PoolAmp<V>{psi[g0 + b], sig[g0 + b]};
+            r[nb + b] = PoolAmp<V>{psi[g1 + b], sig[g1 + b]};
+        }
+    }
+    __syncthreads();
+    const int part = warp & ((1 << t.lw) - 1);
+    for (int k = warp >> t.lw; k < t.nk; k += nw >> t.lw) {
+        const GPoolList l = lists[t.k0 + k];
+        const uint32_t *sg = signs + l.s0 + (t.er >> 5);
+        const uint32_t mask = __funnelshift_r(sg[0], sg[1], (uint32_t)t.er & 31u);
+        V s1 = qfbs::v_zero(V()), s2 = s1;
+        for (int q = part << 5 | lane; q < l.nb; q += 32 << t.lw) {
+            const uint32_t word = __ldg(words + l.b0 + q);
+            const PoolAmp<V> *x = row + (word & ((1u << kPoolIdx) - 1u));
+            const PoolAmp<V> *y = row + nb + (word >> kPoolIdx & ((1u << kPoolIdx) - 1u));
+            V t1 = qfbs::v_zero(V()), t2 = t1;
+#pragma unroll 4
+            for (int e = 0; e < t.ne; ++e) {
+                const PoolAmp<V> a = pool_ld(x + (size_t)2 * e * nb), b = pool_ld(y + (size_t)2 * e * nb);
+                const uint32_t neg = mask << (31 - e);
+                pool_acc(t1, qfbs::v_flip(a.w, neg), b.v);
+                pool_acc(t2, b.w, qfbs::v_flip(a.v, neg));
+            }
+            s1 = v_add(s1, qfbs::v_flip(t1, word));
+            s2 = v_add(s2, qfbs::v_flip(t2, word));
+        }
+        double x = pool_re(l.h, s1) + pool_re(l.g, s2);
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if (lane == 0) partial[t.part0 + (k << t.lw) + part] = x;
+    }
+}
+
+// grad[mu] = 2 x the sum of operator mu's partials, in order: entries
+// [at[mu], at[mu + 1]) of idx.  One warp per operator.
+__global__ void __launch_bounds__(256) k_cg_pool_grad(const double *__restrict__ partial,
+                                                      const int32_t *__restrict__ at,
+                                                      const int32_t *__restrict__ idx, int n,
+                                                      double *__restrict__ grad) {
+    const int mu = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (mu >= n) return;
+    double x = 0.0;
+    for (int k = at[mu] + lane; k < at[mu + 1]; k += 32) x += partial[idx[k]];
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if (lane == 0) grad[mu] = 2.0 * x;
+}
+
 // psi = |ref> in every slot (psi zeroed beforehand).
 template <class V>
 __global__ void k_cg_ref(GLaunch L, int ref_i) {

@@ -3245,6 +3245,13 @@ struct qfb_ucc_s {
     int2 *pranges = nullptr;   // pool steps of each operator
     StepDev *pool_steps = nullptr;  // full space: the pool's steps on the device
     unsigned pchunks = 1;
+    // global-memory sector, one state: the pool's inner products by alpha list
+    int ptasks = 0;
+    size_t psmem = 0;
+    const qfbg::GPoolTask *ptask = nullptr;
+    const qfbg::GPoolList *plists = nullptr;
+    const uint32_t *pents = nullptr, *pwords = nullptr, *psigns = nullptr;
+    const int32_t *pat = nullptr, *pidx = nullptr;
     qfbs::SStream pstream{};   // global-memory sector: the pool's inner-product records
     qfbs::PStream ppairs{};    // shared-memory sector: the pool's pair lists
     // PQE residuals (qfb_ucc_set_residuals): Re(<I_k|U^dagger H U|ref> phase_k)
@@ -4173,6 +4180,20 @@ static int ucc_pool_stage(qfb_ucc u) {
     if (!u->pool) return fail(QFB_EINVAL, "qfb_ucc_run: no pool set (qfb_ucc_set_pool)");
     const int B = u->nbatch;
     unsigned chunks = u->pchunks;
+    if (u->ptasks > 0) {
+        double *part = (double *)u->ppart;
+        if (u->greal)
+            qfbg::k_cg_pool<double><<<u->ptasks, 256, u->psmem, t_stream>>>(u->GL, u->ptask, u->pents, u->plists,
+                                                                          u->pwords, u->psigns, part);
+        else
+            qfbg::k_cg_pool<double2><<<u->ptasks, 256, u->psmem, t_stream>>>(u->GL, u->ptask, u->pents, u->plists,
+                                                                           u->pwords, u->psigns, part);
+        QFB_LAUNCHED();
+        qfbg::k_cg_pool_grad<<<(unsigned)((u->npool + 7) / 8), 256, 0, t_stream>>>(part, u->pat, u->pidx, u->npool,
+                                                                                 u->pgrad);
+        QFB_LAUNCHED();
+        return QFB_OK;
+    }
     if (u->gsec) {
         const dim3 grid(u->pchunks, u->g_ygrid, (unsigned)u->pstream.n);
         if (u->greal)
@@ -4543,6 +4564,107 @@ int qfb_ucc_destroy(qfb_ucc u) {
     return QFB_OK;
 }
 
+// The pool's inner products on one state of the global-memory sector, by alpha
+// list (qfbg::k_cg_pool).
+struct PoolHost {
+    std::vector<qfbg::GPoolTask> task;
+    std::vector<qfbg::GPoolList> lists;
+    std::vector<uint32_t> ents, words, signs;
+    std::vector<int32_t> at, idx;  // per operator: its partials
+    int npart = 0, ne = 1;         // partials; most alpha entries of a task
+};
+// Shared memory of a task's staged rows: four CTAs an SM, unless one entry of
+// a wide sector needs more.
+constexpr size_t kPoolSmem = 48 * 1024, kPoolSmemMax = 200 * 1024;
+
+static size_t pool_smem(const SectorPlan &sp, bool real, int ne) {
+    return (size_t)ne * 2 * (size_t)sp.nbeta * (real ? 16 : 32);
+}
+
+static bool build_pool(const SectorPlan &sp, const std::vector<CStep> &cs, int nop, bool real, PoolHost &P) {
+    if (sp.nbeta >= 1 << qfbg::kPoolIdx || pool_smem(sp, real, 1) > kPoolSmemMax) return false;
+    const int ne_max = std::max(1, std::min(32, (int)(kPoolSmem / pool_smem(sp, real, 1))));
+    // alpha lists by the strings they move, and the (beta list, operator) pairs
+    // that meet each; a list of pairs (i1, i0) is the list (i0, i1) with both
+    // spins' ends and the two coefficients exchanged
+    struct Alpha {
+        std::vector<uint32_t> list;
+        std::vector<std::pair<qfbg::GPoolList, int>> meets;
+    };
+    std::map<std::vector<uint32_t>, int> aid, bid;
+    std::vector<Alpha> alpha;
+    std::vector<int2> bspan;
+    std::vector<uint32_t> a, b;
+    int64_t total = 0;
+    for (const CStep &c : cs)
+        for (const auto &pt : c.pats) {
+            if (pt.a.empty() || pt.b.empty()) continue;
+            const bool swap = pt.a[0].r0 > pt.a[0].r1;
+            a.clear();
+            b.clear();
+            for (const qfbs::SEntry &e : pt.a)
+                a.push_back(swap ? (uint32_t)e.r1 | (uint32_t)e.r0 << 16 : (uint32_t)e.r0 | (uint32_t)e.r1 << 16);
+            for (const qfbs::SEntry &e : pt.b)
+                b.push_back((uint32_t)(swap ? e.r1 : e.r0) | (uint32_t)(swap ? e.r0 : e.r1) << qfbg::kPoolIdx |
+                            (e.s & 1u) << 31);
+            auto ia = aid.emplace(a, (int)alpha.size());
+            if (ia.second) alpha.push_back(Alpha{a, {}});
+            auto ib = bid.emplace(b, (int)bspan.size());
+            if (ib.second) {
+                bspan.push_back(make_int2((int)P.words.size(), (int)b.size()));
+                P.words.insert(P.words.end(), b.begin(), b.end());
+            }
+            const int2 sp2 = bspan[(size_t)ib.first->second];
+            const double2 gn = swap ? pt.hn : pt.gn, hn = swap ? pt.gn : pt.hn;
+            qfbg::GPoolList l{};
+            l.b0 = sp2.x;
+            l.nb = sp2.y;
+            l.s0 = (int32_t)P.signs.size();
+            l.h = make_double2(c.gamma * hn.x, c.gamma * hn.y);
+            l.g = make_double2(c.gamma * gn.x, c.gamma * gn.y);
+            P.signs.resize(P.signs.size() + (a.size() + 31) / 32, 0u);
+            for (size_t k = 0; k < a.size(); ++k)
+                P.signs[(size_t)l.s0 + k / 32] |= (pt.a[k].s & 1u) << (k & 31);
+            alpha[(size_t)ia.first->second].meets.emplace_back(l, c.param);
+            total += (int64_t)a.size() * sp2.y;
+        }
+    P.signs.push_back(0u);  // (a task reads two words)
+    // pairs of a task: about six tasks an SM (three: 126 us where six take 116,
+    // sixteen 125: rows staged more often)
+    const int64_t most = std::max<int64_t>(4096, total / (6 * (int64_t)sm_count()));
+    std::vector<std::vector<int32_t>> idx((size_t)nop);
+    for (const Alpha &A : alpha) {
+        const int e0 = (int)P.ents.size(), na = (int)A.list.size(), k0 = (int)P.lists.size();
+        P.ents.insert(P.ents.end(), A.list.begin(), A.list.end());
+        for (const auto &m : A.meets) P.lists.push_back(m.first);
+        const int ne = std::min(ne_max, na);
+        P.ne = std::max(P.ne, ne);
+        for (int e = 0; e < na; e += ne) {
+            const int n = std::min(ne, na - e);
+            for (int k = 0; k < (int)A.meets.size();) {
+                int64_t pairs = 0;
+                int j = k;
+                while (j < (int)A.meets.size() && (j - k < 8 || pairs < most)) pairs += (int64_t)n * A.meets[(size_t)j++].first.nb;
+                const int lw = j - k <= 1 ? 3 : j - k <= 2 ? 2 : j - k <= 4 ? 1 : 0;
+                P.task.push_back(qfbg::GPoolTask{e0 + e, n, k0 + k, j - k, P.npart, e, lw, 0});
+                for (int q = k; q < j; ++q)
+                    for (int w = 0; w < 1 << lw; ++w) idx[(size_t)A.meets[(size_t)q].second].push_back(P.npart++);
+                k = j;
+            }
+        }
+    }
+    // the longest tasks first
+    std::stable_sort(P.task.begin(), P.task.end(), [](const qfbg::GPoolTask &a, const qfbg::GPoolTask &b) {
+        return (int64_t)a.ne * a.nk > (int64_t)b.ne * b.nk;
+    });
+    for (const auto &v : idx) {
+        P.at.push_back((int32_t)P.idx.size());
+        P.idx.insert(P.idx.end(), v.begin(), v.end());
+    }
+    P.at.push_back((int32_t)P.idx.size());
+    return !P.task.empty();
+}
+
 int qfb_ucc_set_pool(qfb_ucc u, qfb_prog pool) {
     if (!u || !pool) return fail(QFB_EINVAL, "qfb_ucc_set_pool: null argument");
     if (!pool->params_contiguous || pool->nparam < 1)
@@ -4555,6 +4677,7 @@ int qfb_ucc_set_pool(qfb_ucc u, qfb_prog pool) {
     qfbs::SStream ps{};
     StreamHost sh;
     PairHost ph;  // shared-memory sector: the pool as pair lists
+    PoolHost pl;  // global-memory sector, one state: by alpha list
     unsigned chunks = 1;
     if (u->compact || u->gsec) {
         std::vector<CStep> cs;
@@ -4572,6 +4695,11 @@ int qfb_ucc_set_pool(qfb_ucc u, qfb_prog pool) {
             return fail(QFB_ENOSYS, "qfb_ucc_set_pool: complex pool coefficients on an evaluator "
                                     "with real states (create it with qfb_ucc_config(4))");
         chunks = u->compact ? kSectorThreads / 32 : global_grid(stream_max_pairs(sh), u->GL.spw);
+        // (several states: k_cg_ip_many reads them together)
+        if (u->gsec && B == 1 && build_pool(*u->splan, cs, M, u->greal != 0, pl)) {
+            sh = StreamHost{};
+            chunks = 1;
+        }
     } else {
         uint64_t most = 1;
         for (const auto &st : pool->h_steps) {
@@ -4590,12 +4718,23 @@ int qfb_ucc_set_pool(qfb_ucc u, qfb_prog pool) {
         return o;
     };
     const size_t o_pg = take(sizeof(double) * (size_t)B * M);
-    const size_t o_pp = take(sizeof(double2) * nst * B * chunks);
+    const size_t o_pp = take(pl.task.empty() ? sizeof(double2) * nst * B * chunks : sizeof(double) * (size_t)pl.npart);
     const size_t o_pr = take(sizeof(int2) * M);
     const size_t o_ps = take((u->compact || u->gsec) ? 16 : sizeof(StepDev) * nst);
     const size_t o_rec = take(sizeof(uint4) * sh.rec.size());
     const size_t o_sp = take(sizeof(int2) * sh.span.size());
     const size_t o_pl = take(u->compact ? pair_bytes(ph) : 16);
+    struct Up {
+        const void *p;
+        size_t n, o;
+    } ups[] = {{pl.task.data(), sizeof(qfbg::GPoolTask) * pl.task.size(), 0},
+               {pl.ents.data(), sizeof(uint32_t) * pl.ents.size(), 0},
+               {pl.lists.data(), sizeof(qfbg::GPoolList) * pl.lists.size(), 0},
+               {pl.words.data(), sizeof(uint32_t) * pl.words.size(), 0},
+               {pl.at.data(), sizeof(int32_t) * pl.at.size(), 0},
+               {pl.idx.data(), sizeof(int32_t) * pl.idx.size(), 0},
+               {pl.signs.data(), sizeof(uint32_t) * pl.signs.size(), 0}};
+    for (Up &x : ups) x.o = take(x.n);
     void *blob = nullptr;
     int rc = dev_alloc(&blob, off);
     if (rc) return rc;
@@ -4615,6 +4754,15 @@ int qfb_ucc_set_pool(qfb_ucc u, qfb_prog pool) {
     if (e == cudaSuccess && !sh.span.empty())
         e = cudaMemcpyAsync(base + o_sp, sh.span.data(), sizeof(int2) * sh.span.size(),
                             cudaMemcpyHostToDevice, t_stream);
+    for (const Up &x : ups)
+        if (e == cudaSuccess && x.n) e = cudaMemcpyAsync(base + x.o, x.p, x.n, cudaMemcpyHostToDevice, t_stream);
+    const size_t psmem = pl.task.empty() ? 0 : pool_smem(*u->splan, u->greal != 0, pl.ne);
+    if (e == cudaSuccess && psmem > kPoolSmem) {
+        e = cudaFuncSetAttribute(qfbg::k_cg_pool<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPoolSmemMax);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(qfbg::k_cg_pool<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kPoolSmemMax);
+    }
     qfbs::PStream pp{};
     if (e == cudaSuccess && u->compact && pair_upload(ph, base + o_pl, pp)) e = cudaErrorUnknown;
     if (e == cudaSuccess) e = cudaStreamSynchronize(t_stream);
@@ -4642,6 +4790,15 @@ int qfb_ucc_set_pool(qfb_ucc u, qfb_prog pool) {
     ps.maxw = std::max(sh.maxw, 1);
     u->pstream = ps;
     u->ppairs = pp;
+    u->ptasks = (int)pl.task.size();
+    u->psmem = psmem;
+    u->ptask = (const qfbg::GPoolTask *)(base + ups[0].o);
+    u->pents = (const uint32_t *)(base + ups[1].o);
+    u->plists = (const qfbg::GPoolList *)(base + ups[2].o);
+    u->pwords = (const uint32_t *)(base + ups[3].o);
+    u->pat = (const int32_t *)(base + ups[4].o);
+    u->pidx = (const int32_t *)(base + ups[5].o);
+    u->psigns = (const uint32_t *)(base + ups[6].o);
     return QFB_OK;
 }
 
