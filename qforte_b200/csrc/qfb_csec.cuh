@@ -294,6 +294,10 @@ __global__ void k_cg_ref(GLaunch L, int ref_i) {
 // sigma = H psi from the sector's H rows: one warp per output row i, lanes
 // over (slot, entry sub-index) as in k_cg_step; energy partials per slot.
 // epart[s * gridDim.x + blockIdx.x] = sum over this block's rows of conj(psi) sigma.
+// Bound by the rows' stream from HBM (one state) and the gathers of psi from L2
+// (several); four entries in flight per lane, us, one / four: 20 qubits (5.6e7
+// entries, 667 MB) 1 state 186 / 145, 6 states 660 / 506; 18 qubits (8.9e6) 1 state
+// 30 / 21, 8 states 110 / 86, 24 states 316 / 277.
 template <bool REAL, class V>
 __global__ void __launch_bounds__(256) k_cg_h_rows(GLaunch L, const int32_t *__restrict__ rowptr,
                                                    const uint32_t *__restrict__ col,
@@ -307,11 +311,29 @@ __global__ void __launch_bounds__(256) k_cg_h_rows(GLaunch L, const int32_t *__r
     const int per = 32 / L.spw, sub = lane / L.spw;
     const int s = blockIdx.y * L.spw + (lane % L.spw);
     const bool live = s < L.B;
+    constexpr int U = 4;  // entries in flight per lane
     double2 en = make_double2(0.0, 0.0);
     for (int i = blockIdx.x * nwarp + warp; i < L.nsec; i += gridDim.x * nwarp) {
         V acc = v_zero(V());
         const int e1 = rowptr[i + 1];
-        for (int e = rowptr[i] + sub; e < e1; e += per) {
+        int e = rowptr[i] + sub;
+        if constexpr (REAL) {
+            for (; e + (U - 1) * per < e1; e += U * per) {
+                uint32_t c[U];
+                double f[U];
+                V x[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    c[u] = __ldcs(&col[e + u * per]);
+                    f[u] = __ldcs(&val_r[e + u * per]);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) x[u] = live ? psi[(size_t)c[u] * L.B + s] : v_zero(V());
+#pragma unroll
+                for (int u = 0; u < U; ++u) qfbs::v_acc(acc, f[u], x[u]);
+            }
+        }
+        for (; e < e1; e += per) {
             const uint32_t c = __ldg(&col[e]);
             const V x = live ? psi[(size_t)c * L.B + s] : v_zero(V());
             if constexpr (REAL) {
