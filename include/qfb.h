@@ -164,8 +164,8 @@ QFB_API int qfb_gates_regs(int reg_bits);
  * FP64 tensor cores (mma.sync), the product of its gates, one per assignment
  * of the thread bits its controls test, and one factor per amplitude vector
  * (complex64 states widened to FP64 for the products); 0 applies the phase's
- * gates one by one; 2 (the default) is 1 for states of 128 MiB and more
- * (larger than L2) and 0 below.
+ * gates one by one; 2 (the default) is 1 for states of 16 MiB and more
+ * (complex64: 128 MiB) and 0 below.
  * Both forms give the result of the gates in list order (up to the rounding
  * of the fused products).  No counterpart in the reference; set by the
  * autotuner. */

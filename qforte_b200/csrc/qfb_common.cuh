@@ -64,6 +64,11 @@ struct qfb_state_s {
     double2 *d;       // [nbatch][nbasis]
 };
 
+// A gate list in register-blocked tiles (qfb_core.cu), and whether gate lists
+// are applied that way (qfb_gates_config, qfb_gates_dense).
+bool gate_tiles_on();
+int apply_gate_list(qfb_state s, const std::vector<qfb_gate> &gates);
+
 // ---- device side ----------------------------------------------------------
 
 __device__ __forceinline__ double2 c_mul(double2 a, double2 b) {

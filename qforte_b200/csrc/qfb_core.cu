@@ -419,7 +419,10 @@ inline bool is_one(const qfb_complex &c) { return c.re == 1.0 && c.im == 0.0; }
 inline bool ceq(const qfb_complex &a, const qfb_complex &b) {
     return a.re == b.re && a.im == b.im;
 }
-inline double cabs_h(const qfb_complex &c) { return std::hypot(c.re, c.im); }
+inline double cabs_h(const qfb_complex &c) {
+    if (c.im == 0.0) return std::fabs(c.re);
+    return c.re == 0.0 ? std::fabs(c.im) : std::hypot(c.re, c.im);
+}
 
 constexpr double kThr = 1.0e-16;  // Computer::compute_threshold_ (computer.h:172)
 
@@ -500,7 +503,9 @@ int launch_single_t(A *d, uint64_t nbasis, int nbatch, const HGate &h) {
 
 int launch_single(qfb_state s, const HGate &h) { return launch_single_t(s->d, s->nbasis, s->nbatch, h); }
 
-constexpr int kGateTileDefault = 10;  // 2^10 amplitudes = 18 KB of shared memory per tile
+// Default tile bits: 10 where the fused form is taken, 11 for smaller complex128
+// states (20 layers, us, 10 / 11: 12 qubits 213 / 197, 18 qubits 395 / 367).
+constexpr int kGateTileDefault = 10, kGateTileSmall = 11, kGateTileSmallQubits = 19;
 constexpr int kGateTileMax = 12;
 int g_gate_tile_bits = 0;  // 0: kGateTileDefault; -1: one pass per gate
 int g_gate_low_bits = 3;
@@ -508,10 +513,12 @@ int g_gate_low_bits = 3;
 int g_gate_reg_bits = 0;  // 0: default
 // Form of the tile phases: 0 gate by gate; 1 fused (8 x 8 matrices on the
 // FP64 tensor cores) where it applies; 2 (default) fused for states of at
-// least kFusedMinBytes (larger than L2: below it the gate-by-gate form is
-// faster, the tile traffic being L2-resident).
+// least kFusedMinBytes.  Below it the time goes to planning, and the matrices
+// cost more of it (20 random layers, us, gate by gate / fused: 18 qubits 460 /
+// 500, 19 qubits 517 / 518, 20 qubits 973 / 577, 21 qubits 1,499 / 809, 24 qubits
+// 11,471 / 5,600).
 int g_gate_fused = 2;
-constexpr uint64_t kFusedMinBytes = 1ull << 27;
+constexpr uint64_t kFusedMinBytes = 1ull << 24, kFusedMinBytesC64 = 1ull << 27;
 
 // Register bits R of a tile of b qubits: 2^(b-R) threads (<= 256) hold 2^R
 // amplitudes each.  Default 3 (8 amplitudes, 80 registers a thread, three
@@ -524,8 +531,8 @@ inline int tile_reg_bits(int b) {
 
 // Tile shape for an n-qubit state: false when every gate takes its own pass
 // (tile_bits -1, or a state smaller than two 128-byte chunks).
-bool gate_tile_shape(int n, int &b, int &L) {
-    b = g_gate_tile_bits == 0 ? kGateTileDefault : g_gate_tile_bits;
+bool gate_tile_shape(int n, int &b, int &L, bool c64 = false) {
+    b = g_gate_tile_bits != 0 ? g_gate_tile_bits : (c64 || n > kGateTileSmallQubits) ? kGateTileDefault : kGateTileSmall;
     if (b < 0 || n < 4) return false;
     L = std::max(3, std::min(g_gate_low_bits, n));
     b = std::max(4, std::min(b, n));
@@ -539,12 +546,15 @@ inline int fused_bytes(int plain) {
     return ((plain + 15) & ~15) + 2 * (1 << qfbt::kMaxThreadBits) * (int)sizeof(uint32_t);
 }
 
+// Shared memory of the gate-by-gate form: the same, then two staged phases.
+inline int stage_bytes(int plain) { return ((plain + 15) & ~15) + 2 * (int)sizeof(qfbt::TStage); }
+
 int gate_tile_smem() {
     static std::once_flag once;
     static cudaError_t err = cudaSuccess;
     std::call_once(once, [] {
-        auto bytes = [](int b) { return (int)(sizeof(double2) * qfbt::tpad_size(b) + 16); };
-        auto bytes8 = [](int b) { return (int)(sizeof(float2) * qfbt::tpad8_size(b) + 16); };
+        auto bytes = [](int b) { return stage_bytes((int)(sizeof(double2) * qfbt::tpad_size(b) + 16)); };
+        auto bytes8 = [](int b) { return stage_bytes((int)(sizeof(float2) * qfbt::tpad8_size(b) + 16)); };
         auto attr = [&](const void *f, int n) {
             if (err == cudaSuccess)
                 err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, n);
@@ -566,52 +576,110 @@ struct GatePlanWin {
     int64_t single;  // >= 0: a window of one gate, applied by its own pass
 };
 
-// Greedy windows: scanning the unapplied gates in order, a gate joins the
-// current window when no earlier unapplied gate shares one of its qubits
-// (gates on disjoint qubits commute) and its qubits fit in the window's b
-// qubits together with those already chosen; a gate that cannot join blocks
-// its qubits for the rest of the scan.  The window's qubits always include
-// the lowest L, and are filled up to b with the lowest unused ones.
-void plan_gate_windows(const std::vector<HGate> &hg, int n, int b, int L,
-                       std::vector<GatePlanWin> &wins, std::vector<WGate> &wg) {
-    const int64_t N = (int64_t)hg.size();
-    const uint64_t all = (n >= 64) ? ~0ull : (1ull << n) - 1ull;
-    const uint64_t low = (1ull << L) - 1ull;
-    std::vector<char> done((size_t)N, 0);
-    int64_t first = 0;
+// Windows: sets Q of at most b qubits, each with the gates that can run when only
+// Q's qubits advance (a gate is ready when it is the next one on all its qubits,
+// so only gates on disjoint qubits change order).  Q holds the lowest L qubits
+// and grows by the qubit, or the qubit and the partner of its next two-qubit gate,
+// that lets the most further gates run per qubit added: taking qubits as the gate
+// list names them fills Q with qubits whose partners are outside (27 qubits, 40
+// random layers, 1,600 gates: 89 windows, this way 71).  Q is filled up to b
+// with the lowest unused qubits.
+struct WindowPlanner {
+    const std::vector<HGate> &hg;
+    int n, b, L;
+    std::vector<uint64_t> qm;            // the gates' qubits
+    std::vector<int32_t> list, at, end;  // per qubit: its gates in order, the next one
     std::vector<int64_t> sel;
-    while (first < N) {
-        uint64_t Q = low, blocked = 0;
-        sel.clear();
-        int64_t scanned = 0;
-        for (int64_t i = first; i < N && blocked != all && scanned < 16384; ++i) {
-            if (done[i]) continue;
-            ++scanned;
-            const uint64_t gm = hg[i].qubits;
-            if (gm & blocked) {
-                blocked |= gm;
+    int64_t left;
+    WindowPlanner(const std::vector<HGate> &gates, int n_, int b_, int L_)
+        : hg(gates), n(n_), b(b_), L(L_), at((size_t)n_, 0), end((size_t)n_, 0), left((int64_t)gates.size()) {
+        qm.reserve(hg.size());
+        for (const HGate &h : hg) {
+            qm.push_back(h.qubits);
+            for (uint64_t m = h.qubits; m; m &= m - 1) ++end[(size_t)__builtin_ctzll(m)];
+        }
+        int32_t total = 0;
+        for (int q = 0; q < n; ++q) {
+            at[(size_t)q] = total;
+            total += end[(size_t)q];
+            end[(size_t)q] = at[(size_t)q];
+        }
+        list.resize((size_t)total);
+        for (size_t i = 0; i < hg.size(); ++i)
+            for (uint64_t m = qm[i]; m; m &= m - 1) list[(size_t)end[(size_t)__builtin_ctzll(m)]++] = (int32_t)i;
+    }
+    int front(int q) const { return at[(size_t)q] < end[(size_t)q] ? list[(size_t)at[(size_t)q]] : -1; }
+    // Run what can run on Q, starting from the qubits `from`; gates appended to sel.
+    void run(uint64_t Q, uint64_t from) {
+        while (from) {
+            const int q = __builtin_ctzll(from);
+            const int g = front(q);
+            const uint64_t gm = g < 0 ? 0 : qm[(size_t)g], rest = gm & (gm - 1) ? gm & ~(1ull << q) : 0;
+            if (g < 0 || (gm & ~Q) || (rest && front(__builtin_ctzll(rest)) != g)) {
+                from &= from - 1;
                 continue;
             }
-            const uint64_t nq = Q | gm;
-            if (__builtin_popcountll(nq) <= b) {
-                Q = nq;
-                sel.push_back(i);
-                done[i] = 1;
-            } else {
-                blocked |= gm;
+            for (uint64_t m = gm; m; m &= m - 1) ++at[(size_t)__builtin_ctzll(m)];
+            from |= gm;
+            sel.push_back(g);
+        }
+    }
+    void undo(size_t keep) {
+        for (; sel.size() > keep; sel.pop_back())
+            for (uint64_t m = qm[(size_t)sel.back()]; m; m &= m - 1) --at[(size_t)__builtin_ctzll(m)];
+    }
+    // The next window, its gates (tile coordinates) appended to wg; false at the end.
+    bool next(GatePlanWin &pw, std::vector<WGate> &wg) {
+        if (left == 0) return false;
+        const uint64_t all = (n >= 64) ? ~0ull : (1ull << n) - 1ull;
+        uint64_t Q = (1ull << L) - 1ull;
+        sel.clear();
+        run(Q, Q);
+        while (__builtin_popcountll(Q) < b) {
+            const int room = b - __builtin_popcountll(Q);
+            const size_t have = sel.size();
+            uint64_t best = 0;
+            int64_t gain = 0;
+            auto consider = [&](uint64_t S) {
+                run(Q | S, S);
+                const int64_t g = (int64_t)(sel.size() - have);
+                if (g * __builtin_popcountll(best) > gain * __builtin_popcountll(S) || (best == 0 && g > 0)) {
+                    best = S;
+                    gain = g;
+                }
+                undo(have);
+            };
+            // the partner of each qubit's next two-qubit gate
+            uint64_t mate[64];
+            for (int q = 0; q < n; ++q) {
+                mate[q] = 0;
+                for (int32_t k = at[(size_t)q]; k < end[(size_t)q] && !mate[q]; ++k)
+                    mate[q] = qm[(size_t)list[(size_t)k]] & ~(1ull << q);
             }
+            for (int q = 0; q < n; ++q) {
+                const uint64_t bit = 1ull << q;
+                if ((Q & bit) || front(q) < 0) continue;
+                if (!mate[q] || (mate[q] & Q) || room < 2) {
+                    consider(bit);
+                } else {
+                    const int m = __builtin_ctzll(mate[q]);
+                    if (m > q || mate[m] != bit) consider(bit | mate[q]);
+                }
+            }
+            if (!best) break;
+            Q |= best;
+            run(Q, best);
         }
         if (sel.empty()) {
-            // the first unapplied gate fits no tile of this shape: its own pass
-            sel.push_back(first);
-            done[first] = 1;
+            // no gate fits a tile of this shape: a ready one's own pass
+            for (int q = 0; q < n && sel.empty(); ++q) run(all, front(q) < 0 ? 0 : 1ull << q);
+            undo(1);
         }
-        while (first < N && done[first]) ++first;
-        GatePlanWin pw{};
+        left -= (int64_t)sel.size();
+        pw = GatePlanWin{};
         if (sel.size() == 1) {
             pw.single = sel[0];
-            wins.push_back(pw);
-            continue;
+            return true;
         }
         for (int q = 0; q < n && __builtin_popcountll(Q) < b; ++q) Q |= 1ull << q;
         auto loc = [&](int q) { return __builtin_popcountll(Q & ((1ull << q) - 1ull)); };
@@ -643,8 +711,15 @@ void plan_gate_windows(const std::vector<HGate> &hg, int n, int b, int L,
             }
             wg.push_back(w);
         }
-        wins.push_back(pw);
+        return true;
     }
+};
+
+void plan_gate_windows(const std::vector<HGate> &hg, int n, int b, int L,
+                       std::vector<GatePlanWin> &wins, std::vector<WGate> &wg) {
+    WindowPlanner P(hg, n, b, L);
+    GatePlanWin pw;
+    while (P.next(pw, wg)) wins.push_back(pw);
 }
 
 struct TilePlan {
@@ -657,12 +732,18 @@ struct TilePlan {
     std::vector<double2> fm;        // fused form: segment matrices, per-thread factors
 };
 
-// The bits of v, lowest first, placed on the set bits of m.
-uint64_t deposit_host(uint64_t v, uint64_t m) {
-    uint64_t r = 0;
-    for (; m; m &= m - 1, v >>= 1)
-        if (v & 1ull) r |= m & (~m + 1);
-    return r;
+// A phase's thread table (tl | offset << 16 per thread), bit j of the thread
+// number on tile bit tb[j]; offsets add up over tile bits.
+template <class Off>
+void push_threads(std::vector<uint32_t> &threads, const std::vector<int> &tb, const Off &toff) {
+    const size_t t0 = threads.size();
+    threads.resize(t0 + ((size_t)1 << tb.size()));
+    uint32_t *e = threads.data() + t0;
+    e[0] = 0;
+    for (size_t j = 0; j < tb.size(); ++j) {
+        const uint32_t bit = 1u << tb[j], v = bit | toff(bit) << 16;
+        for (size_t t = 0; t < (size_t)1 << j; ++t) e[t + ((size_t)1 << j)] = e[t] + v;
+    }
 }
 
 // The 4x4 matrix of SWAP exactly (unit entries at (0,0), (1,2), (2,1), (3,3)).
@@ -681,62 +762,67 @@ inline double2 cmul_h(double2 a, double2 b) {
 }
 inline double2 cadd_h(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 
-// One op of a phase on the 2^R registers of the thread with tile bits tl,
-// exactly as qfbt::apply_op applies it.
-void top_apply_host(const qfbt::TOp &o, const double2 *m4, uint32_t tl, int R, double2 *v) {
+// One op of a phase on the rows of an 8 x 8 matrix (row k: what register k
+// receives), for the thread with tile bits tl, as qfbt::apply_op applies it.
+void top_apply_rows(const qfbt::TOp &o, const double2 *m4, uint32_t tl, double2 (*v)[8]) {
     if ((tl & o.tctl) != o.tctl) return;
-    const uint32_t NR = 1u << R, cm = o.aux & 0xffu, cv = (o.aux >> 16) & 0xffu;
-    const uint32_t opc = o.opc;
+    const uint32_t cm = o.aux & 0xffu, cv = (o.aux >> 16) & 0xffu, opc = o.opc;
+    auto scale = [](double2 f, double2 *r) {
+        for (int c = 0; c < 8; ++c) r[c] = cmul_h(f, r[c]);
+    };
     if (opc < qfbt::OPC_DIAG) {
         const uint32_t kind = opc / 4, tb = 1u << (opc % 4);
-        for (uint32_t k = 0; k < NR; ++k) {
+        for (uint32_t k = 0; k < 8; ++k) {
             if ((k & tb) || (k & cm) != cv) continue;
-            const double2 x0 = v[k], x1 = v[k | tb];
-            if (kind == qfbt::OP_PSWAP) {
-                v[k] = x1;
-                v[k | tb] = x0;
-            } else if (kind == qfbt::OP_ANTI) {
-                v[k] = cmul_h(o.m[1], x1);
-                v[k | tb] = cmul_h(o.m[2], x0);
-            } else {
-                v[k] = cadd_h(cmul_h(o.m[0], x0), cmul_h(o.m[1], x1));
-                v[k | tb] = cadd_h(cmul_h(o.m[2], x0), cmul_h(o.m[3], x1));
+            double2 *r0 = v[k], *r1 = v[k | tb];
+            for (int c = 0; c < 8; ++c) {
+                const double2 x0 = r0[c], x1 = r1[c];
+                if (kind == qfbt::OP_PSWAP) {
+                    r0[c] = x1;
+                    r1[c] = x0;
+                } else if (kind == qfbt::OP_ANTI) {
+                    r0[c] = cmul_h(o.m[1], x1);
+                    r1[c] = cmul_h(o.m[2], x0);
+                } else {
+                    r0[c] = cadd_h(cmul_h(o.m[0], x0), cmul_h(o.m[1], x1));
+                    r1[c] = cadd_h(cmul_h(o.m[2], x0), cmul_h(o.m[3], x1));
+                }
             }
         }
     } else if (opc < qfbt::OPC_DIAG_THREAD) {
         const uint32_t dset = (opc - qfbt::OPC_DIAG) / 4 + 1, tb = 1u << ((opc - qfbt::OPC_DIAG) % 4);
-        for (uint32_t k = 0; k < NR; ++k) {
+        for (uint32_t k = 0; k < 8; ++k) {
             if ((k & cm) != cv) continue;
             if (k & tb) {
-                if (dset & 2u) v[k] = cmul_h(o.m[3], v[k]);
+                if (dset & 2u) scale(o.m[3], v[k]);
             } else if (dset & 1u) {
-                v[k] = cmul_h(o.m[0], v[k]);
+                scale(o.m[0], v[k]);
             }
         }
     } else if (opc == qfbt::OPC_DIAG_THREAD) {
         const bool one = (tl & o.tbit) != 0;
         if (!(((o.aux >> 8) & 3u) & (one ? 2u : 1u))) return;
-        const double2 f = o.m[one ? 3 : 0];
-        for (uint32_t k = 0; k < NR; ++k)
-            if ((k & cm) == cv) v[k] = cmul_h(f, v[k]);
+        for (uint32_t k = 0; k < 8; ++k)
+            if ((k & cm) == cv) scale(o.m[one ? 3 : 0], v[k]);
     } else if (opc < qfbt::OPC_BSWAP) {
         const uint32_t tb = 1u << ((opc - qfbt::OPC_GEN4) / 4), cb = 1u << ((opc - qfbt::OPC_GEN4) % 4);
         const double2 *m = m4 + o.aux;
-        for (uint32_t k = 0; k < NR; ++k) {
+        for (uint32_t k = 0; k < 8; ++k) {
             if (k & (tb | cb)) continue;
-            const uint32_t idx[4] = {k, k | tb, k | cb, k | tb | cb};
-            double2 y[4];
-            for (int i = 0; i < 4; ++i) {
-                double2 acc = make_double2(0.0, 0.0);
-                for (int j = 0; j < 4; ++j) acc = cadd_h(acc, cmul_h(m[4 * i + j], v[idx[j]]));
-                y[i] = acc;
+            double2 *r[4] = {v[k], v[k | tb], v[k | cb], v[k | tb | cb]};
+            for (int c = 0; c < 8; ++c) {
+                const double2 x[4] = {r[0][c], r[1][c], r[2][c], r[3][c]};
+                for (int i = 0; i < 4; ++i) {
+                    double2 acc = make_double2(0.0, 0.0);
+                    for (int j = 0; j < 4; ++j) acc = cadd_h(acc, cmul_h(m[4 * i + j], x[j]));
+                    r[i][c] = acc;
+                }
             }
-            for (int i = 0; i < 4; ++i) v[idx[i]] = y[i];
         }
     } else {
         const uint32_t tb = 1u << ((opc - qfbt::OPC_BSWAP) / 4), cb = 1u << ((opc - qfbt::OPC_BSWAP) % 4);
-        for (uint32_t k = 0; k < NR; ++k)
-            if ((k & tb) && !(k & cb)) std::swap(v[k], v[k ^ tb ^ cb]);
+        for (uint32_t k = 0; k < 8; ++k)
+            if ((k & tb) && !(k & cb)) std::swap_ranges(v[k], v[k] + 8, v[k ^ tb ^ cb]);
     }
 }
 
@@ -770,7 +856,7 @@ void fuse_phase(TilePlan &tp, const qfbt::TPhase &ph, int b, bool c64) {
     const uint32_t T = ((1u << b) - 1u) & ~S;  // thread bits
     std::vector<int> run_ops;
     std::vector<qfbt::TOp> fac_ops;
-    std::vector<double2> col(NR), mat;
+    double2 mat[NR][NR];
     struct Seg {
         uint32_t D;  // variant bits
         qfbt::TSeg h;
@@ -788,23 +874,19 @@ void fuse_phase(TilePlan &tp, const qfbt::TPhase &ph, int b, bool c64) {
         sg.h.m0 = (uint32_t)mats.size();
         sg.h.nd = (uint32_t)dbits.size();
         for (size_t j = 0; j < dbits.size(); ++j) sg.h.dsel |= (uint32_t)dbits[j] << (4 * j);
-        mat.assign((size_t)NR * NR, make_double2(0.0, 0.0));
         for (uint32_t x = 0; x < nvar; ++x) {
             uint32_t tl = 0;
             for (size_t j = 0; j < dbits.size(); ++j)
                 if (x >> j & 1u) tl |= 1u << dbits[j];
-            for (uint32_t c = 0; c < NR; ++c) {
-                std::fill(col.begin(), col.end(), make_double2(0.0, 0.0));
-                col[c] = make_double2(1.0, 0.0);
-                for (int oi : run_ops) top_apply_host(tp.ops[oi], tp.m4.data(), tl, R, col.data());
-                for (uint32_t r = 0; r < NR; ++r) {
-                    mat[r * NR + c] = col[r];
-                    if (col[r].x != 0.0 || col[r].y != 0.0) sg.h.mm |= r ^ c;
-                }
-            }
+            for (uint32_t r = 0; r < NR; ++r)
+                for (uint32_t c = 0; c < NR; ++c) mat[r][c] = make_double2(r == c ? 1.0 : 0.0, 0.0);
+            for (int oi : run_ops) top_apply_rows(tp.ops[oi], tp.m4.data(), tl, mat);
+            for (uint32_t r = 0; r < NR; ++r)
+                for (uint32_t c = 0; c < NR; ++c)
+                    if (mat[r][c].x != 0.0 || mat[r][c].y != 0.0) sg.h.mm |= r ^ c;
             for (uint32_t kb = 0; kb < 2; ++kb)
                 for (uint32_t lane = 0; lane < 32; ++lane)
-                    mats.push_back(mat[(lane >> 2) * NR + 4 * kb + (lane & 3)]);
+                    mats.push_back(mat[lane >> 2][4 * kb + (lane & 3)]);
 
         }
         segs.push_back(sg);
@@ -849,12 +931,7 @@ void fuse_phase(TilePlan &tp, const qfbt::TPhase &ph, int b, bool c64) {
         for (int p = 0; p < b; ++p)
             if (free_bits >> p & 1u) tb.push_back(p);
         const int th0 = (int)tp.threads.size();
-        for (uint32_t t = 0; t < nth; ++t) {
-            uint32_t tl = 0;
-            for (size_t j = 0; j < tb.size(); ++j)
-                if (t >> j & 1u) tl |= 1u << tb[j];
-            tp.threads.push_back(tl | (toff(tl) << 16));
-        }
+        push_threads(tp.threads, tb, toff);
         return th0;
     };
     // group the segments into phases
@@ -891,7 +968,10 @@ void fuse_phase(TilePlan &tp, const qfbt::TPhase &ph, int b, bool c64) {
             for (uint32_t t = 0; t < nth; ++t) {
                 double2 f = make_double2(1.0, 0.0);
                 const uint32_t tl = tp.threads[q.th0 + t] & 0xffffu;
-                for (const qfbt::TOp &o : fac_ops) top_apply_host(o, tp.m4.data(), tl, 0, &f);
+                for (const qfbt::TOp &o : fac_ops) {
+                    const uint32_t one = (tl & o.tbit) != 0;
+                    if ((tl & o.tctl) == o.tctl && (o.aux >> (8 + one) & 1u)) f = cmul_h(o.m[one ? 3 : 0], f);
+                }
                 tp.fm.push_back(f);
             }
         }
@@ -930,6 +1010,8 @@ void plan_tile_phases(const WGate *g, int ng, int b, int R, qfbt::TRun &run, Til
     std::vector<int> sel;
     int first = 0;
     run.p0 = (int)tp.ph.size();
+    run.o0 = (int)tp.ops.size();
+    run.th0 = (int)tp.threads.size();
     while (first < ng) {
         uint32_t S = 0, blocked = 0;
         sel.clear();
@@ -992,12 +1074,8 @@ void plan_tile_phases(const WGate *g, int ng, int b, int R, qfbt::TRun &run, Til
             ph.roff[k] = toff(l);
         }
         ph.th0 = (int)tp.threads.size();
-        for (uint32_t tid = 0; tid < (1u << (b - R)); ++tid) {
-            uint32_t tl = 0;
-            for (size_t j = 0; j < tb.size(); ++j)
-                if (tid >> j & 1u) tl |= 1u << tb[j];
-            tp.threads.push_back(tl | (toff(tl) << 16));
-        }
+        const bool fuse = fused && R == 3 && b - R >= 5;  // (its phases have their own tables)
+        if (!fuse) push_threads(tp.threads, tb, toff);
         ph.o0 = (int)tp.ops.size();
         auto swap2 = [](double2 &x, double2 &y) {
             const double2 t = x;
@@ -1086,7 +1164,7 @@ void plan_tile_phases(const WGate *g, int ng, int b, int R, qfbt::TRun &run, Til
             ph.soff[k] = toff(l);
         }
         ph.no = (int)tp.ops.size() - ph.o0;
-        if (fused && R == 3 && b - R >= 5)
+        if (fuse)
             fuse_phase(tp, ph, b, c64);
         else
             tp.ph.push_back(ph);
@@ -1253,12 +1331,9 @@ int apply_gates_dense(qfb_state s, const std::vector<HGate> &hg, int K) {
     return rc;
 }
 
-// Runs of a gate list and the phases of each run.
-void plan_gate_tiles(const std::vector<HGate> &hg, int n, int b, int L,
-                     std::vector<GatePlanWin> &wins, TilePlan &tp, std::vector<qfbt::TRun> &runs,
-                     bool c64 = false, bool fused = false) {
-    std::vector<WGate> wg;
-    plan_gate_windows(hg, n, b, L, wins, wg);
+// The phases of each window's run.
+void plan_tile_runs(const std::vector<GatePlanWin> &wins, const std::vector<WGate> &wg, TilePlan &tp,
+                    std::vector<qfbt::TRun> &runs, bool c64, bool fused) {
     runs.assign(wins.size(), qfbt::TRun{});
     for (size_t i = 0; i < wins.size(); ++i) {
         const GatePlanWin &pw = wins[i];
@@ -1266,11 +1341,23 @@ void plan_gate_tiles(const std::vector<HGate> &hg, int n, int b, int L,
         qfbt::TRun &r = runs[i];
         r.qmask = pw.w.qmask;
         r.ch0 = (int)tp.chunks.size();
-        for (uint64_t c = 0; c < (1ull << (pw.w.b - 3)); ++c)
-            tp.chunks.push_back(deposit_host(c, pw.w.qmask & ~7ull));
+        tp.chunks.push_back(0);
+        uint64_t m = pw.w.qmask & ~7ull;
+        for (size_t half = 1; m; m &= m - 1, half <<= 1)
+            for (size_t c = 0; c < half; ++c)
+                tp.chunks.push_back(tp.chunks[(size_t)r.ch0 + c] | (m & (~m + 1)));
         plan_tile_phases(wg.data() + pw.w.g0, pw.w.ng, pw.w.b, tile_reg_bits(pw.w.b), r, tp, c64,
                          fused);
     }
+}
+
+// Runs of a gate list and the phases of each run.
+void plan_gate_tiles(const std::vector<HGate> &hg, int n, int b, int L,
+                     std::vector<GatePlanWin> &wins, TilePlan &tp, std::vector<qfbt::TRun> &runs,
+                     bool c64 = false, bool fused = false) {
+    std::vector<WGate> wg;
+    plan_gate_windows(hg, n, b, L, wins, wg);
+    plan_tile_runs(wins, wg, tp, runs, c64, fused);
 }
 
 // Bounds-check and classify a gate list for an nqubit state.
@@ -1288,32 +1375,16 @@ int classify_gates(const qfb_gate *gates, int64_t ngates, int nqubit, const char
     return QFB_OK;
 }
 
-// Apply classified gates to nbatch states of 2^n amplitudes of A (double2, or
-// float2 for the complex64 variant): register-blocked tile runs, one pass per
-// gate where a gate joins no run (or the tile shape says so).
+// Upload the phases of a group of windows and launch them.
 template <class A>
-int apply_gates_tiles(A *d, int n, int nbatch, const std::vector<HGate> &hg) {
-    const uint64_t nbasis = 1ull << n;
-    int b = 0, L = 0;
-    if (!gate_tile_shape(n, b, L) || hg.size() == 1) {
-        for (const HGate &h : hg) {
-            const int rc = launch_single_t(d, nbasis, nbatch, h);
-            if (rc) return rc;
-        }
-        return QFB_OK;
-    }
-    constexpr bool c64 = sizeof(A) == sizeof(float2);
-    std::vector<GatePlanWin> wins;
-    TilePlan tp;
-    std::vector<qfbt::TRun> runs;
-    const bool fused = g_gate_fused == 1 ||
-                       (g_gate_fused == 2 && sizeof(A) * nbasis * (uint64_t)nbatch >= kFusedMinBytes);
-    plan_gate_tiles(hg, n, b, L, wins, tp, runs, c64, fused);
+int launch_tile_runs(A *d, uint64_t nbasis, int nbatch, const std::vector<HGate> &hg,
+                     const std::vector<GatePlanWin> &wins, const std::vector<qfbt::TRun> &runs,
+                     const TilePlan &tp, bool fused) {
     // one upload of phases, ops, 4x4 matrices, chunk and thread tables and
     // the fused form
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const size_t bp = al(sizeof(qfbt::TPhase) * tp.ph.size());
-    const size_t bo = al(sizeof(qfbt::TOp) * tp.ops.size());
+    const size_t bo = al(sizeof(qfbt::TOp) * (tp.ops.size() + qfbt::kStageOps));
     const size_t bm = al(sizeof(double2) * tp.m4.size());
     const size_t bc = al(sizeof(uint64_t) * tp.chunks.size());
     const size_t bt = al(sizeof(uint32_t) * tp.threads.size());
@@ -1344,7 +1415,7 @@ int apply_gates_tiles(A *d, int n, int nbatch, const std::vector<HGate> &hg) {
     const uint32_t *d_th = (const uint32_t *)(ub + bp + bo + bm + bc);
     const qfbt::TSeg *d_sg = (const qfbt::TSeg *)(ub + bp + bo + bm + bc + bt);
     const double2 *d_fm = (const double2 *)(ub + bp + bo + bm + bc + bt + bs);
-    int rc = gate_tile_smem();
+    int rc = QFB_OK;
     for (size_t i = 0; i < wins.size() && rc == QFB_OK; ++i) {
         const GatePlanWin &pw = wins[i];
         if (pw.single >= 0) {
@@ -1354,7 +1425,7 @@ int apply_gates_tiles(A *d, int n, int nbatch, const std::vector<HGate> &hg) {
         const int tb = pw.w.b, R = tile_reg_bits(tb);
         const size_t smem0 = sizeof(A) * qfbt::tpad_size_of<A>(tb) + 16;
         const bool fz = fused && R == 3 && tb - R >= 5;
-        const size_t smem = fz ? (size_t)fused_bytes((int)smem0) : smem0;
+        const size_t smem = fz ? (size_t)fused_bytes((int)smem0) : (size_t)stage_bytes((int)smem0);
         const dim3 grid((unsigned)(nbasis >> tb), nbatch), block(1u << (tb - R));
 #define QFB_TILE(RR, FF)                                                                        \
     qfbt::k_gate_tile<RR, A, FF><<<grid, block, smem, t_stream>>>(d, nbasis, runs[i], d_ph, d_ops, \
@@ -1374,6 +1445,42 @@ int apply_gates_tiles(A *d, int n, int nbatch, const std::vector<HGate> &hg) {
     return rc;
 }
 
+// Apply classified gates to nbatch states of 2^n amplitudes of A (double2, or
+// float2 for the complex64 variant): register-blocked tile runs, one pass per
+// gate where a gate joins no run (or the tile shape says so).
+template <class A>
+int apply_gates_tiles(A *d, int n, int nbatch, const std::vector<HGate> &hg) {
+    const uint64_t nbasis = 1ull << n;
+    int b = 0, L = 0;
+    constexpr bool c64 = sizeof(A) == sizeof(float2);
+    if (!gate_tile_shape(n, b, L, c64) || hg.size() == 1) {
+        for (const HGate &h : hg) {
+            const int rc = launch_single_t(d, nbasis, nbatch, h);
+            if (rc) return rc;
+        }
+        return QFB_OK;
+    }
+    const bool fused = g_gate_fused == 1 ||
+                       (g_gate_fused == 2 && sizeof(A) * nbasis * (uint64_t)nbatch >= (c64 ? kFusedMinBytesC64 : kFusedMinBytes));
+    int rc = gate_tile_smem();
+    if (rc) return rc;
+    // planned, uploaded and launched a few windows at a time: the device runs one
+    // group while the host plans the next
+    WindowPlanner P(hg, n, b, L);
+    for (int group = 4; rc == QFB_OK; group = std::min(2 * group, 16)) {
+        std::vector<GatePlanWin> wins;
+        std::vector<WGate> wg;
+        GatePlanWin pw;
+        while ((int)wins.size() < group && P.next(pw, wg)) wins.push_back(pw);
+        if (wins.empty()) break;
+        TilePlan tp;
+        std::vector<qfbt::TRun> runs;
+        plan_tile_runs(wins, wg, tp, runs, c64, fused);
+        rc = launch_tile_runs<A>(d, nbasis, nbatch, hg, wins, runs, tp, fused);
+    }
+    return rc;
+}
+
 // Sum of |amplitude|^2 of a complex64 state, accumulated in FP64.
 __global__ void k_norm2_c64(const float2 *__restrict__ psi, uint64_t n, double2 *__restrict__ part) {
     double acc = 0.0;
@@ -1387,6 +1494,14 @@ __global__ void k_norm2_c64(const float2 *__restrict__ psi, uint64_t n, double2 
 }
 
 }  // namespace
+
+bool gate_tiles_on() { return g_gate_tile_bits >= 0 && g_gate_dense == 0; }
+
+int apply_gate_list(qfb_state s, const std::vector<qfb_gate> &gates) {
+    std::vector<HGate> hg;
+    const int rc = classify_gates(gates.data(), (int64_t)gates.size(), s->nqubit, "apply_gate_list", hg);
+    return rc || hg.empty() ? rc : apply_gates_tiles<double2>(s->d, s->nqubit, s->nbatch, hg);
+}
 
 // ===========================================================================
 // C ABI

@@ -124,6 +124,7 @@ struct TRun {
     int32_t b;       // tile bits
     int32_t ch0;     // first entry of this run's chunk table
     int32_t p0, np;  // phases
+    int32_t o0, th0; // the first phase's ops and thread table
 };
 // chunk table entry c of a run: the global offset of the tile's chunk c
 // (8 amplitudes on qubits 0..2), i.e. c's bits placed on the tile's qubits
@@ -360,57 +361,57 @@ __device__ __forceinline__ void ap_bswap(A (&v)[1 << R]) {
 #define QFBT_TT16(B, X) X(B + 0, 0, 0) X(B + 1, 0, 1) X(B + 2, 0, 2) X(B + 3, 0, 3) X(B + 4, 1, 0) X(B + 5, 1, 1) X(B + 6, 1, 2) X(B + 7, 1, 3) X(B + 8, 2, 0) X(B + 9, 2, 1) X(B + 10, 2, 2) X(B + 11, 2, 3) X(B + 12, 3, 0) X(B + 13, 3, 1) X(B + 14, 3, 2) X(B + 15, 3, 3)
 
 template <int R, class A>
-__device__ __forceinline__ void apply_op(A (&v)[1 << R], const TOp *__restrict__ op, uint32_t tl,
+__device__ __forceinline__ void apply_op(A (&v)[1 << R], const TOp *op, uint32_t tl,
                                          const double2 *__restrict__ m4) {
     using S = typename AmpT<A>::S;
     auto cv_ = [](double2 z) { return AmpT<A>::cvt(z); };
-    const uint4 hdr = __ldg(reinterpret_cast<const uint4 *>(op));
+    const uint4 hdr = *reinterpret_cast<const uint4 *>(op);
     if ((tl & hdr.y) != hdr.y) return;  // a control on one of the thread's bits is 0
     const uint32_t cm = hdr.w & 0xffu, cv = (hdr.w >> 16) & 0xffu;
     switch (hdr.x) {
 #define X(N, T)                                                                            \
     case N:                                                                                \
         for_pairs<R, T>(v, cm, cv,                                                         \
-                        FDense<A>{cv_(__ldg(&op->m[0])), cv_(__ldg(&op->m[1])),            \
-                                  cv_(__ldg(&op->m[2])), cv_(__ldg(&op->m[3]))});          \
+                        FDense<A>{cv_(op->m[0]), cv_(op->m[1]),            \
+                                  cv_(op->m[2]), cv_(op->m[3])});          \
         break;
         QFBT_T4(0, X)
 #undef X
 #define X(N, T)                                                                            \
     case N:                                                                                \
         for_pairs<R, T>(v, cm, cv,                                                         \
-                        FReal<A>{(S)__ldg(&op->m[0].x), (S)__ldg(&op->m[1].x),             \
-                                 (S)__ldg(&op->m[2].x), (S)__ldg(&op->m[3].x)});           \
+                        FReal<A>{(S)op->m[0].x, (S)op->m[1].x,             \
+                                 (S)op->m[2].x, (S)op->m[3].x});           \
         break;
         QFBT_T4(4, X)
 #undef X
 #define X(N, T)                                                                            \
     case N:                                                                                \
         for_pairs<R, T>(v, cm, cv,                                                         \
-                        FRxi<A>{(S)__ldg(&op->m[0].x), (S)__ldg(&op->m[1].y),              \
-                                (S)__ldg(&op->m[2].y), (S)__ldg(&op->m[3].x)});            \
+                        FRxi<A>{(S)op->m[0].x, (S)op->m[1].y,              \
+                                (S)op->m[2].y, (S)op->m[3].x});            \
         break;
         QFBT_T4(8, X)
 #undef X
 #define X(N, T) case N: for_pairs<R, T>(v, cm, cv, FPswap{}); break;
         QFBT_T4(12, X)
 #undef X
-#define X(N, T) case N: for_pairs<R, T>(v, cm, cv, FAnti<A>{cv_(__ldg(&op->m[1])), cv_(__ldg(&op->m[2]))}); break;
+#define X(N, T) case N: for_pairs<R, T>(v, cm, cv, FAnti<A>{cv_(op->m[1]), cv_(op->m[2])}); break;
         QFBT_T4(16, X)
 #undef X
-#define X(N, T) case N: ap_diag<R, T, 1>(v, cm, cv, cv_(__ldg(&op->m[0])), cv_(__ldg(&op->m[3]))); break;
+#define X(N, T) case N: ap_diag<R, T, 1>(v, cm, cv, cv_(op->m[0]), cv_(op->m[3])); break;
         QFBT_T4(20, X)
 #undef X
-#define X(N, T) case N: ap_diag<R, T, 2>(v, cm, cv, cv_(__ldg(&op->m[0])), cv_(__ldg(&op->m[3]))); break;
+#define X(N, T) case N: ap_diag<R, T, 2>(v, cm, cv, cv_(op->m[0]), cv_(op->m[3])); break;
         QFBT_T4(24, X)
 #undef X
-#define X(N, T) case N: ap_diag<R, T, 3>(v, cm, cv, cv_(__ldg(&op->m[0])), cv_(__ldg(&op->m[3]))); break;
+#define X(N, T) case N: ap_diag<R, T, 3>(v, cm, cv, cv_(op->m[0]), cv_(op->m[3])); break;
         QFBT_T4(28, X)
 #undef X
         case OPC_DIAG_THREAD: {
             // the diagonal bit is one of this thread's bits: one factor for all registers
             const bool one = (tl & hdr.z) != 0;
-            if ((hdr.w >> 8) & (one ? 2u : 1u)) ap_scale<R>(v, cm, cv, cv_(__ldg(&op->m[one ? 3 : 0])));
+            if ((hdr.w >> 8) & (one ? 2u : 1u)) ap_scale<R>(v, cm, cv, cv_(op->m[one ? 3 : 0]));
             break;
         }
 #define X(N, T, C) case N: ap_gen4<R, T, C>(v, m4 + (int)hdr.w); break;
@@ -567,6 +568,19 @@ __host__ __device__ __forceinline__ uint32_t tpad_size_of(int b) {
     return sizeof(A) == 16 ? tpad_size(b) : tpad8_size(b);
 }
 
+// Gate by gate: a phase's header, first ops and thread table as the CTA holds
+// them, copied while the phase before runs.  Read from global memory as they
+// came up, each was an L2 access on the path of a CTA that has nothing else to
+// do: 12 qubits, 8 layers (4 runs of 4 CTAs) 95 us on the device, this way
+// 70 us.
+constexpr int kStageOps = 16;
+struct TStage {
+    TPhase ph;
+    TOp ops[kStageOps];
+    uint32_t thr[1 << kMaxThreadBits];
+};
+static_assert(sizeof(TStage) % 16 == 0, "TStage is copied in 16-byte words");
+
 // One CTA per tile (blockIdx.x: tile position over the qubits outside Q;
 // blockIdx.y: batch slot); 2^(b-R) threads, 2^R amplitudes each.  A: double2
 // (complex128) or float2 (the complex64 throughput variant, arithmetic in
@@ -636,6 +650,24 @@ __global__ void __launch_bounds__(256, F ? 4 : R == 4 ? 1 : 3)
     } else {
         for (int c = tid; c < nch; c += nth)
             bulk_g2s(smem_u32(tile + tpad_of<A>((uint32_t)c << 3)), s + __ldg(&ch[c]), kChunk, bar_a);
+        TStage *st = reinterpret_cast<TStage *>(
+            t_smem + ((sizeof(A) * tpad_size_of<A>(b) + 16 + 15) & ~(size_t)15));
+        // phases follow one another in all three arrays (ops padded at the end)
+        auto fetch = [&](int p, int o0) {
+            constexpr int HW = (int)sizeof(TPhase) / 16, OW = kStageOps * (int)sizeof(TOp) / 16;
+            const int tw = nth / 4;  // 16-byte words of the thread table
+            const uint4 *hs = reinterpret_cast<const uint4 *>(phases + run.p0 + p);
+            const uint4 *os = reinterpret_cast<const uint4 *>(ops + o0);
+            const uint32_t *ts = threads + run.th0 + (size_t)p * nth;
+            TStage *d = st + (p & 1);
+            for (int i = tid; i < HW + OW + tw; i += nth) {
+                if (i < HW) cp_async16(smem_u32(reinterpret_cast<uint4 *>(&d->ph) + i), hs + i);
+                else if (i < HW + OW) cp_async16(smem_u32(reinterpret_cast<uint4 *>(d->ops) + i - HW), os + i - HW);
+                else cp_async16(smem_u32(d->thr + 4 * (i - HW - OW)), ts + 4 * (i - HW - OW));
+            }
+            cp_async_commit();
+        };
+        if (run.np > 0) fetch(0, run.o0);
         const uint64_t limit = g_tile_wait_limit_ns;
         if (limit == 0 || !mbar_wait_bounded(bar_a, 0, limit)) {
             // the copies did not complete in time: flag it, give them a second
@@ -643,22 +675,30 @@ __global__ void __launch_bounds__(256, F ? 4 : R == 4 ? 1 : 3)
             // released, and leave the tile unwritten
             if (tid == 0) atomicExch(&g_tile_wait_err, 1);
             mbar_wait_bounded(bar_a, 0, kWaitLimitNs);
+            cp_async_wait_all();
             return;
         }
+        cp_async_wait_all();
+        __syncthreads();
 
         for (int p = 0; p < run.np; ++p) {
-            const TPhase *ph = phases + run.p0 + p;
-            const uint32_t tw = __ldg(&threads[__ldg(&ph->th0) + tid]);
+            const TStage *ph = st + (p & 1);
+            const int o0 = ph->ph.o0, no = ph->ph.no;
+            if (p + 1 < run.np) fetch(p + 1, o0 + no);
+            const uint32_t tw = ph->thr[tid];
             const uint32_t tl = tw & 0xffffu;
             A *t0 = tile + (tw >> 16);
             A v[1 << R];
 #pragma unroll
-            for (int k = 0; k < (1 << R); ++k) v[k] = t0[__ldg(&ph->roff[k])];
-            const int o0 = __ldg(&ph->o0), o1 = o0 + __ldg(&ph->no);
-            for (int o = o0; o < o1; ++o) apply_op<R, A>(v, ops + o, tl, m4);
+            for (int k = 0; k < (1 << R); ++k) v[k] = t0[ph->ph.roff[k]];
+            for (int o = 0; o < no; ++o)
+                apply_op<R, A>(v, o < kStageOps ? ph->ops + o : ops + o0 + o, tl, m4);
 #pragma unroll
-            for (int k = 0; k < (1 << R); ++k) t0[__ldg(&ph->soff[k])] = v[k];
-            if (p + 1 < run.np) __syncthreads();
+            for (int k = 0; k < (1 << R); ++k) t0[ph->ph.soff[k]] = v[k];
+            if (p + 1 < run.np) {
+                cp_async_wait_all();
+                __syncthreads();
+            }
         }
         fence_async_smem();
         __syncthreads();

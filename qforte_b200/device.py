@@ -205,7 +205,7 @@ def gates_config(tile_bits=0, low_bits=3, reg_bits=0, dense=0, fused=None):
     most that many qubits into dense unitaries applied on the FP64 tensor
     cores instead (states of 10 qubits and more); fused True / False to apply
     each tile phase as fused 8 x 8 matrices on the FP64 tensor cores / its
-    gates one by one (None: fused for states larger than L2)."""
+    gates one by one (None: fused for states of 16 MiB and more)."""
     check(lib().qfb_gates_config(int(tile_bits), int(low_bits)), "qfb_gates_config")
     check(lib().qfb_gates_regs(int(reg_bits)), "qfb_gates_regs")
     check(lib().qfb_gates_dense(int(dense)), "qfb_gates_dense")
