@@ -36,7 +36,6 @@ using qfbs::v_rot;
 constexpr int kWinItems = 192;    // items of a window
 constexpr int kWinIdx = 12;       // bits of a local string or amplitude index
 constexpr int kWinBlobMax = 6144; // words of one class's blob
-constexpr int kWinGroup = 8;      // rounds whose inner products are reduced together
 constexpr int kWinThreads = 512;  // threads of a CTA, at most
 
 // One item: a step's pattern.
@@ -89,18 +88,64 @@ struct VCoef<true, V> {
 
 // Shared memory of a CTA of `spc` slots and `nw` warps, in this order: states
 // (each followed by 32 unused amplitudes), coefficients, items, round sums,
-// group buffers, blobs, ranks, amplitude indices, pair words.
+// blobs, ranks, amplitude indices, pair words.
 __host__ __device__ inline size_t win_al(size_t x) { return (x + 15) & ~(size_t)15; }
 inline size_t win_smem(const VWin &w, int spc, int nw, bool sweep, size_t elem) {
     const size_t cf = elem * (sweep ? 4 : 2) + 16;
     return win_al(elem * (size_t)(w.mab + 32) * spc * (sweep ? 2 : 1)) + cf * (size_t)w.nround * spc +
            sizeof(VItem) * w.nitem +
-           (sweep ? win_al(sizeof(double) * (size_t)w.nround * nw) +
-                        win_al(sizeof(double) * (size_t)nw * kWinGroup * 33)
-                  : 0) +
+           (sweep ? win_al(sizeof(double) * (size_t)w.nround * nw) : 0) +
            win_al(4 * (size_t)w.mwords) + win_al(2 * (size_t)w.mranks) + win_al(4 * (size_t)w.mab) +
            4 * ((size_t)w.nround << (5 + w.lg));
 }
+
+// A slot's states in shared memory: psi, and in the sweep sigma, interleaved
+// where the amplitudes are real (both in one 16-byte access).
+template <bool SWEEP, class V>
+struct WinState {
+    V *v, *w;
+    __device__ __forceinline__ WinState(unsigned char *raw, int sl, int stride, int lspc)
+        : v(reinterpret_cast<V *>(raw) + sl * stride), w(v + (stride << lspc)) {}
+    __device__ __forceinline__ void set(int i, V p, V s) {
+        v[i] = p;
+        if (SWEEP) w[i] = s;
+    }
+    __device__ __forceinline__ V psi(int i) const { return v[i]; }
+    __device__ __forceinline__ V sig(int i) const { return w[i]; }
+    // rotate the pair (l0, l1); sg: bit 31 is its sign.  The pair's inner product.
+    __device__ __forceinline__ double round(uint32_t l0, uint32_t l1, uint32_t sg, const VCoef<SWEEP, V> &co) {
+        const V v0 = v[l0], v1 = v[l1], a = v_flip(co.a, sg), b = v_flip(co.b, sg);
+        V x0 = V(), x1 = V();
+        if (SWEEP) {
+            x0 = w[l0];
+            x1 = w[l1];
+        }
+        v[l0] = v_rot(co.c, v0, a, v1);
+        v[l1] = v_rot(co.c, v1, b, v0);
+        if constexpr (SWEEP) {
+            w[l0] = v_rot(co.c, x0, a, x1);
+            w[l1] = v_rot(co.c, x1, b, x0);
+            return v_flip(v_ip_re(x0, x1, v0, v1, co.g, co.h), sg);
+        }
+        return 0.0;
+    }
+};
+template <>
+struct WinState<true, double> {
+    double2 *x;
+    __device__ __forceinline__ WinState(unsigned char *raw, int sl, int stride, int)
+        : x(reinterpret_cast<double2 *>(raw) + sl * stride) {}
+    __device__ __forceinline__ void set(int i, double p, double s) { x[i] = make_double2(p, s); }
+    __device__ __forceinline__ double psi(int i) const { return x[i].x; }
+    __device__ __forceinline__ double sig(int i) const { return x[i].y; }
+    __device__ __forceinline__ double round(uint32_t l0, uint32_t l1, uint32_t sg, const VCoef<true, double> &co) {
+        const double2 v0 = x[l0], v1 = x[l1];
+        const double a = v_flip(co.a, sg), b = v_flip(co.b, sg);
+        x[l0] = make_double2(v_rot(co.c, v0.x, a, v1.x), v_rot(co.c, v0.y, a, v1.y));
+        x[l1] = make_double2(v_rot(co.c, v1.x, b, v0.x), v_rot(co.c, v1.y, b, v0.y));
+        return v_flip(v_ip_re(v0.y, v1.y, v0.x, v1.x, co.g, co.h), sg);
+    }
+};
 
 // ang[i * B + s] = (cos, sin) of gamma_i * params[s][param_i]
 __global__ void __launch_bounds__(256) k_win_angles(const double *__restrict__ gamma,
@@ -138,18 +183,15 @@ __global__ void __launch_bounds__(kWinThreads) k_win(GLaunch L, VWin W, VTabs T,
     const int4 Bc = __ldg(reinterpret_cast<const int4 *>(T.cls + W.cb0 + cb));
     const int na = A.y, nb = Bc.y, nab = na * nb, stride = nab + 32;
     unsigned char *p = w_raw;
-    V *s_psi = reinterpret_cast<V *>(p), *s_sig = s_psi + (stride << lspc);
     p += win_al(sizeof(V) * (stride << lspc) * (SWEEP ? 2 : 1));
     VCoef<SWEEP, V> *s_cf = reinterpret_cast<VCoef<SWEEP, V> *>(p);  // [slot][round]
     p += sizeof(VCoef<SWEEP, V>) * nr << lspc;
     VItem *s_item = reinterpret_cast<VItem *>(p);
     p += sizeof(VItem) * ni;
-    double *s_sum = nullptr, *s_grp = nullptr;  // sums [warp][round]
+    double *s_sum = nullptr;  // sums [warp][round]
     if (SWEEP) {
         s_sum = reinterpret_cast<double *>(p);
         p += win_al(sizeof(double) * nr * nw);
-        s_grp = reinterpret_cast<double *>(p) + warp * kWinGroup * 33;
-        p += win_al(sizeof(double) * nw * kWinGroup * 33);
     }
     uint32_t *s_a = reinterpret_cast<uint32_t *>(p), *s_b = s_a + A.w;
     p += win_al(4 * (A.w + Bc.w));
@@ -196,17 +238,12 @@ __global__ void __launch_bounds__(kWinThreads) k_win(GLaunch L, VWin W, VTabs T,
 
     const int s0 = blockIdx.y << lspc;
     V *psi = reinterpret_cast<V *>(L.psi), *sig = reinterpret_cast<V *>(L.sig);
-    for (int i = tid; i < nab << lspc; i += nth) {
+    for (int i = tid; i < (nab + 32) << lspc; i += nth) {
         const int e = i >> lspc, sl = i & (spc - 1);
-        const bool in = s0 + sl < L.B;
-        const size_t g = (size_t)s_g[e] * L.B + s0 + sl;
-        s_psi[sl * stride + e] = in ? psi[g] : qfbs::v_zero(V());
-        if (SWEEP) s_sig[sl * stride + e] = in ? sig[g] : qfbs::v_zero(V());
-    }
-    for (int i = tid; i < 32 << lspc; i += nth) {
-        const int at = (i >> 5) * stride + nab + (i & 31);
-        s_psi[at] = qfbs::v_zero(V());
-        if (SWEEP) s_sig[at] = qfbs::v_zero(V());
+        const bool in = e < nab && s0 + sl < L.B;
+        const size_t g = in ? (size_t)s_g[e] * L.B + s0 + sl : 0;
+        WinState<SWEEP, V>(w_raw, sl, stride, lspc)
+            .set(e, in ? psi[g] : qfbs::v_zero(V()), SWEEP && in ? sig[g] : qfbs::v_zero(V()));
     }
     for (int i = tid; i < ni << lspc; i += nth) {
         const int s = s0 + (i & (spc - 1));
@@ -230,53 +267,33 @@ __global__ void __launch_bounds__(kWinThreads) k_win(GLaunch L, VWin W, VTabs T,
 
     const int sl = warp >> lg, t = tid & (G - 1);
     {
-        V *v = s_psi + sl * stride, *w = s_sig + sl * stride;
+        WinState<SWEEP, V> st(w_raw, sl, stride, lspc);
         const uint32_t *wp = s_w + t;
         const VCoef<SWEEP, V> *cp = s_cf + sl * nr;
         uint32_t word = *wp;
         VCoef<SWEEP, V> cf = *cp;
+        qfbs::RSum ip;
         for (int r = 0; r < nr; ++r) {
-            const uint32_t l0 = word & M, l1 = (word >> kWinIdx) & M, sg = word;
+            const uint32_t sg = word;
             const VCoef<SWEEP, V> co = cf;
-            const V v0 = v[l0], v1 = v[l1];
-            V x0 = V(), x1 = V();
-            if (SWEEP) {
-                x0 = w[l0];
-                x1 = w[l1];
-            }
             if (r + 1 < nr) {
                 wp += G;
                 ++cp;
                 word = *wp;
                 cf = *cp;
             }
-            const V a = v_flip(co.a, sg), b = v_flip(co.b, sg);
-            v[l0] = v_rot(co.c, v0, a, v1);
-            v[l1] = v_rot(co.c, v1, b, v0);
-            if constexpr (SWEEP) {
-                w[l0] = v_rot(co.c, x0, a, x1);
-                w[l1] = v_rot(co.c, x1, b, x0);
-            }
+            const double x = st.round(sg & M, (sg >> kWinIdx) & M, sg, co);
             if (lg == 0)
                 __syncwarp();
             else
                 asm volatile("bar.sync %0, %1;" ::"r"(sl + 1), "r"(G) : "memory");
             if constexpr (SWEEP) {
-                // lane sums wait in the group buffer until kWinGroup rounds are
-                // in: lanes 4 g .. 4 g + 3 then add round g's 32 values
-                s_grp[(r & (kWinGroup - 1)) * 33 + lane] =
-                    v_ip_re(x0, x1, v0, v1, v_flip(co.g, sg), v_flip(co.h, sg));
-                if ((r & (kWinGroup - 1)) == kWinGroup - 1 || r + 1 == nr) {
-                    __syncwarp();
-                    const int g8 = lane >> 2, r8 = (r & ~(kWinGroup - 1)) + g8;
-                    double x = 0.0;
-                    if (r8 <= r)
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) x += s_grp[g8 * 33 + (lane & 3) * 8 + j];
-                    x += __shfl_xor_sync(0xffffffffu, x, 1);
-                    x += __shfl_xor_sync(0xffffffffu, x, 2);
-                    if ((lane & 3) == 0 && r8 <= r) s_sum[warp * nr + r8] = x;
-                    __syncwarp();
+                ip.add(r & 3, x);
+                if ((r & 3) == 3 || r + 1 == nr) {
+                    const double sum = ip.sum();
+                    const int rr = (r & ~3) + (lane >> 2);
+                    if ((lane & 3) == 0 && rr <= r) s_sum[warp * nr + rr] = sum;
+                    ip = qfbs::RSum();
                 }
             }
         }
@@ -286,8 +303,9 @@ __global__ void __launch_bounds__(kWinThreads) k_win(GLaunch L, VWin W, VTabs T,
         const int e = i >> lspc, q = i & (spc - 1);
         if (s0 + q < L.B) {
             const size_t g = (size_t)s_g[e] * L.B + s0 + q;
-            psi[g] = s_psi[q * stride + e];
-            if (SWEEP) sig[g] = s_sig[q * stride + e];
+            const WinState<SWEEP, V> st(w_raw, q, stride, lspc);
+            psi[g] = st.psi(e);
+            if (SWEEP) sig[g] = st.sig(e);
         }
     }
     if (SWEEP) {
