@@ -503,9 +503,10 @@ int launch_single_t(A *d, uint64_t nbasis, int nbatch, const HGate &h) {
 
 int launch_single(qfb_state s, const HGate &h) { return launch_single_t(s->d, s->nbasis, s->nbatch, h); }
 
-// Default tile bits: 10 where the fused form is taken, 11 for smaller complex128
-// states (20 layers, us, 10 / 11: 12 qubits 213 / 197, 18 qubits 395 / 367).
-constexpr int kGateTileDefault = 10, kGateTileSmall = 11, kGateTileSmallQubits = 19;
+// Default tile bits: 11 for complex128 (20 layers, us, 10 / 11: gate by gate 12
+// qubits 213 / 197, 18 qubits 395 / 367; fused 21 qubits 800 / 777, 23 qubits 2,756 /
+// 2,708, 27 qubits 45,791 / 45,020), 10 for complex64.
+constexpr int kGateTileDefault = 11, kGateTileC64 = 10;
 constexpr int kGateTileMax = 12;
 int g_gate_tile_bits = 0;  // 0: kGateTileDefault; -1: one pass per gate
 int g_gate_low_bits = 3;
@@ -532,7 +533,7 @@ inline int tile_reg_bits(int b) {
 // Tile shape for an n-qubit state: false when every gate takes its own pass
 // (tile_bits -1, or a state smaller than two 128-byte chunks).
 bool gate_tile_shape(int n, int &b, int &L, bool c64 = false) {
-    b = g_gate_tile_bits != 0 ? g_gate_tile_bits : (c64 || n > kGateTileSmallQubits) ? kGateTileDefault : kGateTileSmall;
+    b = g_gate_tile_bits != 0 ? g_gate_tile_bits : c64 ? kGateTileC64 : kGateTileDefault;
     if (b < 0 || n < 4) return false;
     L = std::max(3, std::min(g_gate_low_bits, n));
     b = std::max(4, std::min(b, n));
@@ -911,8 +912,9 @@ void fuse_phase(TilePlan &tp, const qfbt::TPhase &ph, int b, bool c64) {
     // thread table of a phase with variant bits Dv: vector-index bits 0-2 from
     // the other thread bits, chosen by residue class (tile bit mod 3) so the
     // quarter-warp accesses of the B and D fragments spread over the banks;
-    // then Dv; then the rest
-    auto table = [&](uint32_t Dv) {
+    // then the rest; then Dv (a warp's vectors, index bits 0-4, then share a
+    // variant, and the warp loads one matrix).  in_warp: Dv's bits below bit 5.
+    auto table = [&](uint32_t Dv, uint32_t &in_warp) {
         const int c0 = rbit[0] % 3, c1 = rbit[1] % 3, c2 = 3 - c0 - c1;
         const int want[3] = {c2 >= 0 && c2 < 3 && c2 != c0 && c2 != c1 ? c2 : -1, c1, c2};
         uint32_t free_bits = T & ~Dv;
@@ -927,9 +929,13 @@ void fuse_phase(TilePlan &tp, const qfbt::TPhase &ph, int b, bool c64) {
             free_bits &= ~(1u << pick);
         }
         for (int p = 0; p < b; ++p)
-            if (Dv >> p & 1u) tb.push_back(p);
-        for (int p = 0; p < b; ++p)
             if (free_bits >> p & 1u) tb.push_back(p);
+        in_warp = 0;
+        for (int p = 0; p < b; ++p)
+            if (Dv >> p & 1u) {
+                if (tb.size() < 5) in_warp |= 1u << p;
+                tb.push_back(p);
+            }
         const int th0 = (int)tp.threads.size();
         push_threads(tp.threads, tb, toff);
         return th0;
@@ -950,12 +956,14 @@ void fuse_phase(TilePlan &tp, const qfbt::TPhase &ph, int b, bool c64) {
             Dv |= segs[j].D;
             ++j;
         }
-        q.th0 = table(Dv);
+        uint32_t in_warp = 0;
+        q.th0 = table(Dv, in_warp);
         q.s0 = (int)tp.segs.size();
         q.m0 = (int)tp.fm.size();
         for (size_t k = i; k < j; ++k) {
             qfbt::TSeg h = segs[k].h;
             h.m0 = (uint32_t)q.m0 + (h.m0 - base);
+            if (segs[k].D & in_warp) h.dsel |= qfbt::kVarInWarp;
             tp.segs.push_back(h);
         }
         const uint32_t end = j < segs.size() ? segs[j].h.m0 : (uint32_t)mats.size();
@@ -1844,7 +1852,7 @@ int qfb_gates_fused_plan(const qfb_gate *gates, int64_t ngates, int nqubit, int 
     int64_t np = 0, ns = 0, ne = 0;
     const bool c64 = complex64 != 0;
     auto toff = [c64](uint32_t l) { return c64 ? qfbt::tpad8(l) : qfbt::tpad(l); };
-    if (gate_tile_shape(nqubit, b, L) && ngates > 1) {
+    if (gate_tile_shape(nqubit, b, L, c64) && ngates > 1) {
         std::vector<GatePlanWin> wins;
         TilePlan tp;
         std::vector<qfbt::TRun> runs;

@@ -92,8 +92,8 @@ static_assert(sizeof(TPhase) == 160, "TPhase layout");
 //    thread bits, the bit of a diagonal on a thread bit that is also
 //    controlled by register bits), at most kMaxVarBits of them; the host
 //    builds one matrix per assignment of those bits and orders the thread
-//    table so that the phase's variant bits are vector-index bits 3 and up:
-//    all 8 columns of an n-block share one matrix.
+//    table so that the phase's variant bits are the highest vector-index bits:
+//    all 8 columns of an n-block share one matrix, and as a rule all of a warp.
 //  * Diagonal factors that depend on thread bits alone (a diagonal on a
 //    thread bit, controlled by thread bits or not at all) scale all 8
 //    amplitudes of a vector alike and commute with everything else in the
@@ -108,10 +108,11 @@ static_assert(sizeof(TPhase) == 160, "TPhase layout");
 // splits a phase whose segments hold more than kStage matrix entries into
 // phases on the same registers.
 constexpr int kMaxVarBits = 3;
+constexpr uint32_t kVarInWarp = 1u << 31;  // a segment's variant changes within a warp
 constexpr int kStage = 512;  // matrix entries of one phase
 struct TSeg {
     uint32_t m0;    // first entry of this segment's matrices
-    uint32_t dsel;  // variant bits: tile bit positions, 4 bits each
+    uint32_t dsel;  // variant bits: tile bit positions, 4 bits each; kVarInWarp
     uint32_t mm;    // register bits the matrix mixes (host statistics)
     uint32_t nd;    // number of variant bits
 };
@@ -481,7 +482,7 @@ __device__ __forceinline__ void fused_phase(const TPhase *__restrict__ ph, const
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 const int tv = warp * 32 + (np + u) * 8;  // first vector of the n-block
-                if (np + u == 0 || h.w != 0) {
+                if (np + u == 0 || (h.y & kVarInWarp)) {
                     const double2 *mv = mseg + 64u * seg_variant(thr[tv] & 0xffffu, h);
                     a0[u] = __ldg(mv + lane);
                     a1[u] = __ldg(mv + 32 + lane);

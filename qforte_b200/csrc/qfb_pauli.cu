@@ -5080,6 +5080,7 @@ struct qfb_pack_s {
     size_t smem = 0;    // psi, sigma and the constants of the largest member
     size_t smem_h = 0;  // psi alone
     int chunk = 1;      // items a group of launches takes
+    int Q = 1;          // most CTAs a member's H rows are split over
     size_t bytes = 0, maxpart = 0;
     void *blob = nullptr;
     qfbs::PackMember *d_mem = nullptr;
@@ -5128,7 +5129,8 @@ extern "C" int qfb_pack_create(const qfb_ucc *members, int nmembers, int capacit
         m.nsec = L.nsec;
         m.ref_i = L.ref_i;
         m.nparam = u->nparam;
-        m.pad = 0;
+        m.Q = std::max(1, std::min(kPackSlices, L.nsec / 128));
+        p->Q = std::max(p->Q, m.Q);
         m.fwd = L.fwd;
         m.sweep = L.sweep;
         m.rowptr = L.rowptr;
@@ -5221,10 +5223,8 @@ extern "C" int qfb_pack_launch(qfb_pack p, int nitems) {
     for (int i0 = 0; i0 < nitems; i0 += p->chunk) {
         const int n = std::min(p->chunk, nitems - i0);
         const size_t at = (size_t)i0 * p->maxparam;
-        // about four CTAs an SM for the H rows
-        const int Q = std::max(1, std::min(kPackSlices, 4 * sm_count() / n));
         const qfbs::PackLaunch L{p->d_mem, p->items + i0, p->nmem, p->maxparam, p->params + at,
-                                 p->energy + i0, p->grad + at, p->partial, p->maxpart, p->save, p->maxsec, Q,
+                                 p->energy + i0, p->grad + at, p->partial, p->maxpart, p->save, p->maxsec, p->Q,
                                  p->epart, p->count};
         const int rc = p->sreal ? pack_group<double>(p, L, n) : pack_group<double2>(p, L, n);
         if (rc) return rc;

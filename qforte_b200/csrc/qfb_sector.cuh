@@ -801,7 +801,8 @@ __global__ void __launch_bounds__(kStepThreads, 1) k_sector_forward_pr(SLaunch L
 // problem (its sector, forward and sweep rounds, H rows on the sector and the
 // sweep rounds of each parameter).
 struct PackMember {
-    int nsec, ref_i, nparam, pad;
+    int nsec, ref_i, nparam;
+    int Q;  // CTAs its H rows are split over (its own: an energy's sum never depends on the mix)
     RStream fwd, sweep;
     const int32_t *rowptr;
     const uint32_t *col;
@@ -820,7 +821,7 @@ struct PackLaunch {
     double *partial;       // [items][maxpart]: the sweeps' warp sums
     size_t maxpart;
     void *save;            // V [items][2][maxsec]: psi, sigma
-    int maxsec, Q;         // Q: CTAs an item's H rows are split over
+    int maxsec, Q;         // Q: the most CTAs of a member
     double *epart;         // [items][Q]
     unsigned *count;       // [items]: CTAs done
 };
@@ -918,7 +919,7 @@ __device__ __forceinline__ bool pack_item(const PackLaunch &P, int x, int2 &it) 
 // gradient when items[x].y != 0; energy into energy[x], gradient into
 // grad[x][0 .. nparam).  Three launches serve parameter sets of different
 // problems side by side: the forward programs (a CTA per item), sigma = H psi
-// and the energies (Q CTAs per item: one alone takes ~400 us for the 1.8 M row
+// and the energies (up to 16 CTAs per item: one alone takes ~400 us for the 1.8 M row
 // entries of a 16-qubit problem), the reverse sweeps (a CTA per item).
 template <class V>
 __global__ void __launch_bounds__(kStepThreads, 2) k_pack_forward(PackLaunch P) {
@@ -944,19 +945,20 @@ __global__ void __launch_bounds__(kStepThreads, 2) k_pack_h(PackLaunch P) {
     const int2 it = P.items[x];
     if ((unsigned)it.x >= (unsigned)P.nmem) return;
     const PackMember m = P.members[it.x];
+    if (q >= m.Q) return;
     V *psi = reinterpret_cast<V *>(s_raw);
     V *sv = reinterpret_cast<V *>(P.save) + (size_t)x * 2 * P.maxsec;
     for (int i = tid; i < m.nsec; i += blockDim.x) psi[i] = sv[i];
     __syncthreads();
-    const int r0 = (int)((int64_t)q * m.nsec / P.Q), r1 = (int)((int64_t)(q + 1) * m.nsec / P.Q);
+    const int r0 = (int)((int64_t)q * m.nsec / m.Q), r1 = (int)((int64_t)(q + 1) * m.nsec / m.Q);
     const double e = p_hpsi<V>(m, r0, r1, psi, sv + P.maxsec, s_red);
     if (tid == 0) {
         P.epart[(size_t)x * P.Q + q] = e;
         __threadfence();
-        if (atomicAdd(&P.count[x], 1u) == (unsigned)P.Q - 1u) {
+        if (atomicAdd(&P.count[x], 1u) == (unsigned)m.Q - 1u) {
             __threadfence();
             double t = 0.0;
-            for (int k = 0; k < P.Q; ++k) t += __ldcg(&P.epart[(size_t)x * P.Q + k]);
+            for (int k = 0; k < m.Q; ++k) t += __ldcg(&P.epart[(size_t)x * P.Q + k]);
             P.energy[x] = t;
             P.count[x] = 0u;
         }
