@@ -64,8 +64,9 @@ struct qfb_state_s {
     double2 *d;       // [nbatch][nbasis]
 };
 
-// A gate list in register-blocked tiles (qfb_core.cu), and whether gate lists
-// are applied that way (qfb_gates_config, qfb_gates_dense).
+// A gate list in register-blocked tiles (qfb_core.cu), products of gates rounded
+// once, and whether gate lists are applied that way (qfb_gates_config,
+// qfb_gates_dense).
 bool gate_tiles_on();
 int apply_gate_list(qfb_state s, const std::vector<qfb_gate> &gates);
 

@@ -758,35 +758,46 @@ bool is_swap4(const WGate &g) {
 
 // ---- the fused form of a phase ----------------------------------------------
 
-inline double2 cmul_h(double2 a, double2 b) {
-    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-inline double2 cadd_h(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+
+// Complex numbers of the fused products on the host.
+template <class T>
+struct CplxH {
+    T x = 0, y = 0;
+    CplxH() = default;
+    CplxH(T a, T b) : x(a), y(b) {}
+    explicit CplxH(double2 v) : x(v.x), y(v.y) {}
+    CplxH operator*(const CplxH &b) const { return CplxH(x * b.x - y * b.y, x * b.y + y * b.x); }
+    CplxH operator+(const CplxH &b) const { return CplxH(x + b.x, y + b.y); }
+    double2 round() const { return make_double2((double)x, (double)y); }
+};
 
 // One op of a phase on the rows of an 8 x 8 matrix (row k: what register k
 // receives), for the thread with tile bits tl, as qfbt::apply_op applies it.
-void top_apply_rows(const qfbt::TOp &o, const double2 *m4, uint32_t tl, double2 (*v)[8]) {
+template <class T>
+void top_apply_rows(const qfbt::TOp &o, const double2 *m4, uint32_t tl, CplxH<T> (*v)[8]) {
     if ((tl & o.tctl) != o.tctl) return;
     const uint32_t cm = o.aux & 0xffu, cv = (o.aux >> 16) & 0xffu, opc = o.opc;
-    auto scale = [](double2 f, double2 *r) {
-        for (int c = 0; c < 8; ++c) r[c] = cmul_h(f, r[c]);
+    using C = CplxH<T>;
+    auto scale = [](double2 f, C *r) {
+        for (int c = 0; c < 8; ++c) r[c] = C(f) * r[c];
     };
     if (opc < qfbt::OPC_DIAG) {
         const uint32_t kind = opc / 4, tb = 1u << (opc % 4);
+        const C m[4] = {C(o.m[0]), C(o.m[1]), C(o.m[2]), C(o.m[3])};
         for (uint32_t k = 0; k < 8; ++k) {
             if ((k & tb) || (k & cm) != cv) continue;
-            double2 *r0 = v[k], *r1 = v[k | tb];
+            C *r0 = v[k], *r1 = v[k | tb];
             for (int c = 0; c < 8; ++c) {
-                const double2 x0 = r0[c], x1 = r1[c];
+                const C x0 = r0[c], x1 = r1[c];
                 if (kind == qfbt::OP_PSWAP) {
                     r0[c] = x1;
                     r1[c] = x0;
                 } else if (kind == qfbt::OP_ANTI) {
-                    r0[c] = cmul_h(o.m[1], x1);
-                    r1[c] = cmul_h(o.m[2], x0);
+                    r0[c] = m[1] * x1;
+                    r1[c] = m[2] * x0;
                 } else {
-                    r0[c] = cadd_h(cmul_h(o.m[0], x0), cmul_h(o.m[1], x1));
-                    r1[c] = cadd_h(cmul_h(o.m[2], x0), cmul_h(o.m[3], x1));
+                    r0[c] = m[0] * x0 + m[1] * x1;
+                    r1[c] = m[2] * x0 + m[3] * x1;
                 }
             }
         }
@@ -810,12 +821,12 @@ void top_apply_rows(const qfbt::TOp &o, const double2 *m4, uint32_t tl, double2 
         const double2 *m = m4 + o.aux;
         for (uint32_t k = 0; k < 8; ++k) {
             if (k & (tb | cb)) continue;
-            double2 *r[4] = {v[k], v[k | tb], v[k | cb], v[k | tb | cb]};
+            C *r[4] = {v[k], v[k | tb], v[k | cb], v[k | tb | cb]};
             for (int c = 0; c < 8; ++c) {
-                const double2 x[4] = {r[0][c], r[1][c], r[2][c], r[3][c]};
+                const C x[4] = {r[0][c], r[1][c], r[2][c], r[3][c]};
                 for (int i = 0; i < 4; ++i) {
-                    double2 acc = make_double2(0.0, 0.0);
-                    for (int j = 0; j < 4; ++j) acc = cadd_h(acc, cmul_h(m[4 * i + j], x[j]));
+                    C acc;
+                    for (int j = 0; j < 4; ++j) acc = acc + C(m[4 * i + j]) * x[j];
                     r[i][c] = acc;
                 }
             }
@@ -837,6 +848,7 @@ void top_apply_rows(const qfbt::TOp &o, const double2 *m4, uint32_t tl, double2 
 // entries); otherwise the phase is split into phases on the same registers,
 // each with its own thread table: all but the last store to the load
 // offsets, the next loads them again.
+template <class F>
 void fuse_phase(TilePlan &tp, const qfbt::TPhase &ph, int b, bool c64) {
     constexpr int R = 3;
     auto toff = [c64](uint32_t l) { return c64 ? qfbt::tpad8(l) : qfbt::tpad(l); };
@@ -857,7 +869,7 @@ void fuse_phase(TilePlan &tp, const qfbt::TPhase &ph, int b, bool c64) {
     const uint32_t T = ((1u << b) - 1u) & ~S;  // thread bits
     std::vector<int> run_ops;
     std::vector<qfbt::TOp> fac_ops;
-    double2 mat[NR][NR];
+    CplxH<F> mat[NR][NR];
     struct Seg {
         uint32_t D;  // variant bits
         qfbt::TSeg h;
@@ -880,14 +892,14 @@ void fuse_phase(TilePlan &tp, const qfbt::TPhase &ph, int b, bool c64) {
             for (size_t j = 0; j < dbits.size(); ++j)
                 if (x >> j & 1u) tl |= 1u << dbits[j];
             for (uint32_t r = 0; r < NR; ++r)
-                for (uint32_t c = 0; c < NR; ++c) mat[r][c] = make_double2(r == c ? 1.0 : 0.0, 0.0);
+                for (uint32_t c = 0; c < NR; ++c) mat[r][c] = CplxH<F>(r == c ? 1 : 0, 0);
             for (int oi : run_ops) top_apply_rows(tp.ops[oi], tp.m4.data(), tl, mat);
             for (uint32_t r = 0; r < NR; ++r)
                 for (uint32_t c = 0; c < NR; ++c)
-                    if (mat[r][c].x != 0.0 || mat[r][c].y != 0.0) sg.h.mm |= r ^ c;
+                    if (mat[r][c].x != 0 || mat[r][c].y != 0) sg.h.mm |= r ^ c;
             for (uint32_t kb = 0; kb < 2; ++kb)
                 for (uint32_t lane = 0; lane < 32; ++lane)
-                    mats.push_back(mat[lane >> 2][4 * kb + (lane & 3)]);
+                    mats.push_back(mat[lane >> 2][4 * kb + (lane & 3)].round());
 
         }
         segs.push_back(sg);
@@ -974,13 +986,13 @@ void fuse_phase(TilePlan &tp, const qfbt::TPhase &ph, int b, bool c64) {
         if (first && !fac_ops.empty()) {
             q.sc = (int)tp.fm.size();
             for (uint32_t t = 0; t < nth; ++t) {
-                double2 f = make_double2(1.0, 0.0);
+                CplxH<F> f(1, 0);
                 const uint32_t tl = tp.threads[q.th0 + t] & 0xffffu;
                 for (const qfbt::TOp &o : fac_ops) {
                     const uint32_t one = (tl & o.tbit) != 0;
-                    if ((tl & o.tctl) == o.tctl && (o.aux >> (8 + one) & 1u)) f = cmul_h(o.m[one ? 3 : 0], f);
+                    if ((tl & o.tctl) == o.tctl && (o.aux >> (8 + one) & 1u)) f = CplxH<F>(o.m[one ? 3 : 0]) * f;
                 }
-                tp.fm.push_back(f);
+                tp.fm.push_back(f.round());
             }
         }
         if (j < segs.size())  // more segments follow on the same registers
@@ -998,10 +1010,11 @@ void fuse_phase(TilePlan &tp, const qfbt::TPhase &ph, int b, bool c64) {
 // gate that cannot join blocks its bits for the rest of the scan, so only
 // gates on disjoint qubits change order.
 // c64: shared offsets in the complex64 tile layout (qfbt::tpad8).
-// fused: the phases' fused form where it applies (R = 3, at least 32
+// fine: the fused matrices are multiplied out in extended precision and rounded
+// once.  fused: the phases' fused form where it applies (R = 3, at least 32
 // threads).
 void plan_tile_phases(const WGate *g, int ng, int b, int R, qfbt::TRun &run, TilePlan &tp,
-                      bool c64 = false, bool fused = false) {
+                      bool c64 = false, bool fused = false, bool fine = false) {
     auto toff = [c64](uint32_t l) { return c64 ? qfbt::tpad8(l) : qfbt::tpad(l); };
     std::vector<uint32_t> mix((size_t)ng), qm((size_t)ng);
     for (int i = 0; i < ng; ++i) {
@@ -1173,7 +1186,7 @@ void plan_tile_phases(const WGate *g, int ng, int b, int R, qfbt::TRun &run, Til
         }
         ph.no = (int)tp.ops.size() - ph.o0;
         if (fuse)
-            fuse_phase(tp, ph, b, c64);
+            fine ? fuse_phase<long double>(tp, ph, b, c64) : fuse_phase<double>(tp, ph, b, c64);
         else
             tp.ph.push_back(ph);
     }
@@ -1341,7 +1354,7 @@ int apply_gates_dense(qfb_state s, const std::vector<HGate> &hg, int K) {
 
 // The phases of each window's run.
 void plan_tile_runs(const std::vector<GatePlanWin> &wins, const std::vector<WGate> &wg, TilePlan &tp,
-                    std::vector<qfbt::TRun> &runs, bool c64, bool fused) {
+                    std::vector<qfbt::TRun> &runs, bool c64, bool fused, bool fine = false) {
     runs.assign(wins.size(), qfbt::TRun{});
     for (size_t i = 0; i < wins.size(); ++i) {
         const GatePlanWin &pw = wins[i];
@@ -1355,7 +1368,7 @@ void plan_tile_runs(const std::vector<GatePlanWin> &wins, const std::vector<WGat
             for (size_t c = 0; c < half; ++c)
                 tp.chunks.push_back(tp.chunks[(size_t)r.ch0 + c] | (m & (~m + 1)));
         plan_tile_phases(wg.data() + pw.w.g0, pw.w.ng, pw.w.b, tile_reg_bits(pw.w.b), r, tp, c64,
-                         fused);
+                         fused, fine);
     }
 }
 
@@ -1457,7 +1470,7 @@ int launch_tile_runs(A *d, uint64_t nbasis, int nbatch, const std::vector<HGate>
 // float2 for the complex64 variant): register-blocked tile runs, one pass per
 // gate where a gate joins no run (or the tile shape says so).
 template <class A>
-int apply_gates_tiles(A *d, int n, int nbatch, const std::vector<HGate> &hg) {
+int apply_gates_tiles(A *d, int n, int nbatch, const std::vector<HGate> &hg, bool fine = false) {
     const uint64_t nbasis = 1ull << n;
     int b = 0, L = 0;
     constexpr bool c64 = sizeof(A) == sizeof(float2);
@@ -1483,7 +1496,7 @@ int apply_gates_tiles(A *d, int n, int nbatch, const std::vector<HGate> &hg) {
         if (wins.empty()) break;
         TilePlan tp;
         std::vector<qfbt::TRun> runs;
-        plan_tile_runs(wins, wg, tp, runs, c64, fused);
+        plan_tile_runs(wins, wg, tp, runs, c64, fused, fine);
         rc = launch_tile_runs<A>(d, nbasis, nbatch, hg, wins, runs, tp, fused);
     }
     return rc;
@@ -1508,7 +1521,7 @@ bool gate_tiles_on() { return g_gate_tile_bits >= 0 && g_gate_dense == 0; }
 int apply_gate_list(qfb_state s, const std::vector<qfb_gate> &gates) {
     std::vector<HGate> hg;
     const int rc = classify_gates(gates.data(), (int64_t)gates.size(), s->nqubit, "apply_gate_list", hg);
-    return rc || hg.empty() ? rc : apply_gates_tiles<double2>(s->d, s->nqubit, s->nbatch, hg);
+    return rc || hg.empty() ? rc : apply_gates_tiles<double2>(s->d, s->nqubit, s->nbatch, hg, true);
 }
 
 // ===========================================================================
