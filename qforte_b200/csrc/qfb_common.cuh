@@ -9,6 +9,7 @@
 #include <atomic>
 #include <cstdio>
 #include <string>
+#include <vector>
 
 #include "../../include/qfb.h"
 
