@@ -65,11 +65,19 @@ struct qfb_state_s {
     double2 *d;       // [nbatch][nbasis]
 };
 
-// A gate list in register-blocked tiles (qfb_core.cu), products of gates rounded
-// once, and whether gate lists are applied that way (qfb_gates_config,
-// qfb_gates_dense).
+// exp(i phi P) of a Pauli string P (masks x and z, ny = popcount(x & z) mod 4) on
+// at most two qubits.
+struct PauliRot {
+    uint64_t x, z;
+    int ny;
+    double phi;
+};
+
+// Such exponentials in list order by register-blocked tiles (qfb_core.cu),
+// products rounded once, and whether gate lists are applied that way
+// (qfb_gates_config, qfb_gates_dense).
 bool gate_tiles_on();
-int apply_gate_list(qfb_state s, const std::vector<qfb_gate> &gates);
+int apply_rotations(qfb_state s, const std::vector<PauliRot> &rots);
 
 // ---- device side ----------------------------------------------------------
 

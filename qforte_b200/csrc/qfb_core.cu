@@ -1518,10 +1518,73 @@ __global__ void k_norm2_c64(const float2 *__restrict__ psi, uint64_t n, double2 
 
 bool gate_tiles_on() { return g_gate_tile_bits >= 0 && g_gate_dense == 0; }
 
-int apply_gate_list(qfb_state s, const std::vector<qfb_gate> &gates) {
+// exp(i phi P) = cos phi + i sin phi P: one-qubit strings and products of two Z (a Z
+// rotation, then a controlled one) as 2 x 2 matrices, the rest as 4 x 4.  Kinds and
+// nonzero entries follow from the string alone: classify_gate's threshold would
+// take a string for the identity as soon as cos phi rounds to 1.
+static void rot_gates(const PauliRot &p, std::vector<HGate> &out) {
+    const double c = std::cos(p.phi), s = std::sin(p.phi);
+    const uint64_t q = p.x | p.z;
+    const int t = q ? __builtin_ctzll(q) : 0;
+    const int hi = q & (q - 1) ? 63 - __builtin_clzll(q) : t;
+    auto gate2 = [&](int kind, int ctrl) -> Gate2 & {
+        HGate h{};
+        h.form = 0;
+        h.qubits = 1ull << t | (ctrl < 0 ? 0ull : 1ull << ctrl);
+        h.g2.kind = kind;
+        h.g2.t = t;
+        h.g2.c = ctrl;
+        h.g2.diag_set = kind == K_DIAG ? 3 : 0;
+        out.push_back(h);
+        return out.back().g2;
+    };
+    if (p.x == 0 && hi != t) {  // Z Z: e^{i phi Z_t}, then e^{-2 i phi Z_t} where the other is 1
+        Gate2 &a = gate2(K_DIAG, -1);
+        a.a = make_double2(c, s);
+        a.d = make_double2(c, -s);
+        const double c2 = std::cos(2.0 * p.phi), s2 = std::sin(2.0 * p.phi);
+        Gate2 &b = gate2(K_DIAG, hi);
+        b.a = make_double2(c2, -s2);
+        b.d = make_double2(c2, s2);
+        return;
+    }
+    // basis index bit 0: qubit t, bit 1: qubit hi
+    const int dim = hi == t ? 2 : 4;
+    const int xl = (int)(p.x >> t & 1) | (hi == t ? 0 : (int)(p.x >> hi & 1) << 1);
+    const int zl = (int)(p.z >> t & 1) | (hi == t ? 0 : (int)(p.z >> hi & 1) << 1);
+    double2 m[16] = {};
+    uint32_t nz = 0;
+    for (int j = 0; j < dim; ++j) {
+        m[dim * j + j].x += c;
+        // i sin phi i^ny (-1)^popcount(j & z) at row j ^ x
+        const int ph = (p.ny + 1 + 2 * (__builtin_popcount(j & zl) & 1)) & 3, at = dim * (j ^ xl) + j;
+        if (ph & 1) m[at].y += ph == 1 ? s : -s;
+        else m[at].x += ph == 0 ? s : -s;
+        nz |= 1u << (dim * j + j) | 1u << at;
+    }
+    if (dim == 2) {
+        Gate2 &g = gate2(xl ? K_DENSE : K_DIAG, -1);
+        g.a = m[0];
+        g.b = m[1];
+        g.cc = m[2];
+        g.d = m[3];
+        return;
+    }
+    HGate h{};
+    h.form = 1;
+    h.qubits = q;
+    h.g4.t = t;
+    h.g4.c = hi;
+    h.g4.nz = nz;
+    for (int k = 0; k < 16; ++k) h.g4.m[k] = m[k];
+    out.push_back(h);
+}
+
+int apply_rotations(qfb_state s, const std::vector<PauliRot> &rots) {
     std::vector<HGate> hg;
-    const int rc = classify_gates(gates.data(), (int64_t)gates.size(), s->nqubit, "apply_gate_list", hg);
-    return rc || hg.empty() ? rc : apply_gates_tiles<double2>(s->d, s->nqubit, s->nbatch, hg, true);
+    hg.reserve(rots.size() + rots.size() / 2);
+    for (const PauliRot &p : rots) rot_gates(p, hg);
+    return hg.empty() ? QFB_OK : apply_gates_tiles<double2>(s->d, s->nqubit, s->nbatch, hg, true);
 }
 
 // ===========================================================================

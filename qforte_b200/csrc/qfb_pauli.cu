@@ -2045,53 +2045,20 @@ static int enqueue_gradient(const qfb_prog_s *kp, const qfb_prog_s *up, double2 
     return QFB_OK;
 }
 
-// A program's strings as gates, when each acts on at most two qubits: exp(i phi
-// P) = cos phi + i sin phi P, one-qubit strings and products of two Z (a Z
-// rotation, then a controlled one) as 2 x 2 matrices, the rest as 4 x 4.
-static bool prog_gates(const qfb_prog_s *p, const double *params, int sign, std::vector<qfb_gate> &out) {
+// A program's strings in the order they apply, when each acts on at most two
+// qubits.
+static bool prog_rotations(const qfb_prog_s *p, const double *params, int sign, std::vector<PauliRot> &out) {
     const size_t n = p->h_strs.size();
     std::vector<uint64_t> x(n);
     for (const StepDev &st : p->h_steps)
         for (int k = st.s0; k < st.s0 + st.ns; ++k) x[(size_t)k] = st.x;
     for (size_t k = 0; k < n; ++k)
         if (__builtin_popcountll(x[k] | p->h_strs[k].z) > 2) return false;
-    out.reserve(n + n / 2);
-    auto gate = [&](int t, int c) -> qfb_gate & {
-        out.push_back(qfb_gate{});
-        out.back().target = t;
-        out.back().control = c;
-        return out.back();
-    };
+    out.reserve(n);
     for (size_t i = 0; i < n; ++i) {
         const size_t k = sign > 0 ? i : n - 1 - i;
         const StrDev &sd = p->h_strs[k];
-        const double phi = (double)sign * sd.scale * params[sd.param], c = std::cos(phi), s = std::sin(phi);
-        const uint64_t q = x[k] | sd.z;
-        const int t = q ? __builtin_ctzll(q) : 0;
-        const int hi = q & (q - 1) ? 63 - __builtin_clzll(q) : t;
-        if (x[k] == 0 && hi != t) {  // Z Z: e^{i phi Z_t}, then e^{-2 i phi Z_t} where the other is 1
-            qfb_gate &a = gate(t, t);
-            a.mat[0][0] = qfb_complex{c, s};
-            a.mat[1][1] = qfb_complex{c, -s};
-            qfb_gate &b = gate(t, hi);
-            b.mat[0][0] = b.mat[1][1] = qfb_complex{1.0, 0.0};
-            b.mat[2][2] = qfb_complex{std::cos(2.0 * phi), -std::sin(2.0 * phi)};
-            b.mat[3][3] = qfb_complex{std::cos(2.0 * phi), std::sin(2.0 * phi)};
-            continue;
-        }
-        // basis index bit 0: qubit t, bit 1: qubit hi
-        const int dim = hi == t ? 2 : 4;
-        const int xl = (int)(x[k] >> t & 1) | (hi == t ? 0 : (int)(x[k] >> hi & 1) << 1);
-        const int zl = (int)(sd.z >> t & 1) | (hi == t ? 0 : (int)(sd.z >> hi & 1) << 1);
-        qfb_gate &g = gate(t, hi);
-        for (int j = 0; j < dim; ++j) {
-            g.mat[j][j].re += c;
-            // i sin phi i^ny (-1)^popcount(j & z) at row j ^ x
-            const int ph = (sd.ny + 1 + 2 * (__builtin_popcount(j & zl) & 1)) & 3;
-            qfb_complex &m = g.mat[j ^ xl][j];
-            if (ph & 1) m.im += ph == 1 ? s : -s;
-            else m.re += ph == 0 ? s : -s;
-        }
+        out.push_back(PauliRot{x[k], sd.z, (int)sd.ny, (double)sign * sd.scale * params[sd.param]});
     }
     return true;
 }
@@ -2112,8 +2079,8 @@ int qfb_prog_apply(qfb_prog p, qfb_state s, const double *params, int32_t nrows,
     if (rc) return rc;
     if (p->h_steps.empty()) return QFB_OK;
     if (nrows == 1 && s->nqubit >= kProgGateQubits && gate_tiles_on()) {
-        std::vector<qfb_gate> gates;
-        if (prog_gates(p, params, sign, gates)) return apply_gate_list(s, gates);
+        std::vector<PauliRot> rots;
+        if (prog_rotations(p, params, sign, rots)) return apply_rotations(s, rots);
     }
     if (sign > 0) {
         rc = ensure_plans(p, s->nqubit, true);
