@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "qfb_common.cuh"
+#include "qfb_ddrows.h"
 #include "qfb_dense.cuh"
 #include "qfb_gatetile.cuh"
 
@@ -515,9 +516,10 @@ int g_gate_reg_bits = 0;  // 0: default
 // Form of the tile phases: 0 gate by gate; 1 fused (8 x 8 matrices on the
 // FP64 tensor cores) where it applies; 2 (default) fused for states of at
 // least kFusedMinBytes.  Below it the time goes to planning, and the matrices
-// cost more of it (20 random layers, us, gate by gate / fused: 18 qubits 460 /
-// 500, 19 qubits 517 / 518, 20 qubits 973 / 577, 21 qubits 1,499 / 809, 24 qubits
-// 11,471 / 5,600).
+// cost more of it (20 random layers, us, gate by gate / fused: 18 qubits 493 /
+// 688, 19 qubits 600 / 727, 20 qubits 1,076 / 826, 21 qubits 1,696 / 967, 24 qubits
+// 13,338 / 5,568; 8 layers of Rx and cX-Rz-cX chains: 18 qubits 390 / 356, 20 qubits
+// 880 / 497, 24 qubits 10,844 / 3,652).
 int g_gate_fused = 2;
 constexpr uint64_t kFusedMinBytes = 1ull << 24, kFusedMinBytesC64 = 1ull << 27;
 
@@ -758,7 +760,6 @@ bool is_swap4(const WGate &g) {
 
 // ---- the fused form of a phase ----------------------------------------------
 
-
 // Complex numbers of the fused products on the host.
 template <class T>
 struct CplxH {
@@ -771,70 +772,104 @@ struct CplxH {
     double2 round() const { return make_double2((double)x, (double)y); }
 };
 
-// One op of a phase on the rows of an 8 x 8 matrix (row k: what register k
-// receives), for the thread with tile bits tl, as qfbt::apply_op applies it.
+// A product of gates, an 8 x 8 matrix by rows (row k: what register k receives), in
+// doubles (complex64 states) or in long double (CPUs without AVX2).
 template <class T>
-void top_apply_rows(const qfbt::TOp &o, const double2 *m4, uint32_t tl, CplxH<T> (*v)[8]) {
-    if ((tl & o.tctl) != o.tctl) return;
-    const uint32_t cm = o.aux & 0xffu, cv = (o.aux >> 16) & 0xffu, opc = o.opc;
-    using C = CplxH<T>;
-    auto scale = [](double2 f, C *r) {
-        for (int c = 0; c < 8; ++c) r[c] = C(f) * r[c];
-    };
-    if (opc < qfbt::OPC_DIAG) {
-        const uint32_t kind = opc / 4, tb = 1u << (opc % 4);
-        const C m[4] = {C(o.m[0]), C(o.m[1]), C(o.m[2]), C(o.m[3])};
-        for (uint32_t k = 0; k < 8; ++k) {
-            if ((k & tb) || (k & cm) != cv) continue;
-            C *r0 = v[k], *r1 = v[k | tb];
-            for (int c = 0; c < 8; ++c) {
-                const C x0 = r0[c], x1 = r1[c];
-                if (kind == qfbt::OP_PSWAP) {
-                    r0[c] = x1;
-                    r1[c] = x0;
-                } else if (kind == qfbt::OP_ANTI) {
-                    r0[c] = m[1] * x1;
-                    r1[c] = m[2] * x0;
-                } else {
-                    r0[c] = m[0] * x0 + m[1] * x1;
-                    r1[c] = m[2] * x0 + m[3] * x1;
-                }
+struct RowsH {
+    using F = T;
+    CplxH<T> v[8][8];
+    void reset() {
+        for (int r = 0; r < 8; ++r)
+            for (int c = 0; c < 8; ++c) v[r][c] = CplxH<T>(r == c ? 1 : 0, 0);
+    }
+    template <int N>
+    void mix(const int (&k)[N], const double2 *m) {
+        for (int c = 0; c < 8; ++c) {
+            CplxH<T> x[N];
+            for (int j = 0; j < N; ++j) x[j] = v[k[j]][c];
+            for (int i = 0; i < N; ++i) {
+                CplxH<T> acc = CplxH<T>(m[N * i]) * x[0];
+                for (int j = 1; j < N; ++j) acc = acc + CplxH<T>(m[N * i + j]) * x[j];
+                v[k[i]][c] = acc;
             }
         }
+    }
+    void swap(int a, int b) { std::swap_ranges(v[a], v[a] + 8, v[b]); }
+    double2 get(int r, int c) const { return v[r][c].round(); }
+};
+// The same in double-double (qfb_ddrows.h).
+struct RowsDD {
+    using F = long double;
+    qfbh::Rows8 r;
+    int touched;  // the register bits mixed so far: bit 2 joins the column halves
+    void reset() {
+        std::memset(&r, 0, sizeof(r));
+        for (int k = 0; k < 8; ++k) r.xh[k][k] = 1.0;
+        touched = 0;
+    }
+    template <int N>
+    void mix(const int (&k)[N], const double2 *m) {
+        for (int j = 1; j < N; ++j) touched |= k[j] ^ k[0];
+        qfbh::dd_mix(r, k, N, &m->x, touched & 4 ? 3u : 1u << (k[0] >> 2));
+    }
+    void swap(int a, int b) {
+        touched |= a ^ b;
+        for (auto *p : {r.xh, r.xl, r.yh, r.yl}) std::swap_ranges(p[a], p[a] + 8, p[b]);
+    }
+    double2 get(int k, int c) const { return make_double2(r.xh[k][c], r.yh[k][c]); }
+};
+
+// One op of a phase on a product's rows, for the thread with tile bits tl, as
+// qfbt::apply_op applies it.
+template <class M>
+void top_apply_rows(const qfbt::TOp &o, const double2 *m4, uint32_t tl, M &mat) {
+    if ((tl & o.tctl) != o.tctl) return;
+    const int cm = (int)(o.aux & 0xffu), cv = (int)((o.aux >> 16) & 0xffu);
+    const uint32_t opc = o.opc;
+    auto scale = [&](const double2 &f, int k) {
+        const int at[1] = {k};
+        mat.mix(at, &f);
+    };
+    if (opc < qfbt::OPC_DIAG) {
+        const uint32_t kind = opc / 4;
+        const int tb = 1 << (opc % 4);
+        double2 m[4] = {o.m[0], o.m[1], o.m[2], o.m[3]};
+        if (kind == qfbt::OP_ANTI) m[0] = m[3] = make_double2(0.0, 0.0);
+        for (int k = 0; k < 8; ++k) {
+            if ((k & tb) || (k & cm) != cv) continue;
+            const int at[2] = {k, k | tb};
+            if (kind == qfbt::OP_PSWAP)
+                mat.swap(at[0], at[1]);
+            else
+                mat.mix(at, m);
+        }
     } else if (opc < qfbt::OPC_DIAG_THREAD) {
-        const uint32_t dset = (opc - qfbt::OPC_DIAG) / 4 + 1, tb = 1u << ((opc - qfbt::OPC_DIAG) % 4);
-        for (uint32_t k = 0; k < 8; ++k) {
+        const uint32_t dset = (opc - qfbt::OPC_DIAG) / 4 + 1;
+        const int tb = 1 << ((opc - qfbt::OPC_DIAG) % 4);
+        for (int k = 0; k < 8; ++k) {
             if ((k & cm) != cv) continue;
             if (k & tb) {
-                if (dset & 2u) scale(o.m[3], v[k]);
+                if (dset & 2u) scale(o.m[3], k);
             } else if (dset & 1u) {
-                scale(o.m[0], v[k]);
+                scale(o.m[0], k);
             }
         }
     } else if (opc == qfbt::OPC_DIAG_THREAD) {
         const bool one = (tl & o.tbit) != 0;
         if (!(((o.aux >> 8) & 3u) & (one ? 2u : 1u))) return;
-        for (uint32_t k = 0; k < 8; ++k)
-            if ((k & cm) == cv) scale(o.m[one ? 3 : 0], v[k]);
+        for (int k = 0; k < 8; ++k)
+            if ((k & cm) == cv) scale(o.m[one ? 3 : 0], k);
     } else if (opc < qfbt::OPC_BSWAP) {
-        const uint32_t tb = 1u << ((opc - qfbt::OPC_GEN4) / 4), cb = 1u << ((opc - qfbt::OPC_GEN4) % 4);
-        const double2 *m = m4 + o.aux;
-        for (uint32_t k = 0; k < 8; ++k) {
+        const int tb = 1 << ((opc - qfbt::OPC_GEN4) / 4), cb = 1 << ((opc - qfbt::OPC_GEN4) % 4);
+        for (int k = 0; k < 8; ++k) {
             if (k & (tb | cb)) continue;
-            C *r[4] = {v[k], v[k | tb], v[k | cb], v[k | tb | cb]};
-            for (int c = 0; c < 8; ++c) {
-                const C x[4] = {r[0][c], r[1][c], r[2][c], r[3][c]};
-                for (int i = 0; i < 4; ++i) {
-                    C acc;
-                    for (int j = 0; j < 4; ++j) acc = acc + C(m[4 * i + j]) * x[j];
-                    r[i][c] = acc;
-                }
-            }
+            const int at[4] = {k, k | tb, k | cb, k | tb | cb};
+            mat.mix(at, m4 + o.aux);
         }
     } else {
-        const uint32_t tb = 1u << ((opc - qfbt::OPC_BSWAP) / 4), cb = 1u << ((opc - qfbt::OPC_BSWAP) % 4);
-        for (uint32_t k = 0; k < 8; ++k)
-            if ((k & tb) && !(k & cb)) std::swap_ranges(v[k], v[k] + 8, v[k ^ tb ^ cb]);
+        const int tb = 1 << ((opc - qfbt::OPC_BSWAP) / 4), cb = 1 << ((opc - qfbt::OPC_BSWAP) % 4);
+        for (int k = 0; k < 8; ++k)
+            if ((k & tb) && !(k & cb)) mat.swap(k, k ^ tb ^ cb);
     }
 }
 
@@ -848,11 +883,10 @@ void top_apply_rows(const qfbt::TOp &o, const double2 *m4, uint32_t tl, CplxH<T>
 // entries); otherwise the phase is split into phases on the same registers,
 // each with its own thread table: all but the last store to the load
 // offsets, the next loads them again.
-template <class F>
+template <class M>
 void fuse_phase(TilePlan &tp, const qfbt::TPhase &ph, int b, bool c64) {
     constexpr int R = 3;
     auto toff = [c64](uint32_t l) { return c64 ? qfbt::tpad8(l) : qfbt::tpad(l); };
-    constexpr uint32_t NR = 8;
     const uint32_t nth = 1u << (b - R);
     const int nvb = b - R - 3;  // vector-index bits above the n-block columns
     // a segment's variant bits must all fit there (8-qubit tiles have 2)
@@ -869,7 +903,8 @@ void fuse_phase(TilePlan &tp, const qfbt::TPhase &ph, int b, bool c64) {
     const uint32_t T = ((1u << b) - 1u) & ~S;  // thread bits
     std::vector<int> run_ops;
     std::vector<qfbt::TOp> fac_ops;
-    CplxH<F> mat[NR][NR];
+    using F = typename M::F;
+    M mat;
     struct Seg {
         uint32_t D;  // variant bits
         qfbt::TSeg h;
@@ -891,16 +926,14 @@ void fuse_phase(TilePlan &tp, const qfbt::TPhase &ph, int b, bool c64) {
             uint32_t tl = 0;
             for (size_t j = 0; j < dbits.size(); ++j)
                 if (x >> j & 1u) tl |= 1u << dbits[j];
-            for (uint32_t r = 0; r < NR; ++r)
-                for (uint32_t c = 0; c < NR; ++c) mat[r][c] = CplxH<F>(r == c ? 1 : 0, 0);
+            mat.reset();
             for (int oi : run_ops) top_apply_rows(tp.ops[oi], tp.m4.data(), tl, mat);
-            for (uint32_t r = 0; r < NR; ++r)
-                for (uint32_t c = 0; c < NR; ++c)
-                    if (mat[r][c].x != 0 || mat[r][c].y != 0) sg.h.mm |= r ^ c;
-            for (uint32_t kb = 0; kb < 2; ++kb)
-                for (uint32_t lane = 0; lane < 32; ++lane)
-                    mats.push_back(mat[lane >> 2][4 * kb + (lane & 3)].round());
-
+            for (int kb = 0; kb < 2; ++kb)
+                for (int lane = 0; lane < 32; ++lane) {
+                    const int r = lane >> 2, c = 4 * kb + (lane & 3);
+                    mats.push_back(mat.get(r, c));
+                    if (mats.back().x != 0.0 || mats.back().y != 0.0) sg.h.mm |= (uint32_t)(r ^ c);
+                }
         }
         segs.push_back(sg);
         run_ops.clear();
@@ -985,15 +1018,20 @@ void fuse_phase(TilePlan &tp, const qfbt::TPhase &ph, int b, bool c64) {
         q.sc = -1;
         if (first && !fac_ops.empty()) {
             q.sc = (int)tp.fm.size();
-            for (uint32_t t = 0; t < nth; ++t) {
+            // once per assignment of the bits the factors test
+            uint32_t used = 0;
+            for (const qfbt::TOp &o : fac_ops) used |= o.tbit | o.tctl;
+            std::vector<double2> f_of((size_t)used + 1);
+            for (uint32_t tl = used;; tl = (tl - 1) & used) {
                 CplxH<F> f(1, 0);
-                const uint32_t tl = tp.threads[q.th0 + t] & 0xffffu;
                 for (const qfbt::TOp &o : fac_ops) {
                     const uint32_t one = (tl & o.tbit) != 0;
                     if ((tl & o.tctl) == o.tctl && (o.aux >> (8 + one) & 1u)) f = CplxH<F>(o.m[one ? 3 : 0]) * f;
                 }
-                tp.fm.push_back(f.round());
+                f_of[tl] = f.round();
+                if (tl == 0) break;
             }
+            for (uint32_t t = 0; t < nth; ++t) tp.fm.push_back(f_of[tp.threads[q.th0 + t] & used]);
         }
         if (j < segs.size())  // more segments follow on the same registers
             std::memcpy(q.soff, q.roff, sizeof(q.roff));
@@ -1010,11 +1048,10 @@ void fuse_phase(TilePlan &tp, const qfbt::TPhase &ph, int b, bool c64) {
 // gate that cannot join blocks its bits for the rest of the scan, so only
 // gates on disjoint qubits change order.
 // c64: shared offsets in the complex64 tile layout (qfbt::tpad8).
-// fine: the fused matrices are multiplied out in extended precision and rounded
-// once.  fused: the phases' fused form where it applies (R = 3, at least 32
-// threads).
+// fused: the phases' fused form where it applies (R = 3, at least 32 threads);
+// dd: its products in double-double, else in long double.
 void plan_tile_phases(const WGate *g, int ng, int b, int R, qfbt::TRun &run, TilePlan &tp,
-                      bool c64 = false, bool fused = false, bool fine = false) {
+                      bool c64 = false, bool fused = false, bool dd = qfbh::dd_available()) {
     auto toff = [c64](uint32_t l) { return c64 ? qfbt::tpad8(l) : qfbt::tpad(l); };
     std::vector<uint32_t> mix((size_t)ng), qm((size_t)ng);
     for (int i = 0; i < ng; ++i) {
@@ -1186,7 +1223,8 @@ void plan_tile_phases(const WGate *g, int ng, int b, int R, qfbt::TRun &run, Til
         }
         ph.no = (int)tp.ops.size() - ph.o0;
         if (fuse)
-            fine ? fuse_phase<long double>(tp, ph, b, c64) : fuse_phase<double>(tp, ph, b, c64);
+            c64 ? fuse_phase<RowsH<double>>(tp, ph, b, c64)
+                : dd ? fuse_phase<RowsDD>(tp, ph, b, c64) : fuse_phase<RowsH<long double>>(tp, ph, b, c64);
         else
             tp.ph.push_back(ph);
     }
@@ -1354,7 +1392,8 @@ int apply_gates_dense(qfb_state s, const std::vector<HGate> &hg, int K) {
 
 // The phases of each window's run.
 void plan_tile_runs(const std::vector<GatePlanWin> &wins, const std::vector<WGate> &wg, TilePlan &tp,
-                    std::vector<qfbt::TRun> &runs, bool c64, bool fused, bool fine = false) {
+                    std::vector<qfbt::TRun> &runs, bool c64, bool fused,
+                    bool dd = qfbh::dd_available()) {
     runs.assign(wins.size(), qfbt::TRun{});
     for (size_t i = 0; i < wins.size(); ++i) {
         const GatePlanWin &pw = wins[i];
@@ -1368,17 +1407,17 @@ void plan_tile_runs(const std::vector<GatePlanWin> &wins, const std::vector<WGat
             for (size_t c = 0; c < half; ++c)
                 tp.chunks.push_back(tp.chunks[(size_t)r.ch0 + c] | (m & (~m + 1)));
         plan_tile_phases(wg.data() + pw.w.g0, pw.w.ng, pw.w.b, tile_reg_bits(pw.w.b), r, tp, c64,
-                         fused, fine);
+                         fused, dd);
     }
 }
 
 // Runs of a gate list and the phases of each run.
 void plan_gate_tiles(const std::vector<HGate> &hg, int n, int b, int L,
                      std::vector<GatePlanWin> &wins, TilePlan &tp, std::vector<qfbt::TRun> &runs,
-                     bool c64 = false, bool fused = false) {
+                     bool c64 = false, bool fused = false, bool dd = qfbh::dd_available()) {
     std::vector<WGate> wg;
     plan_gate_windows(hg, n, b, L, wins, wg);
-    plan_tile_runs(wins, wg, tp, runs, c64, fused);
+    plan_tile_runs(wins, wg, tp, runs, c64, fused, dd);
 }
 
 // Bounds-check and classify a gate list for an nqubit state.
@@ -1470,7 +1509,7 @@ int launch_tile_runs(A *d, uint64_t nbasis, int nbatch, const std::vector<HGate>
 // float2 for the complex64 variant): register-blocked tile runs, one pass per
 // gate where a gate joins no run (or the tile shape says so).
 template <class A>
-int apply_gates_tiles(A *d, int n, int nbatch, const std::vector<HGate> &hg, bool fine = false) {
+int apply_gates_tiles(A *d, int n, int nbatch, const std::vector<HGate> &hg) {
     const uint64_t nbasis = 1ull << n;
     int b = 0, L = 0;
     constexpr bool c64 = sizeof(A) == sizeof(float2);
@@ -1496,7 +1535,7 @@ int apply_gates_tiles(A *d, int n, int nbatch, const std::vector<HGate> &hg, boo
         if (wins.empty()) break;
         TilePlan tp;
         std::vector<qfbt::TRun> runs;
-        plan_tile_runs(wins, wg, tp, runs, c64, fused, fine);
+        plan_tile_runs(wins, wg, tp, runs, c64, fused);
         rc = launch_tile_runs<A>(d, nbasis, nbatch, hg, wins, runs, tp, fused);
     }
     return rc;
@@ -1584,7 +1623,7 @@ int apply_rotations(qfb_state s, const std::vector<PauliRot> &rots) {
     std::vector<HGate> hg;
     hg.reserve(rots.size() + rots.size() / 2);
     for (const PauliRot &p : rots) rot_gates(p, hg);
-    return hg.empty() ? QFB_OK : apply_gates_tiles<double2>(s->d, s->nqubit, s->nbatch, hg, true);
+    return hg.empty() ? QFB_OK : apply_gates_tiles<double2>(s->d, s->nqubit, s->nbatch, hg);
 }
 
 // ===========================================================================
@@ -1933,6 +1972,18 @@ int qfb_gates_fused_plan(const qfb_gate *gates, int64_t ngates, int nqubit, int 
         TilePlan tp;
         std::vector<qfbt::TRun> runs;
         plan_gate_tiles(hg, nqubit, b, L, wins, tp, runs, c64, true);
+        if (!c64) {  // the products in double-double are those in long double, rounded once
+            std::vector<GatePlanWin> wins2;
+            TilePlan tp2;
+            std::vector<qfbt::TRun> runs2;
+            plan_gate_tiles(hg, nqubit, b, L, wins2, tp2, runs2, c64, true, false);
+            if (tp2.fm.size() != tp.fm.size())
+                return fail(QFB_EINVAL, "qfb_gates_fused_plan: forms of different sizes");
+            auto off = [](double x, double y) { return !(std::fabs(x - y) <= 2.3e-16 * std::fabs(y) + 1e-17); };
+            for (size_t k = 0; k < tp.fm.size(); ++k)
+                if (off(tp.fm[k].x, tp2.fm[k].x) || off(tp.fm[k].y, tp2.fm[k].y))
+                    return fail(QFB_EINVAL, "qfb_gates_fused_plan: matrix entry %zu differs", k);
+        }
         for (size_t w = 0; w < wins.size(); ++w) {
             if (wins[w].single >= 0) continue;
             const qfbt::TRun &r = runs[w];
