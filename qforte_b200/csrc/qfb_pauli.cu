@@ -185,90 +185,57 @@ __global__ void k_seg_sum(const double2 *__restrict__ partial, const int32_t *__
     if (threadIdx.x == 0) out[(uint64_t)b * gridDim.x + s] = acc;
 }
 
-// dst[k] = sum_g f_g(k ^ x_g) src[k ^ x_g]; one output per thread, written once.
-__global__ void __launch_bounds__(256) k_sum_apply(
-    double2 *__restrict__ dst, const double2 *__restrict__ src, uint64_t nbasis,
-    const GroupDev *__restrict__ groups, const TermDev *__restrict__ terms, int32_t ngroups) {
-    const uint64_t off = (uint64_t)blockIdx.y * nbasis;
-    for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nbasis;
-         k += (uint64_t)gridDim.x * blockDim.x) {
-        double2 acc = make_double2(0.0, 0.0);
-        for (int g = 0; g < ngroups; ++g) {
-            const GroupDev gr = groups[g];
-            const uint64_t j = k ^ gr.x;
-            const double2 a = src[off + j];
-            if (gr.real) {
-                double f = 0.0;
-                for (int t = gr.begin; t < gr.end; ++t) {
-                    const double c = __ldg(&terms[t].c.x);
-                    f += parity64(j & __ldg(&terms[t].z)) ? -c : c;
-                }
-                acc.x += f * a.x;
-                acc.y += f * a.y;
-            } else {
-                double2 f = make_double2(0.0, 0.0);
-                for (int t = gr.begin; t < gr.end; ++t) {
-                    const double2 c = terms[t].c;
-                    if (parity64(j & terms[t].z)) { f.x -= c.x; f.y -= c.y; }
-                    else { f.x += c.x; f.y += c.y; }
-                }
-                acc = c_add(acc, c_mul(f, a));
-            }
-        }
-        dst[off + k] = acc;
-    }
-}
-
-// dst = O src with four outputs per thread: k = k0 | d, d = 0..3.  For a
-// group x the four inputs j_d = (k0 ^ x) ^ d form one aligned quad, and
-// popcount(j_d & z) = popcount((k0 ^ x) & z) + popcount(d & z): one parity per
-// term serves all four outputs.  Terms are read in the real form (z, Re c)
-// when the group is real.
+// dst = O src with four outputs per thread, for NS states at a time: k = k0 | d,
+// d = 0..3.  For a group x the four inputs j_d = (k0 ^ x) ^ d form one aligned quad,
+// and popcount(j_d & z) = popcount((k0 ^ x) & z) + popcount(d & z): one parity per
+// term serves all four outputs of the NS states.  Terms are read in the real form
+// (z, Re c) when the group is real.  Work items are (quad, NS states), so a batch
+// of small states fills blocks as one large state does.
+template <int NS, typename IDX>
 __global__ void __launch_bounds__(256) k_sum_apply4(
-    double2 *__restrict__ dst, const double2 *__restrict__ src, uint64_t nbasis,
+    double2 *__restrict__ dst, const double2 *__restrict__ src, uint64_t nbasis, int nbatch,
     const GroupDev *__restrict__ groups, const TermDev *__restrict__ terms,
     const double2 *__restrict__ rterms, int32_t ngroups) {
-    const uint64_t off = (uint64_t)blockIdx.y * nbasis;
-    const uint64_t nquad = nbasis >> 2;
-    for (uint64_t qd = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; qd < nquad;
-         qd += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t k0 = qd << 2;
-        double2 acc0 = make_double2(0.0, 0.0), acc1 = acc0, acc2 = acc0, acc3 = acc0;
+    const uint64_t nquad = nbasis >> 2, items = nquad * (uint64_t)((nbatch + NS - 1) / NS);
+    for (uint64_t it = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; it < items;
+         it += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t sg = NS == 1 ? 0 : it / nquad, k0 = (it - sg * nquad) << 2;
+        const uint64_t off = sg * NS * nbasis;
+        const int ns = NS == 1 ? 1 : (int)min((uint64_t)NS, (uint64_t)nbatch - sg * NS);
+        double2 acc[NS][4];
+#pragma unroll
+        for (int s = 0; s < NS; ++s)
+#pragma unroll
+            for (int d = 0; d < 4; ++d) acc[s][d] = make_double2(0.0, 0.0);
         for (int g = 0; g < ngroups; ++g) {
             const uint64_t x = __ldg(&groups[g].x);
             const int tb = __ldg(&groups[g].begin), te = __ldg(&groups[g].end);
             const int real = __ldg(&groups[g].real);
-            const uint64_t base = k0 ^ x;
-            const uint64_t qb = base & ~3ull;
-            // a[e] = src[qb | e]; input of output d is a[d ^ (x & 3)]
-            double2 a0 = src[off + qb], a1 = src[off + qb + 1];
-            double2 a2 = src[off + qb + 2], a3 = src[off + qb + 3];
-            if (x & 1) {
-                double2 t = a0; a0 = a1; a1 = t;
-                t = a2; a2 = a3; a3 = t;
-            }
-            if (x & 2) {
-                double2 t = a0; a0 = a2; a2 = t;
-                t = a1; a1 = a3; a3 = t;
-            }
+            const uint64_t base = k0 ^ x, qb = base & ~3ull;
+            const IDX bz = (IDX)base;
+            // f[d]: the coefficient of output d
+            double2 f[4];
             if (real) {
-                double f0 = 0.0, f1 = 0.0, f2 = 0.0, f3 = 0.0;
+                double r0 = 0.0, r1 = 0.0, r2 = 0.0, r3 = 0.0;
+#pragma unroll 4
                 for (int t = tb; t < te; ++t) {
                     const double2 zc = __ldg(&rterms[t]);  // (z bits, Re c)
-                    const uint64_t z = (uint64_t)__double_as_longlong(zc.x);
-                    const double c = parity64(base & z) ? -zc.y : zc.y;
-                    const double c1 = (z & 1) ? -c : c;
-                    f0 += c;
-                    f1 += c1;
-                    f2 += (z & 2) ? -c : c;
-                    f3 += (z & 2) ? -c1 : c1;
+                    const IDX z = (IDX)__double_as_longlong(zc.x);
+                    const uint32_t zl = (uint32_t)z, s2 = (zl & 2u) << 30;
+                    const uint32_t odd = sizeof(IDX) == 4 ? (uint32_t)__popc((uint32_t)(bz & z))
+                                                          : (uint32_t)__popcll((uint64_t)(bz & z));
+                    const double c = qfbs::v_flip(zc.y, odd << 31), c1 = qfbs::v_flip(c, zl << 31);
+                    r0 += c;
+                    r1 += c1;
+                    r2 += qfbs::v_flip(c, s2);
+                    r3 += qfbs::v_flip(c1, s2);
                 }
-                acc0.x += f0 * a0.x; acc0.y += f0 * a0.y;
-                acc1.x += f1 * a1.x; acc1.y += f1 * a1.y;
-                acc2.x += f2 * a2.x; acc2.y += f2 * a2.y;
-                acc3.x += f3 * a3.x; acc3.y += f3 * a3.y;
+                f[0] = make_double2(r0, 0.0);
+                f[1] = make_double2(r1, 0.0);
+                f[2] = make_double2(r2, 0.0);
+                f[3] = make_double2(r3, 0.0);
             } else {
-                double2 f0 = make_double2(0.0, 0.0), f1 = f0, f2 = f0, f3 = f0;
+                f[0] = f[1] = f[2] = f[3] = make_double2(0.0, 0.0);
                 for (int t = tb; t < te; ++t) {
                     const uint64_t z = __ldg(&terms[t].z);
                     double2 c = terms[t].c;
@@ -276,24 +243,53 @@ __global__ void __launch_bounds__(256) k_sum_apply4(
                     const double2 c1 = (z & 1) ? make_double2(-c.x, -c.y) : c;
                     const double2 c2 = (z & 2) ? make_double2(-c.x, -c.y) : c;
                     const double2 c3 = (z & 2) ? make_double2(-c1.x, -c1.y) : c1;
-                    f0 = c_add(f0, c); f1 = c_add(f1, c1); f2 = c_add(f2, c2); f3 = c_add(f3, c3);
+                    f[0] = c_add(f[0], c);
+                    f[1] = c_add(f[1], c1);
+                    f[2] = c_add(f[2], c2);
+                    f[3] = c_add(f[3], c3);
                 }
-                acc0 = c_add(acc0, c_mul(f0, a0));
-                acc1 = c_add(acc1, c_mul(f1, a1));
-                acc2 = c_add(acc2, c_mul(f2, a2));
-                acc3 = c_add(acc3, c_mul(f3, a3));
+            }
+#pragma unroll
+            for (int s = 0; s < NS; ++s) {
+                if (s >= ns) break;
+                // the input of output d is src[qb | (d ^ (x & 3))]
+                const double2 *p = src + off + (uint64_t)s * nbasis + qb;
+                double2 a0 = p[0], a1 = p[1], a2 = p[2], a3 = p[3];
+                if (x & 1) {
+                    double2 t = a0; a0 = a1; a1 = t;
+                    t = a2; a2 = a3; a3 = t;
+                }
+                if (x & 2) {
+                    double2 t = a0; a0 = a2; a2 = t;
+                    t = a1; a1 = a3; a3 = t;
+                }
+                if (real) {
+                    acc[s][0].x += f[0].x * a0.x; acc[s][0].y += f[0].x * a0.y;
+                    acc[s][1].x += f[1].x * a1.x; acc[s][1].y += f[1].x * a1.y;
+                    acc[s][2].x += f[2].x * a2.x; acc[s][2].y += f[2].x * a2.y;
+                    acc[s][3].x += f[3].x * a3.x; acc[s][3].y += f[3].x * a3.y;
+                } else {
+                    acc[s][0] = c_add(acc[s][0], c_mul(f[0], a0));
+                    acc[s][1] = c_add(acc[s][1], c_mul(f[1], a1));
+                    acc[s][2] = c_add(acc[s][2], c_mul(f[2], a2));
+                    acc[s][3] = c_add(acc[s][3], c_mul(f[3], a3));
+                }
             }
         }
-        dst[off + k0] = acc0;
-        dst[off + k0 + 1] = acc1;
-        dst[off + k0 + 2] = acc2;
-        dst[off + k0 + 3] = acc3;
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            if (s >= ns) break;
+            double2 *p = dst + off + (uint64_t)s * nbasis + k0;
+#pragma unroll
+            for (int d = 0; d < 4; ++d) p[d] = acc[s][d];
+        }
     }
 }
 
-// dst = O src (DOT: <bra|O|src> instead), states of 8 qubits and more: 2^8
-// outputs a block, the groups dealt to its 8 warps.  A group's coefficient on output k, d its bits
-// 2-4, is the sum over its terms of
+// dst = O src (DOT: <bra|O|src> instead): 2^8 outputs a block, the blocks of four
+// terms dealt to its 8 warps.  total: amplitudes of a state, or of a whole batch of
+// states below 2^8 amplitudes (the masks leave the index bits above a state alone).
+// A group's coefficient on output k, d its bits 2-4, is the sum over its terms of
 //     (-1)^popcount(d & z's bits 2-4)  c (-1)^popcount(((k with d = 0) ^ x) & z):
 // an 8 x terms matrix of signs times a terms x 32 matrix of signed coefficients,
 // done on the FP64 matrix units four terms at a time.  So a warp takes one parity
@@ -308,6 +304,10 @@ __global__ void __launch_bounds__(256) k_sum_apply4(
 // (981 groups, 5,793 terms) 1 state 762 / 88, 64 states 6,033 / 4,496; 12 qubits
 // 206 / 20 and 314 / 98; <psi|H|psi> group by group (k_sum_expval) / this kernel:
 // 16 qubits 1 state 492 / 84; 12 qubits 20.4 / 18.0; 8 qubits 3.7 / 5.4.
+//
+// Few groups leave a block little to do between its barriers, and one of many terms
+// forms them again for every state; there k_sum_apply4 and k_sum_expval take over
+// (sum_form, expval_by_tiles).
 constexpr int kSumTileBits = 8;
 constexpr int kSumWarps = 8;
 constexpr int kSumAhead = 8;  // blocks a warp stages (four terms each: one a lane)
@@ -316,19 +316,20 @@ struct SumBlock {  // of four terms
     uint32_t fl;  // bit 0: first of its group, 1: last, 2: the coefficients are imaginary parts
     uint32_t pad;
 };
-template <bool DOT, typename IDX>
+// PART: the last tile holds fewer than 256 outputs.
+template <bool DOT, bool PART, typename IDX>
 __global__ void __launch_bounds__(32 * kSumWarps, 2) k_sum_tile(
     double2 *__restrict__ dst, const double2 *__restrict__ bra, const double2 *__restrict__ src,
-    uint64_t nbasis, const SumBlock *__restrict__ blocks, const double2 *__restrict__ terms,
+    uint64_t total, const SumBlock *__restrict__ blocks, const double2 *__restrict__ terms,
     const int32_t *__restrict__ slice, double2 *__restrict__ partial) {
     __shared__ double2 s_acc[kSumWarps][256];
     __shared__ double2 s_term[kSumWarps][4 * kSumAhead];
     __shared__ uint4 s_block[kSumWarps][kSumAhead];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = lane >> 2, col = lane & 3;
-    const uint64_t off = (uint64_t)blockIdx.y * nbasis;
+    const uint64_t off = (uint64_t)blockIdx.y * total;
     const int b0 = slice[warp], b1 = slice[warp + 1];
     double2 dot = make_double2(0.0, 0.0);
-    for (uint64_t tile = blockIdx.x; tile < nbasis >> 8; tile += gridDim.x) {
+    for (uint64_t tile = blockIdx.x; tile < (total + 255) >> 8; tile += gridDim.x) {
         const IDX kb = (IDX)(tile << 8);
         double2 acc[8], a[8];
         double f[8];
@@ -353,7 +354,8 @@ __global__ void __launch_bounds__(32 * kSumWarps, 2) k_sum_tile(
             if (bl.z & 1u) {
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
-                    a[q] = __ldg(&src[off + (uint64_t)((kb | (IDX)(q << 5 | lane)) ^ x)]);
+                    const uint64_t at = (uint64_t)((kb | (IDX)(q << 5 | lane)) ^ x);
+                    a[q] = __ldg(&src[off + (PART && at >= total ? 0 : at)]);
                 }
             }
             const IDX z = (IDX)__double_as_longlong(zc.x);
@@ -400,11 +402,11 @@ __global__ void __launch_bounds__(32 * kSumWarps, 2) k_sum_tile(
         double2 t = make_double2(0.0, 0.0);
 #pragma unroll
         for (int w = 0; w < kSumWarps; ++w) t = c_add(t, s_acc[w][threadIdx.x]);
-        const uint64_t k = off + (tile << 8) + threadIdx.x;
+        const uint64_t k = (tile << 8) + threadIdx.x;
         if (DOT)
-            dot = c_add(dot, c_cjmul(bra[k], t));
-        else
-            dst[k] = t;
+            dot = c_add(dot, c_cjmul(bra[off + k], t));
+        else if (!PART || k < total)
+            dst[off + k] = t;
     }
     if (DOT) {
         dot = block_sum(dot);
@@ -1507,35 +1509,68 @@ static void make_table(qfb_prog_s *p, StepDev &st) {
     }
 }
 
-// Blocks of k_sum_tile per state.
-static unsigned tile_grid(uint64_t nbasis) {
-    return (unsigned)std::min<uint64_t>(nbasis >> kSumTileBits, 16 * (uint64_t)sm_count());
+// The kernel of H psi: by estimates of each one's time for G groups of T terms in all
+// (us, 2^26 amplitudes, fitted to 1 to 24 groups of 1 to 300 terms).  Below 2^18
+// amplitudes every kernel waits for its own latency, which the tiles share best.
+// us, tiles / quads / quads of 4 states: 20 qubits, 64 states: one string 1,282 / 395 /
+// 411, 8 groups of 6 terms 1,725 / 1,746 / 1,635, 24 of 6 3,090 / 5,330 / 4,550, 200
+// diagonal terms 3,343 / 4,086 / 1,150; 20 qubits, one state: one string 21 / 10 / -,
+// 24 groups of 6 52 / 84 / -; 12 qubits, 8 states, 200 diagonal terms 6 / 28 / 23.
+enum SumForm { SUM_TILES, SUM_QUADS, SUM_QUADS4 };
+static SumForm sum_form(const qfb_sum_s *h, uint64_t nbasis, int B) {
+    if (nbasis < 4 || nbasis * (uint64_t)B < 1ull << 18) return SUM_TILES;
+    const double G = h->ngroups, T = (double)h->nterms, NB = (T + 3.0 * G) / 4.0;
+    const double tiles = 1150.0 + 40.0 * std::max(G, std::min(8.0, NB)) + 25.0 * NB;
+    const double quads = 400.0 + 110.0 * G + 20.0 * T;
+    const double quads4 = B < 4 || nbasis * (uint64_t)B < 1ull << 20 ? quads : 400.0 + 180.0 * G + 6.0 * T;
+    if (tiles <= std::min(quads, quads4)) return SUM_TILES;
+    return quads <= quads4 ? SUM_QUADS : SUM_QUADS4;
+}
+// The same for <bra|O|ket> of one segment: k_sum_tile, or k_sum_expval, which takes a
+// pass over both states per group (us, tiles / by groups: 20 qubits, 64 states: one
+// string 1,623 / 281, 8 strings 1,748 / 1,457, 8 groups of 6 1,908 / 2,633, 64 diagonal
+// terms 2,858 / 2,459, 200 3,752 / 7,389).  States below a tile go by groups.
+static bool expval_by_tiles(const qfb_sum_s *h, uint64_t nbasis, int B) {
+    if (h->nsegment != 1 || h->ngroups > 65535 || nbasis < 1ull << kSumTileBits) return false;
+    if (nbasis * (uint64_t)B < 1ull << 18) return nbasis * (uint64_t)B >= 4096;
+    const double G = h->ngroups, T = (double)h->nterms, NB = (T + 3.0 * G) / 4.0;
+    return 1500.0 + 30.0 * std::max(G, std::min(8.0, NB)) + 45.0 * NB < 100.0 + 130.0 * G + 35.0 * T;
 }
 
+// Blocks of k_sum_tile for so many amplitudes.
+static unsigned tile_grid(uint64_t total) {
+    return (unsigned)std::min<uint64_t>((total + 255) >> kSumTileBits, 16 * (uint64_t)sm_count());
+}
+
+// partial (DOT): tile_grid(nbasis) sums per state.
 template <bool DOT>
-static int launch_tiles(const qfb_sum_s *h, double2 *dst, const double2 *bra, const double2 *src,
-                        uint64_t nbasis, int B, double2 *partial) {
+static int launch_tiles(const qfb_sum_s *h, double2 *dst, const double2 *bra, const double2 *src, uint64_t nbasis,
+                        int B, double2 *partial) {
     const SumTiles &tv = *h->tiles;
-    for (int b = 0; b < B; b += 65535) {  // grid.y's limit
-        const dim3 grid(tile_grid(nbasis), (unsigned)std::min(65535, B - b));
-        const uint64_t at = (uint64_t)b * nbasis;
-        double2 *part = DOT ? partial + (size_t)b * grid.x : nullptr;
-        if (nbasis <= 1ull << 32)
-            k_sum_tile<DOT, uint32_t><<<grid, 32 * kSumWarps, 0, t_stream>>>(
-                DOT ? nullptr : dst + at, DOT ? bra + at : nullptr, src + at, nbasis, tv.blocks, tv.terms, tv.slice, part);
-        else
-            k_sum_tile<DOT, uint64_t><<<grid, 32 * kSumWarps, 0, t_stream>>>(
-                DOT ? nullptr : dst + at, DOT ? bra + at : nullptr, src + at, nbasis, tv.blocks, tv.terms, tv.slice, part);
+    auto launch = [&](dim3 grid, size_t at, uint64_t total, double2 *part) -> int {
+        const bool small = total <= 1ull << 32;
+        auto k = small ? k_sum_tile<DOT, false, uint32_t> : k_sum_tile<DOT, false, uint64_t>;
+        if (!DOT && total & 255) k = small ? k_sum_tile<DOT, !DOT, uint32_t> : k_sum_tile<DOT, !DOT, uint64_t>;
+        k<<<grid, 32 * kSumWarps, 0, t_stream>>>(DOT ? nullptr : dst + at, DOT ? bra + at : nullptr, src + at, total,
+                                                 tv.blocks, tv.terms, tv.slice, part);
         QFB_LAUNCHED();
-    }
-    return QFB_OK;
+        return QFB_OK;
+    };
+    if (nbasis >> kSumTileBits == 0) return launch(dim3(tile_grid(nbasis * B)), 0, nbasis * (uint64_t)B, partial);
+    // state by state (a state's tiles share L2), as many a launch as grid.y takes
+    int rc = QFB_OK;
+    const unsigned per = tile_grid(nbasis);
+    for (int b = 0; rc == QFB_OK && b < B; b += 65535)
+        rc = launch(dim3(per, (unsigned)std::min(65535, B - b)), (size_t)b * nbasis, nbasis,
+                    DOT ? partial + (size_t)b * per : nullptr);
+    return rc;
 }
 
 extern "C" {
 
 static int enqueue_sum_apply(const qfb_sum_s *h, double2 *dst, const double2 *src,
                              uint64_t nbasis, int B);
-static int ensure_tiles(qfb_sum_s *h, int nqubit);
+static int ensure_tiles(qfb_sum_s *h);
 
 int qfb_sum_create(const qfb_pauli *paulis, const qfb_complex *coeffs, const int32_t *segment,
                    int64_t nterms, int32_t nsegment, qfb_sum *out) {
@@ -1677,10 +1712,8 @@ int qfb_sum_expval(qfb_sum h, qfb_state bra, qfb_state ket, qfb_complex *out) {
         for (size_t i = 0; i < nout; ++i) out[i] = qfb_complex{0.0, 0.0};
         return QFB_OK;
     }
-    // one sum over all groups: by outputs, where there are enough of them
-    const bool tv = h->nsegment == 1 && h->ngroups <= 65535 && bra->nqubit >= kSumTileBits &&
-                    bra->nbasis * (uint64_t)B >= 4096;
-    int rc = tv ? ensure_tiles(h, bra->nqubit) : QFB_OK;
+    const bool tv = expval_by_tiles(h, bra->nbasis, B);
+    int rc = tv ? ensure_tiles(h) : QFB_OK;
     if (rc) return rc;
     const uint64_t npair = bra->nbasis >> 1;
     const unsigned chunks = tv ? tile_grid(bra->nbasis) : chunks_for(npair, B, h->ngroups);
@@ -1731,7 +1764,7 @@ int qfb_sum_apply(qfb_sum h, qfb_state dst, qfb_state src) {
         if (g.h >= src->nqubit)
             return fail(QFB_EINVAL, "qfb_sum_apply: operator acts on qubit %d of a %d-qubit state",
                         g.h, src->nqubit);
-    int rc = ensure_tiles(h, src->nqubit);
+    int rc = ensure_tiles(h);
     if (rc) return rc;
     return enqueue_sum_apply(h, dst->d, src->d, src->nbasis, src->nbatch);
 }
@@ -1890,8 +1923,7 @@ static int enqueue_prog(const qfb_prog_s *p, double2 *psi, int nqubit, int B,
 }
 
 
-static int ensure_tiles(qfb_sum_s *h, int nqubit) {
-    if (nqubit < kSumTileBits) return QFB_OK;
+static int ensure_tiles(qfb_sum_s *h) {
     // sums are shared between threads
     static std::mutex mu;
     std::lock_guard<std::mutex> lk(mu);
@@ -1916,8 +1948,9 @@ static int ensure_tiles(qfb_sum_s *h, int nqubit) {
                     ft.push_back(zc);
                 }
             }
-    // the warps take consecutive groups of about equal work: a block about 30
-    // instructions, a group's amplitudes about 45
+    // the warps take consecutive blocks of about equal work (a block about 30
+    // instructions, a group's amplitudes about 45); a cut inside a group makes two
+    // groups of it, whose products with the amplitudes are summed as all others are
     std::vector<int32_t> slice(kSumWarps + 1, (int32_t)fb.size());
     {
         auto cost = [](const SumBlock &b) { return (int64_t)(30 + (b.fl & 1u ? 45 : 0)); };
@@ -1927,8 +1960,11 @@ static int ensure_tiles(qfb_sum_s *h, int nqubit) {
         int w = 1;
         for (size_t i = 0; i < fb.size(); ++i) {
             at += cost(fb[i]);
-            if (fb[i].fl & 2u)
-                while (w < kSumWarps && at * kSumWarps >= all * w) slice[(size_t)w++] = (int32_t)i + 1;
+            while (w < kSumWarps && at * kSumWarps >= all * w) {
+                slice[(size_t)w++] = (int32_t)i + 1;
+                fb[i].fl |= 2u;
+                if (i + 1 < fb.size()) fb[i + 1].fl |= 1u;
+            }
         }
     }
     fb.resize(fb.size() + 2 * kSumAhead, SumBlock{0, 0, 0});
@@ -1957,16 +1993,22 @@ static int ensure_tiles(qfb_sum_s *h, int nqubit) {
 
 static int enqueue_sum_apply(const qfb_sum_s *h, double2 *dst, const double2 *src,
                              uint64_t nbasis, int B) {
-    if (h->tiles && nbasis >> kSumTileBits)
-        return launch_tiles<false>(h, dst, nullptr, src, nbasis, B, nullptr);
-    if (nbasis >= 4) {
-        const dim3 grid(grid_for(nbasis >> 2, 256), B);
-        k_sum_apply4<<<grid, 256, 0, t_stream>>>(dst, src, nbasis, h->d_groups, h->d_terms,
-                                                 h->d_rterms, h->ngroups);
-    } else {
-        const dim3 grid(grid_for(nbasis, 256), B);
-        k_sum_apply<<<grid, 256, 0, t_stream>>>(dst, src, nbasis, h->d_groups, h->d_terms,
-                                                h->ngroups);
+    const uint64_t total = nbasis * (uint64_t)B;
+    switch (sum_form(h, nbasis, B)) {
+        case SUM_TILES:
+            return launch_tiles<false>(h, dst, nullptr, src, nbasis, B, nullptr);
+        case SUM_QUADS: {
+            auto k = total <= 1ull << 32 ? k_sum_apply4<1, uint32_t> : k_sum_apply4<1, uint64_t>;
+            k<<<grid_for(total >> 2, 256), 256, 0, t_stream>>>(dst, src, total, 1, h->d_groups, h->d_terms,
+                                                               h->d_rterms, h->ngroups);
+            break;
+        }
+        case SUM_QUADS4: {
+            auto k = nbasis <= 1ull << 32 ? k_sum_apply4<4, uint32_t> : k_sum_apply4<4, uint64_t>;
+            k<<<grid_for((nbasis >> 2) * (uint64_t)((B + 3) / 4), 256), 256, 0, t_stream>>>(
+                dst, src, nbasis, B, h->d_groups, h->d_terms, h->d_rterms, h->ngroups);
+            break;
+        }
     }
     QFB_LAUNCHED();
     return QFB_OK;
@@ -4363,7 +4405,7 @@ static int ucc_create_impl(qfb_prog fprog, qfb_prog gprog, qfb_prog uprog, qfb_s
         for (const auto &sd : p->h_strs)
             if (sd.z >> nqubit) return fail(QFB_EINVAL, "qfb_ucc_create: program beyond qubit");
     }
-    int prc = ensure_tiles(ham, nqubit);
+    int prc = ensure_tiles(ham);
     if (prc == QFB_OK) prc = ensure_plans(fprog, nqubit, true);
     if (prc == QFB_OK && gprog) prc = ensure_plans(gprog, nqubit, false, uprog);
     if (prc) return prc;
