@@ -289,11 +289,15 @@ QFB_API int qfb_ucc_path(qfb_ucc u, int32_t *path);
 /* 1 when the evaluator's compact states are stored as real doubles (see
  * qfb_ucc_config), else 0.  No counterpart in the reference. */
 QFB_API int qfb_ucc_real_states(qfb_ucc u, int32_t *real);
-/* Parameter sets one CTA of the compact shared-memory forward program holds:
- * 2 with real states (two sets in one 16-byte slot per amplitude, for
- * batches of more sets than the SMs take at once), 1 otherwise, 0 off the compact shared-memory path.  No counterpart in the
- * reference. */
+/* Parameter sets one CTA of the compact shared-memory forward program can hold:
+ * 2 with real states (two sets in one 16-byte slot per amplitude), 1 otherwise,
+ * 0 off the compact shared-memory path.  Whether the evaluator's batch is run
+ * so: qfb_ucc_forward_sets.  No counterpart in the reference. */
 QFB_API int qfb_ucc_sets_per_cta(qfb_ucc u, int32_t *sets);
+/* Parameter sets a CTA of this evaluator's forward program takes: 2 where a CTA
+ * can hold two and one each would queue for the SMs, else 1; 0 off the compact
+ * shared-memory path.  No counterpart in the reference. */
+QFB_API int qfb_ucc_forward_sets(qfb_ucc u, int32_t *sets);
 /* Entries of the H rows the compact path streams for each parameter set (0
  * on the other paths).  No counterpart in the reference. */
 QFB_API int qfb_ucc_rows(qfb_ucc u, int64_t *nnz);

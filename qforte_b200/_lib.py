@@ -47,6 +47,7 @@ SIGNATURES = {
     "qfb_set_tile_wait_limit": (ctypes.c_int, [_u64]),
     "qfb_gates_dense": (ctypes.c_int, [ctypes.c_int]),
     "qfb_ucc_sets_per_cta": (ctypes.c_int, [_vp, _vp]),
+    "qfb_ucc_forward_sets": (ctypes.c_int, [_vp, _vp]),
     "qfb_c64_create": (ctypes.c_int, [ctypes.c_int, _vp]),
     "qfb_c64_destroy": (ctypes.c_int, [_vp]),
     "qfb_c64_reset": (ctypes.c_int, [_vp]),

@@ -3927,6 +3927,13 @@ static int sector_smem_attr() {
     return err == cudaSuccess ? QFB_OK : cuda_fail(err, "sector evaluator shared memory");
 }
 
+// Whether the forward program takes its sets in pairs: where single ones would
+// queue (us, single / paired: 16 qubits, 160 sets 106 / 94, 512 sets 213 / 187; 14
+// qubits 23 / 24 and 41 / 34; 12 qubits 11.6 / 13.1 and 20.4 / 18.1).
+static bool forward_paired(const qfb_ucc_s *u) {
+    return u->paired && u->nbatch > sm_count() * (u->SLp.fwd.nth >= 256 ? 1 : 2);
+}
+
 template <class V>
 static int ucc_stage_compact_v(qfb_ucc u, int stage, int with_grad) {
     const qfbs::SLaunch &L = u->SL;
@@ -3935,10 +3942,7 @@ static int ucc_stage_compact_v(qfb_ucc u, int stage, int with_grad) {
     switch (stage) {
         case 1:
             if constexpr (sizeof(V) == sizeof(double)) {
-                // pairs of sets where single ones would queue (us, single / paired: 16
-                // qubits, 160 sets 106 / 94, 512 sets 213 / 187; 14 qubits 23 / 24
-                // and 41 / 34; 12 qubits 11.6 / 13.1 and 20.4 / 18.1)
-                if (u->paired && u->nbatch > sm_count() * (u->SLp.fwd.nth >= 256 ? 1 : 2)) {
+                if (forward_paired(u)) {
                     const qfbs::SLaunch &LP = u->SLp;
                     qfbs::k_sector_forward_pr<<<(u->nbatch + 1) / 2, LP.fwd.nth,
                                                 qfbs::step_smem<qfbs::PCoefPR>(1, L.nsec, sizeof(double2), LP.fwd.n),
@@ -4595,6 +4599,12 @@ int qfb_ucc_real_states(qfb_ucc u, int32_t *real) {
 int qfb_ucc_sets_per_cta(qfb_ucc u, int32_t *sets) {
     if (!u || !sets) return fail(QFB_EINVAL, "qfb_ucc_sets_per_cta: null argument");
     *sets = u->compact ? (u->paired ? 2 : 1) : 0;
+    return QFB_OK;
+}
+
+int qfb_ucc_forward_sets(qfb_ucc u, int32_t *sets) {
+    if (!u || !sets) return fail(QFB_EINVAL, "qfb_ucc_forward_sets: null argument");
+    *sets = u->compact ? (forward_paired(u) ? 2 : 1) : 0;
     return QFB_OK;
 }
 

@@ -48,7 +48,7 @@ __all__ = ["DUCC", "Evaluator", "Pack", "evaluator_config", "UCCNVQE", "ADAPTVQE
 def evaluator_config(compact=True):
     """Process-wide: let evaluators created from now on use the compact
     sector paths (True, the default; real states where every coefficient is
-    real, two parameter sets per CTA in the forward program), the same with
+    real, two parameter sets per CTA in the forward program of large batches), the same with
     one set per CTA ("one-set"), with complex state storage ("complex"), only the
     global-memory one ("global"; "global-complex" with complex storage), or
     keep full-space states (False)."""
@@ -102,10 +102,18 @@ class Evaluator:
 
     @property
     def sets_per_cta(self):
-        """Parameter sets a CTA of the compact forward program holds (2: two
+        """Parameter sets a CTA of the compact forward program can hold (2: two
         real sets per 16-byte slot; 0: not the compact shared path)."""
         n = ctypes.c_int32()
         check(lib().qfb_ucc_sets_per_cta(self.h, ctypes.byref(n)), "qfb_ucc_sets_per_cta")
+        return n.value
+
+    @property
+    def forward_sets(self):
+        """Parameter sets a CTA of this evaluator's forward program takes (2 for
+        batches that one set each would make queue for the SMs)."""
+        n = ctypes.c_int32()
+        check(lib().qfb_ucc_forward_sets(self.h, ctypes.byref(n)), "qfb_ucc_forward_sets")
         return n.value
 
     @property
