@@ -2779,13 +2779,46 @@ struct RoundHost {
     std::vector<int32_t> param;                // per record: parameter of its inner product, or -1
 };
 
+// Whether a pattern's coefficients (gn, hn) are f times another's.
+static bool coef_is(const CStep::Pat &a, const CStep::Pat &b, double f) {
+    return a.gn.x == f * b.gn.x && a.gn.y == f * b.gn.y && a.hn.x == f * b.hn.x && a.hn.y == f * b.hn.y;
+}
+
+// Records of one step (push_rounds): its distinct coefficients.
+static int step_records(const CStep &cs) {
+    int n = 0;
+    for (size_t k = 0; k < cs.pats.size(); ++k) {
+        bool first = true;
+        for (size_t l = 0; l < k && first; ++l)
+            first = !coef_is(cs.pats[k], cs.pats[l], 1.0) && !coef_is(cs.pats[k], cs.pats[l], -1.0);
+        n += first;
+    }
+    return n;
+}
+
+// Shared memory of the sweep (and of a packed item): both states and the constants.
+static size_t compact_smem(int real, int nsec, int nfwd, int nsweep) {
+    const int n = std::max(nfwd, nsweep);
+    return real ? qfbs::step_smem<qfbs::PCoef<true, double>>(2, nsec, sizeof(double), n)
+                : qfbs::step_smem<qfbs::PCoef<true, double2>>(2, nsec, sizeof(double2), n);
+}
+
+// Whether the step kernels' records fit in shared memory beside the states: a step
+// whose patterns differ in their coefficients takes a record for each (one more
+// record fills a stream up to whole rounds).
+static bool records_fit(const SectorPlan &sp, bool real) {
+    int64_t nf = 1, nw = 1;
+    for (const CStep &cs : sp.fsteps) nf += step_records(cs);
+    for (const auto &it : sp.sweep_items) nw += step_records(it.unrot ? sp.usteps[it.step] : sp.ksteps[it.step]);
+    return std::max(nf, nw) < 1 << 16 && compact_smem(real, sp.nsec, (int)nf, (int)nw) <= kStepSmemMax;
+}
+
 // Append one step: a record per pair of pattern coefficients (gn, hn) that
 // differ by more than a sign (a pattern whose coefficients are another's
 // negated joins it with its pairs' signs flipped), its pairs ordered for S
 // bank slots.
 static bool push_rounds(RoundHost &P, const SectorPlan &sp, const CStep &cs, int flags, int S) {
     if (sp.nsec + qfbs::kRoundPad > (1 << qfbs::kPairIdxBits)) return false;
-    auto is = [](double2 a, double2 b, double f) { return a.x == f * b.x && a.y == f * b.y; };
     std::vector<char> done(cs.pats.size(), 0);
     for (size_t k = 0; k < cs.pats.size(); ++k) {
         if (done[k]) continue;
@@ -2793,8 +2826,8 @@ static bool push_rounds(RoundHost &P, const SectorPlan &sp, const CStep &cs, int
         std::vector<uint32_t> pr;
         for (size_t l = k; l < cs.pats.size(); ++l) {
             const auto &pt = cs.pats[l];
-            const bool same = is(pt.gn, p0.gn, 1.0) && is(pt.hn, p0.hn, 1.0);
-            if (done[l] || !(same || (is(pt.gn, p0.gn, -1.0) && is(pt.hn, p0.hn, -1.0)))) continue;
+            const bool same = coef_is(pt, p0, 1.0);
+            if (done[l] || !(same || coef_is(pt, p0, -1.0))) continue;
             done[l] = 1;
             for (const qfbs::SEntry &ea : pt.a)
                 for (const qfbs::SEntry &eb : pt.b) {
@@ -3779,13 +3812,6 @@ static int win_smem_attr() {
     return err == cudaSuccess ? QFB_OK : cuda_fail(err, "window shared memory");
 }
 
-// Shared memory of the sweep (and of a packed item): both states and the constants.
-static size_t compact_smem(int real, int nsec, int nfwd, int nsweep) {
-    const int n = std::max(nfwd, nsweep);
-    return real ? qfbs::step_smem<qfbs::PCoef<true, double>>(2, nsec, sizeof(double), n)
-                : qfbs::step_smem<qfbs::PCoef<true, double2>>(2, nsec, sizeof(double2), n);
-}
-
 // Attach a compact plan and its H rows to an evaluator (shared memory or,
 // with `global`, global memory states).
 static int sector_attach(qfb_ucc u, qfb_sum_s *ham, const std::shared_ptr<SectorPlan> &plan,
@@ -4444,6 +4470,11 @@ static int ucc_create_impl(qfb_prog fprog, qfb_prog gprog, qfb_prog uprog, qfb_s
         };
         if (g_ucc_compact == 1 || g_ucc_compact == 4 || g_ucc_compact == 6) {  // 2, 3: global memory only (3: sigma without stored rows)
             plan = get_plan(true);
+            if (plan) {
+                bool real = !ucc_complex_states() && stream_is_real(plan->fwd) && stream_is_real(plan->sweep);
+                for (const SecGroup &g : sgroups) real = real && g.real;
+                if (!records_fit(*plan, real)) plan = nullptr;
+            }
             compact = plan != nullptr;
         }
         if (!compact) {
