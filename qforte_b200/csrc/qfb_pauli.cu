@@ -3016,7 +3016,7 @@ static int64_t win_max_class(int m, int k, int q) {
     return best;
 }
 
-static int build_windows(const SectorPlan &sp, const std::vector<WinRef> &refs, int nparam,
+static int build_windows(const SectorPlan &sp, const std::vector<WinRef> &refs, int nparam, bool sweep,
                          std::shared_ptr<WinProg> *out) {
     const size_t n = refs.size();
     auto P = std::make_shared<WinProg>();
@@ -3096,7 +3096,7 @@ static int build_windows(const SectorPlan &sp, const std::vector<WinRef> &refs, 
         aparam.push_back(r.cs->param);
         return (int32_t)gamma.size() - 1;
     };
-    size_t lim = n;  // end of the window at hand when its pairs outgrew kWinPairs
+    size_t lim = n;  // end of the window at hand when it outgrew kWinPairs, kWinBlobMax or shared memory
     for (size_t i = 0; i < n;) {
         uint64_t qa = 0, qb = 0;
         size_t j = i, ni = 0;
@@ -3158,24 +3158,25 @@ static int build_windows(const SectorPlan &sp, const std::vector<WinRef> &refs, 
                     pairs = nr << (5 + lg);
                 }
             }
-            bool ok = fits;
-            if (ok && pairs > kWinPairs && j - i > (size_t)kWinMinSteps) {  // fewer steps
+            w.nitem = (int32_t)la.size();
+            w.mab = sa * sb;
+            w.mranks = sa + sb;
+            w.mwords = wa + wb;
+            const bool ok = fits && pairs <= kWinPairs &&
+                            qfbv::win_smem(w, 1, 1 << w.lg, sweep, sizeof(double2)) <= kWinSmemMax;
+            if (!ok && j - i > (size_t)kWinMinSteps) {  // fewer steps
+                const double part = fits && pairs > kWinPairs ? 0.9 * kWinPairs / (double)pairs : 0.75;
                 cls.resize(m0);
                 rank.resize(m1);
                 blob.resize(m2);
-                lim = i + std::max<size_t>(kWinMinSteps, (size_t)((double)(j - i) * 0.9 * kWinPairs / pairs));
+                lim = i + std::max<size_t>(kWinMinSteps, (size_t)((double)(j - i) * part));
                 continue;
             }
-            ok = ok && pairs <= kWinPairs;
             lim = n;
             if (ok) {
                 w.nca = (int32_t)CA.str.size();
                 w.ncb = (int32_t)CB.str.size();
                 w.item0 = (int32_t)items.size();
-                w.nitem = (int32_t)la.size();
-                w.mab = sa * sb;
-                w.mranks = sa + sb;
-                w.mwords = wa + wb;
                 const int64_t nblk = (int64_t)w.nca * w.ncb;
                 size_t at = 0;
                 int32_t r0 = 0;
@@ -3273,7 +3274,7 @@ static int plan_windows(SectorPlan &sp, int nparam) {
         std::vector<WinRef> refs;
         for (size_t i = 0; i < sp.fsteps.size(); ++i)
             refs.push_back(WinRef{&sp.fsteps[i], qfbs::R_ROT, (int)i});
-        const int rc = build_windows(sp, refs, nparam, &sp.wfwd);
+        const int rc = build_windows(sp, refs, nparam, false, &sp.wfwd);
         if (rc) return rc;
     }
     if (!sp.wsweep) {
@@ -3282,7 +3283,7 @@ static int plan_windows(SectorPlan &sp, int nparam) {
             const auto &it = sp.sweep_items[i];
             refs.push_back(WinRef{it.unrot ? &sp.usteps[it.step] : &sp.ksteps[it.step], it.flags, (int)i});
         }
-        const int rc = build_windows(sp, refs, nparam, &sp.wsweep);
+        const int rc = build_windows(sp, refs, nparam, true, &sp.wsweep);
         if (rc) return rc;
     }
     return QFB_OK;
