@@ -58,6 +58,11 @@ class QubitOperator:
     def __init__(self):
         self._t = _Terms()  # [coeff, Circuit]
 
+    def __setstate__(self, state):
+        # (pickles of operators whose terms were a plain list)
+        t = state[1]["_t"]
+        self._t = t if isinstance(t, _Terms) else _Terms(t)
+
     # -- building (bindings.cc:95-116) ----------------------------------------
     def add(self, *args):
         if len(args) == 1:
