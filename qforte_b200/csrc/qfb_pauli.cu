@@ -4118,11 +4118,16 @@ static int win_program(qfb_ucc u, const WinProg &P, bool sweep, const qfbg::GLau
             int lspc;
             size_t smem;
             win_shape(op.w, B, sweep, sizeof(V), lspc, smem);
-            const dim3 grid((unsigned)(op.w.nca * op.w.ncb), (unsigned)((B + (1 << lspc) - 1) >> lspc));
             const dim3 block(32u << (op.w.lg + lspc));
-            QFB_CUDA(launch_pdl(sweep ? qfbv::k_win<true, V> : qfbv::k_win<false, V>, grid, block, smem, t_stream,
-                                L, op.w, P.tabs, (const double2 *)ang, (double)sign, rev ? 1 : 0, lspc,
-                                u->g_wpart));
+            for (int s0 = 0; s0 < B; s0 += 65535 << lspc) {  // grid.y's limit
+                const dim3 grid((unsigned)(op.w.nca * op.w.ncb),
+                                std::min(65535u, (unsigned)((B - s0 + (1 << lspc) - 1) >> lspc)));
+                QFB_CUDA(launch_pdl(sweep ? qfbv::k_win<true, V> : qfbv::k_win<false, V>, grid, block, smem, t_stream,
+                                    L, op.w, P.tabs, (const double2 *)ang, (double)sign, rev ? 1 : 0, lspc, s0,
+                                    u->g_wpart));
+                QFB_LAUNCHED();
+            }
+            continue;
         }
         QFB_LAUNCHED();
     }

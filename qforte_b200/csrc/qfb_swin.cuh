@@ -152,16 +152,16 @@ __global__ void __launch_bounds__(256) k_win_angles(const double *__restrict__ g
                                                     const int32_t *__restrict__ param, int n, int B,
                                                     const double *__restrict__ params, int nparam,
                                                     double2 *__restrict__ ang) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n * B) return;
-    const int i = t / B, s = t - i * B;
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (int64_t)n * B) return;
+    const int i = (int)(t / B), s = (int)(t - (int64_t)i * B);
     double sn, cs;
     sincos(gamma[i] * params[(size_t)s * nparam + param[i]], &sn, &cs);
     ang[t] = make_double2(cs, sn);
 }
 
-// Apply window W to every block and slot.  grid = (blocks, slot groups);
-// 1 << lspc slots per CTA, 1 << W.lg warps per slot.  rev: items in reverse
+// Apply window W to every block and the slots from slot0 on.  grid = (blocks, slot
+// groups); 1 << lspc slots per CTA, 1 << W.lg warps per slot.  rev: items in reverse
 // order; sign multiplies every angle (rev with sign -1: the exact inverse).
 //
 // Bound by the latency of one round after another (a barrier, a shared-memory
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(256) k_win_angles(const double *__restrict__ g
 template <bool SWEEP, class V>
 __global__ void __launch_bounds__(kWinThreads) k_win(GLaunch L, VWin W, VTabs T,
                                                      const double2 *__restrict__ ang, double sign, int rev,
-                                                     int lspc, double *__restrict__ partial) {
+                                                     int lspc, int slot0, double *__restrict__ partial) {
     extern __shared__ __align__(16) unsigned char w_raw[];
     const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nth >> 5;
     const int spc = 1 << lspc, ni = W.nitem, nr = W.nround, lg = W.lg, G = 32 << lg;
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(kWinThreads) k_win(GLaunch L, VWin W, VTabs T,
     __syncthreads();  // s_g is read by other threads than wrote it
     qfbg::g_pdl_enter();
 
-    const int s0 = blockIdx.y << lspc;
+    const int s0 = slot0 + ((int)blockIdx.y << lspc);
     V *psi = reinterpret_cast<V *>(L.psi), *sig = reinterpret_cast<V *>(L.sig);
     for (int i = tid; i < (nab + 32) << lspc; i += nth) {
         const int e = i >> lspc, sl = i & (spc - 1);
