@@ -2087,31 +2087,50 @@ static int enqueue_gradient(const qfb_prog_s *kp, const qfb_prog_s *up, double2 
     return QFB_OK;
 }
 
-// A program's strings in the order they apply, when each acts on at most two
-// qubits.
-static bool prog_rotations(const qfb_prog_s *p, const double *params, int sign, std::vector<PauliRot> &out) {
-    const size_t n = p->h_strs.size();
-    std::vector<uint64_t> x(n);
+// A program of strings on at most two qubits may run as gates: the tile kernel works
+// several strings a register phase, a window kernel pass (or a step's launch, in the
+// inverse) one step.  Below 14 qubits the windows are as fast; from 2^21 amplitudes
+// on, where either reads the state from HBM, gates always win.  In between a step
+// of many strings on one x-mask (products of Z) costs the windows little and the
+// gates two each, so the times are estimated: us, fitted at 14 to 18 qubits.
+//
+// us, windows / gates (the inverse: steps / gates): Ising chain, 6 Trotter steps, 14
+// qubits 278 / 148 (372 / 142), 18 qubits 379 / 197 (517 / 213), 20 qubits 560 / 198, 23
+// qubits 3,819 / 1,749; Heisenberg chain, 6 steps, 14 qubits 462 / 393 (669 / 393), 20
+// qubits 947 / 585; 100 random pairs, 14 qubits 228 / 214 (413 / 214); Z Z on all pairs
+// and X, twice, 14 qubits 208 / 247 (147 / 228), 18 qubits 329 / 430 (270 / 426), 21
+// qubits 1,320 / 725.  The fused products are rounded once: on 23 qubits, 6 steps, an
+// error against 64 bits of 6.0e-15, window by window 5.8e-15.
+constexpr int kProgGateQubits = 14;
+
+static bool prog_as_gates(const qfb_prog_s *p, qfb_state s, int sign) {
+    if (s->nqubit < kProgGateQubits || !gate_tiles_on()) return false;
+    double two = 0.0, four = 0.0;  // 2 x 2 and 4 x 4 gates
     for (const StepDev &st : p->h_steps)
-        for (int k = st.s0; k < st.s0 + st.ns; ++k) x[(size_t)k] = st.x;
-    for (size_t k = 0; k < n; ++k)
-        if (__builtin_popcountll(x[k] | p->h_strs[k].z) > 2) return false;
-    out.reserve(n);
-    for (size_t i = 0; i < n; ++i) {
-        const size_t k = sign > 0 ? i : n - 1 - i;
-        const StrDev &sd = p->h_strs[k];
-        out.push_back(PauliRot{x[k], sd.z, (int)sd.ny, (double)sign * sd.scale * params[sd.param]});
-    }
-    return true;
+        for (int k = st.s0; k < st.s0 + st.ns; ++k) {
+            const int m = __builtin_popcountll(st.x | p->h_strs[(size_t)k].z);
+            if (m > 2) return false;
+            if (m < 2) two += 1.0;
+            else if (st.x == 0) two += 2.0;
+            else four += 1.0;
+        }
+    if (s->nbasis * (uint64_t)s->nbatch >= 1ull << 21 || two + four <= 1.0) return true;
+    const double steps = (double)p->h_steps.size(), strs = (double)p->h_strs.size();
+    const double gates = 9.0 + 0.62 * two + 1.95 * four;
+    return gates < (sign > 0 ? 10.0 + 1.8 * steps + 0.72 * strs : 3.0 + 4.1 * steps);
 }
 
-// States from this many qubits on take a program of short strings as gates: the
-// tile kernel works several strings a register phase, a window kernel pass one.
-// The fused products are rounded once (an error against 64 bits no larger than the
-// windows', 5.8e-15 on 23 qubits).  Transverse-field Ising chain, 6 Trotter steps, us,
-// windows / gates: 12 qubits 192 / 204, 14 qubits 287 / 222, 18 qubits 399 / 296, 20
-// qubits 576 / 433, 23 qubits 3,819 / 1,749, 25 qubits 16,024 / 6,892.
-constexpr int kProgGateQubits = 14;
+// The program's strings in the order they apply.
+static std::vector<PauliRot> prog_rotations(const qfb_prog_s *p, const double *params, int sign) {
+    std::vector<PauliRot> out(p->h_strs.size());
+    for (const StepDev &st : p->h_steps)
+        for (int k = st.s0; k < st.s0 + st.ns; ++k) {
+            const StrDev &sd = p->h_strs[(size_t)k];
+            out[sign > 0 ? (size_t)k : out.size() - 1 - (size_t)k] =
+                PauliRot{st.x, sd.z, (int)sd.ny, (double)sign * sd.scale * params[sd.param]};
+        }
+    return out;
+}
 
 int qfb_prog_apply(qfb_prog p, qfb_state s, const double *params, int32_t nrows, int32_t sign) {
     if (!p || !s) return fail(QFB_EINVAL, "qfb_prog_apply: null argument");
@@ -2120,10 +2139,7 @@ int qfb_prog_apply(qfb_prog p, qfb_state s, const double *params, int32_t nrows,
     int rc = check_prog_state(p, s, nrows, "qfb_prog_apply");
     if (rc) return rc;
     if (p->h_steps.empty()) return QFB_OK;
-    if (nrows == 1 && s->nqubit >= kProgGateQubits && gate_tiles_on()) {
-        std::vector<PauliRot> rots;
-        if (prog_rotations(p, params, sign, rots)) return apply_rotations(s, rots);
-    }
+    if (nrows == 1 && prog_as_gates(p, s, sign)) return apply_rotations(s, prog_rotations(p, params, sign));
     if (sign > 0) {
         rc = ensure_plans(p, s->nqubit, true);
         if (rc) return rc;
