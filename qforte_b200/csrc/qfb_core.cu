@@ -673,11 +673,7 @@ struct WindowPlanner {
             Q |= best;
             run(Q, best);
         }
-        if (sel.empty()) {
-            // no gate fits a tile of this shape: a ready one's own pass
-            for (int q = 0; q < n && sel.empty(); ++q) run(all, front(q) < 0 ? 0 : 1ull << q);
-            undo(1);
-        }
+        // (a ready gate always fits: b leaves two qubits beside the lowest L)
         left -= (int64_t)sel.size();
         pw = GatePlanWin{};
         if (sel.size() == 1) {
