@@ -185,6 +185,61 @@ __global__ void k_seg_sum(const double2 *__restrict__ partial, const int32_t *__
     if (threadIdx.x == 0) out[(uint64_t)b * gridDim.x + s] = acc;
 }
 
+// dst = O src on a few states below 8 qubits (total amplitudes in all): a lane's
+// output is summed in the order of the groups and their terms, as the reference sums
+// it (Krylov methods on spin-degenerate systems read eigenvectors that rounding
+// decides).  The order binds one lane to a chain of additions a group, so the rest is
+// taken off it: the block's warps form the coefficients of 16 groups and fetch their
+// amplitudes while warp 0 adds up the 16 before.
+constexpr int kSmallGroups = 16;
+__global__ void __launch_bounds__(256) k_sum_small(
+    double2 *__restrict__ dst, const double2 *__restrict__ src, uint32_t total,
+    const GroupDev *__restrict__ groups, const TermDev *__restrict__ terms,
+    const double2 *__restrict__ rterms, int32_t ngroups) {
+    __shared__ double2 s_f[2][kSmallGroups][32], s_a[2][kSmallGroups][32];
+    __shared__ int s_real[2][kSmallGroups];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t k = min((uint32_t)blockIdx.x * 32u + lane, total - 1u);
+    double2 acc = make_double2(0.0, 0.0);
+    for (int g0 = 0; g0 < ngroups + kSmallGroups; g0 += kSmallGroups) {
+        const int buf = g0 / kSmallGroups & 1;
+        for (int i = warp; i < kSmallGroups && g0 + i < ngroups; i += 8) {
+            const GroupDev gr = groups[g0 + i];
+            const uint32_t j = k ^ (uint32_t)gr.x;
+            s_a[buf][i][lane] = src[j];
+            if (lane == 0) s_real[buf][i] = gr.real;
+            double2 f = make_double2(0.0, 0.0);
+            if (gr.real) {
+#pragma unroll 4
+                for (int t = gr.begin; t < gr.end; ++t) {
+                    const double2 zc = __ldg(&rterms[t]);
+                    f.x += qfbs::v_flip(zc.y, (uint32_t)__popc(j & (uint32_t)__double_as_longlong(zc.x)) << 31);
+                }
+            } else {
+                for (int t = gr.begin; t < gr.end; ++t) {
+                    const uint32_t odd = (uint32_t)__popc(j & (uint32_t)__ldg(&terms[t].z)) << 31;
+                    f = c_add(f, qfbs::v_flip(terms[t].c, odd));
+                }
+            }
+            s_f[buf][i][lane] = f;
+        }
+        if (warp == 0 && g0 > 0) {
+            const int n = min(kSmallGroups, ngroups - (g0 - kSmallGroups));
+            for (int i = 0; i < n; ++i) {
+                const double2 f = s_f[buf ^ 1][i][lane], x = s_a[buf ^ 1][i][lane];
+                if (s_real[buf ^ 1][i]) {
+                    acc.x += f.x * x.x;
+                    acc.y += f.x * x.y;
+                } else {
+                    acc = c_add(acc, c_mul(f, x));
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (warp == 0 && blockIdx.x * 32u + lane < total) dst[k] = acc;
+}
+
 // dst = O src with four outputs per thread, for NS states at a time: k = k0 | d,
 // d = 0..3.  For a group x the four inputs j_d = (k0 ^ x) ^ d form one aligned quad,
 // and popcount(j_d & z) = popcount((k0 ^ x) & z) + popcount(d & z): one parity per
@@ -1511,18 +1566,21 @@ static void make_table(qfb_prog_s *p, StepDev &st) {
 
 // The kernel of H psi: by estimates of each one's time for G groups of T terms in all
 // (us, 2^26 amplitudes, fitted to 1 to 24 groups of 1 to 300 terms).  Below 2^18
-// amplitudes every kernel waits for its own latency, which the tiles share best.
+// amplitudes every kernel waits for its own latency, which the tiles share best; a
+// few states below 8 qubits keep the order of the sums (k_sum_small).
 // us, tiles / quads / quads of 4 states: 20 qubits, 64 states: one string 1,282 / 395 /
 // 411, 8 groups of 6 terms 1,725 / 1,746 / 1,635, 24 of 6 3,090 / 5,330 / 4,550, 200
 // diagonal terms 3,343 / 4,086 / 1,150; 20 qubits, one state: one string 21 / 10 / -,
 // 24 groups of 6 52 / 84 / -; 12 qubits, 8 states, 200 diagonal terms 6 / 28 / 23.
-enum SumForm { SUM_TILES, SUM_QUADS, SUM_QUADS4 };
+enum SumForm { SUM_SMALL, SUM_TILES, SUM_QUADS, SUM_QUADS4 };
 static SumForm sum_form(const qfb_sum_s *h, uint64_t nbasis, int B) {
-    if (nbasis < 4 || nbasis * (uint64_t)B < 1ull << 18) return SUM_TILES;
+    const uint64_t total = nbasis * (uint64_t)B;
+    if (nbasis < 1ull << kSumTileBits && total < 4096) return SUM_SMALL;
+    if (nbasis < 4 || total < 1ull << 18) return SUM_TILES;
     const double G = h->ngroups, T = (double)h->nterms, NB = (T + 3.0 * G) / 4.0;
     const double tiles = 1150.0 + 40.0 * std::max(G, std::min(8.0, NB)) + 25.0 * NB;
     const double quads = 400.0 + 110.0 * G + 20.0 * T;
-    const double quads4 = B < 4 || nbasis * (uint64_t)B < 1ull << 20 ? quads : 400.0 + 180.0 * G + 6.0 * T;
+    const double quads4 = B < 4 || total < 1ull << 20 ? quads : 400.0 + 180.0 * G + 6.0 * T;
     if (tiles <= std::min(quads, quads4)) return SUM_TILES;
     return quads <= quads4 ? SUM_QUADS : SUM_QUADS4;
 }
@@ -1995,6 +2053,10 @@ static int enqueue_sum_apply(const qfb_sum_s *h, double2 *dst, const double2 *sr
                              uint64_t nbasis, int B) {
     const uint64_t total = nbasis * (uint64_t)B;
     switch (sum_form(h, nbasis, B)) {
+        case SUM_SMALL:
+            k_sum_small<<<(unsigned)((total + 31) / 32), 256, 0, t_stream>>>(
+                dst, src, (uint32_t)total, h->d_groups, h->d_terms, h->d_rterms, h->ngroups);
+            break;
         case SUM_TILES:
             return launch_tiles<false>(h, dst, nullptr, src, nbasis, B, nullptr);
         case SUM_QUADS: {
