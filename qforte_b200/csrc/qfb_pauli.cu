@@ -1822,7 +1822,7 @@ int qfb_sum_apply(qfb_sum h, qfb_state dst, qfb_state src) {
         if (g.h >= src->nqubit)
             return fail(QFB_EINVAL, "qfb_sum_apply: operator acts on qubit %d of a %d-qubit state",
                         g.h, src->nqubit);
-    int rc = ensure_tiles(h);
+    const int rc = sum_form(h, src->nbasis, src->nbatch) == SUM_TILES ? ensure_tiles(h) : QFB_OK;
     if (rc) return rc;
     return enqueue_sum_apply(h, dst->d, src->d, src->nbasis, src->nbatch);
 }
@@ -4519,7 +4519,7 @@ static int ucc_create_impl(qfb_prog fprog, qfb_prog gprog, qfb_prog uprog, qfb_s
         for (const auto &sd : p->h_strs)
             if (sd.z >> nqubit) return fail(QFB_EINVAL, "qfb_ucc_create: program beyond qubit");
     }
-    int prc = ensure_tiles(ham);
+    int prc = sum_form(ham, 1ull << nqubit, nbatch) == SUM_TILES ? ensure_tiles(ham) : QFB_OK;
     if (prc == QFB_OK) prc = ensure_plans(fprog, nqubit, true);
     if (prc == QFB_OK && gprog) prc = ensure_plans(gprog, nqubit, false, uprog);
     if (prc) return prc;
