@@ -166,15 +166,16 @@ QFB_API int qfb_gates_regs(int reg_bits);
  * (complex64 states widened to FP64 for the products); 0 applies the phase's
  * gates one by one; 2 (the default) is 1 for states of 16 MiB and more
  * (complex64: 128 MiB) and 0 below.
- * Both forms give the result of the gates in list order (up to the rounding
- * of the fused products).  No counterpart in the reference; set by the
- * autotuner. */
+ * Both forms give the result of the gates in list order (a complex128 state's
+ * fused products are rounded once).  No counterpart in the reference; set by
+ * the autotuner. */
 QFB_API int qfb_gates_fused(int mode);
 /* Host only: the fused form of the tile runs qfb_apply_gates would apply to
  * one nqubit state (complex64 != 0: a complex64 state) under the current tile
  * shape, each phase checked as the device reads it (thread tables: every
  * thread-bit assignment once, offsets in the tile; segments: variant bits on
- * thread bits, shared by the 8 vectors of each n-block; matrices in range).
+ * thread bits, shared by the 8 vectors of each n-block; matrices in range, and
+ * those of complex128 states equal to long-double products rounded once).
  * Returns QFB_EINVAL on a failed check; else the fused phases, their
  * segments and matrix entries.  No counterpart in the reference. */
 QFB_API int qfb_gates_fused_plan(const qfb_gate *gates, int64_t ngates, int nqubit, int complex64,

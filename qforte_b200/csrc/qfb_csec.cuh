@@ -6,10 +6,12 @@
 // slots of one amplitude are contiguous and every access below is coalesced
 // across slots.  Runs of program steps go out as windows (qfb_swin.cuh); a
 // step by itself is one launch over (pair, slot): the pairs are the alpha-list
-// x beta-list products of the step's record, read from global memory.  sigma = H psi runs one warp per output amplitude with the lanes
-// over slots, from the sector's H rows, or (rows over their budget) one
-// x-group of H per launch from pair records.  When H and every step are real
-// the states are stored as doubles (V = double), else as complex (double2).
+// x beta-list products of the step's record, read from global memory.
+//
+// sigma = H psi runs one warp per output amplitude with the lanes over slots,
+// from the sector's H rows, or (rows over their budget) one x-group of H per
+// launch from pair records.  When H and every step are real the states are
+// stored as doubles (V = double), else as complex (double2).
 #pragma once
 
 #include <cstdint>
@@ -186,9 +188,8 @@ __global__ void __launch_bounds__(256) k_cg_ip_many(GLaunch L, const uint4 *__re
 // per pair and amplitude, become 16-byte gathers from shared memory.
 //
 // Bound by those (two 16-byte loads a pair).  Generalised singles and doubles
-// of 10 orbitals on 63,504 amplitudes (about 2e7 pairs): k_cg_ip_many 634 us,
-// this kernel 116 us (9
-// orbitals, 8 electrons, 15,876 amplitudes: 31 us).
+// of 10 orbitals on 63,504 amplitudes (4.2e7 pairs): k_cg_ip_many 634 us, this
+// kernel 116 us (9 orbitals, 8 electrons, 15,876 amplitudes: 31 us).
 struct GPoolTask {
     int32_t e0, ne;  // alpha entries
     int32_t k0, nk;  // beta lists
