@@ -13,6 +13,7 @@
 // 2,707 / 2,811 / 2,726.
 #include "qfb_ddrows.h"
 
+#if defined(__x86_64__)
 #include <immintrin.h>
 
 namespace qfbh {
@@ -91,3 +92,12 @@ void dd_mix(Rows8 &r, const int *k, int n, const double *m, unsigned halves) {
 }
 
 }  // namespace qfbh
+
+#else  // other hosts: the products in long double
+
+namespace qfbh {
+bool dd_available() { return false; }
+void dd_mix(Rows8 &, const int *, int, const double *, unsigned) {}
+}  // namespace qfbh
+
+#endif
