@@ -1226,6 +1226,10 @@ void plan_tile_phases(const WGate *g, int ng, int b, int R, qfbt::TRun &run, Til
     }
     run.np = (int)tp.ph.size() - run.p0;
     run.b = b;
+    if (!(fused && R == 3 && b - R >= 5) && run.np > 0) {
+        run.n0 = tp.ph[(size_t)run.p0].no;
+        for (int p = run.p0; p + 1 < run.p0 + run.np; ++p) tp.ph[(size_t)p].nm = tp.ph[(size_t)p + 1].no;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1440,7 +1444,7 @@ int launch_tile_runs(A *d, uint64_t nbasis, int nbatch, const std::vector<HGate>
     // the fused form
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const size_t bp = al(sizeof(qfbt::TPhase) * tp.ph.size());
-    const size_t bo = al(sizeof(qfbt::TOp) * (tp.ops.size() + qfbt::kStageOps));
+    const size_t bo = al(sizeof(qfbt::TOp) * tp.ops.size());
     const size_t bm = al(sizeof(double2) * tp.m4.size());
     const size_t bc = al(sizeof(uint64_t) * tp.chunks.size());
     const size_t bt = al(sizeof(uint32_t) * tp.threads.size());

@@ -70,7 +70,8 @@ struct TPhase {
     uint32_t soff[1 << kMaxRegBits];  // store: the same after the phase's relabelings
     int32_t o0, no;                   // ops of this phase
     int32_t th0;                      // this phase's entries of the thread table
-    int32_t nm;                       // fused form: matrix entries of its segments
+    int32_t nm;                       // fused form: matrix entries of its segments; gate
+                                      // by gate: ops of the run's next phase
     int32_t s0, ns;                   // fused form: segments of this phase
     int32_t sc;                       // fused form: per-thread factor table (-1: none)
     int32_t m0;                       // fused form: first matrix entry of its segments
@@ -126,6 +127,7 @@ struct TRun {
     int32_t ch0;     // first entry of this run's chunk table
     int32_t p0, np;  // phases
     int32_t o0, th0; // the first phase's ops and thread table
+    int32_t n0;      // the first phase's number of ops
 };
 // chunk table entry c of a run: the global offset of the tile's chunk c
 // (8 amplitudes on qubits 0..2), i.e. c's bits placed on the tile's qubits
@@ -653,9 +655,10 @@ __global__ void __launch_bounds__(256, F ? 4 : R == 4 ? 1 : 3)
             bulk_g2s(smem_u32(tile + tpad_of<A>((uint32_t)c << 3)), s + __ldg(&ch[c]), kChunk, bar_a);
         TStage *st = reinterpret_cast<TStage *>(
             t_smem + ((sizeof(A) * tpad_size_of<A>(b) + 16 + 15) & ~(size_t)15));
-        // phases follow one another in all three arrays (ops padded at the end)
-        auto fetch = [&](int p, int o0) {
-            constexpr int HW = (int)sizeof(TPhase) / 16, OW = kStageOps * (int)sizeof(TOp) / 16;
+        // phases follow one another in all three arrays
+        auto fetch = [&](int p, int o0, int no) {
+            constexpr int HW = (int)sizeof(TPhase) / 16;
+            const int OW = min(no, kStageOps) * ((int)sizeof(TOp) / 16);
             const int tw = nth / 4;  // 16-byte words of the thread table
             const uint4 *hs = reinterpret_cast<const uint4 *>(phases + run.p0 + p);
             const uint4 *os = reinterpret_cast<const uint4 *>(ops + o0);
@@ -668,7 +671,7 @@ __global__ void __launch_bounds__(256, F ? 4 : R == 4 ? 1 : 3)
             }
             cp_async_commit();
         };
-        if (run.np > 0) fetch(0, run.o0);
+        if (run.np > 0) fetch(0, run.o0, run.n0);
         const uint64_t limit = g_tile_wait_limit_ns;
         if (limit == 0 || !mbar_wait_bounded(bar_a, 0, limit)) {
             // the copies did not complete in time: flag it, give them a second
@@ -685,7 +688,7 @@ __global__ void __launch_bounds__(256, F ? 4 : R == 4 ? 1 : 3)
         for (int p = 0; p < run.np; ++p) {
             const TStage *ph = st + (p & 1);
             const int o0 = ph->ph.o0, no = ph->ph.no;
-            if (p + 1 < run.np) fetch(p + 1, o0 + no);
+            if (p + 1 < run.np) fetch(p + 1, o0 + no, ph->ph.nm);
             const uint32_t tw = ph->thr[tid];
             const uint32_t tl = tw & 0xffffu;
             A *t0 = tile + (tw >> 16);
