@@ -827,13 +827,14 @@ struct PackLaunch {
 };
 
 // Rows r0 .. r1 of sigma = H psi (a warp per row, the lanes over the row's
-// entries) and this CTA's share of <psi|H|psi>, summed in a fixed order.
+// entries) and, in warp 0, this CTA's share of <psi|H|psi>, its rows' parts (s_en,
+// kPackRows of them) summed in an order that does not depend on the block.
+constexpr int kPackRows = 512;
 template <class V>
 __device__ __forceinline__ double p_hpsi(const PackMember &m, int r0, int r1, const V *psi, V *sig,
-                                         double *s_red) {
+                                         double *s_en) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     constexpr int U = 4;  // row entries in flight per lane
-    double en = 0.0;
     for (int i = r0 + warp; i < r1; i += nw) {
         V acc = v_zero(V());
         const int e1 = m.rowptr[i + 1];
@@ -868,13 +869,15 @@ __device__ __forceinline__ double p_hpsi(const PackMember &m, int r0, int r1, co
         acc = p_sum1(acc);
         if (lane == 0) {
             sig[i] = acc;
-            en += v_cj(psi[i], acc).x;
+            s_en[i - r0] = v_cj(psi[i], acc).x;
         }
     }
-    if (lane == 0) s_red[warp] = en;
     __syncthreads();
     double t = 0.0;
-    for (int k = 0; k < nw; ++k) t += s_red[k];
+    if (warp == 0) {
+        for (int k = lane; k < r1 - r0; k += 32) t += s_en[k];
+        t = p_sum1(t);
+    }
     return t;
 }
 
@@ -940,7 +943,7 @@ __global__ void __launch_bounds__(kStepThreads, 2) k_pack_forward(PackLaunch P) 
 template <class V>
 __global__ void __launch_bounds__(kStepThreads, 2) k_pack_h(PackLaunch P) {
     extern __shared__ __align__(16) unsigned char s_raw[];
-    __shared__ double s_red[kStepThreads / 32];
+    __shared__ double s_en[kPackRows];
     const int x = blockIdx.y, q = blockIdx.x, tid = threadIdx.x;
     const int2 it = P.items[x];
     if ((unsigned)it.x >= (unsigned)P.nmem) return;
@@ -951,7 +954,7 @@ __global__ void __launch_bounds__(kStepThreads, 2) k_pack_h(PackLaunch P) {
     for (int i = tid; i < m.nsec; i += blockDim.x) psi[i] = sv[i];
     __syncthreads();
     const int r0 = (int)((int64_t)q * m.nsec / m.Q), r1 = (int)((int64_t)(q + 1) * m.nsec / m.Q);
-    const double e = p_hpsi<V>(m, r0, r1, psi, sv + P.maxsec, s_red);
+    const double e = p_hpsi<V>(m, r0, r1, psi, sv + P.maxsec, s_en);
     if (tid == 0) {
         P.epart[(size_t)x * P.Q + q] = e;
         __threadfence();
@@ -963,6 +966,29 @@ __global__ void __launch_bounds__(kStepThreads, 2) k_pack_h(PackLaunch P) {
             P.count[x] = 0u;
         }
     }
+}
+
+// The three in one CTA per item, for members whose rows one CTA takes (sectors below
+// 256 amplitudes): the launches would take longer than the work.  Energy and gradient,
+// us, three launches / this kernel: 64 items of 4 amplitudes 14.8 / 8.3, of 36 20.6 /
+// 14.4, of 100 29.8 / 21.5; 2,000 items 53 / 17, 70 / 53 and 114 / 90.
+template <class V>
+__global__ void __launch_bounds__(kStepThreads, sizeof(V) == sizeof(double) ? 2 : 1) k_pack_one(PackLaunch P) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    __shared__ double s_en[kPackRows];
+    int2 it;
+    if (!pack_item(P, blockIdx.x, it)) return;
+    const PackMember m = P.members[it.x];
+    V *psi = reinterpret_cast<V *>(s_raw);
+    const double *par = P.params + (size_t)blockIdx.x * P.maxparam;
+    pack_forward<V>(m, par, psi, step_coef<PCoef<false, V>>(s_raw, 1, m.nsec, sizeof(V)));
+    V *sv = reinterpret_cast<V *>(P.save) + (size_t)blockIdx.x * 2 * P.maxsec;
+    const double e = p_hpsi<V>(m, 0, m.nsec, psi, sv + P.maxsec, s_en);
+    if (threadIdx.x == 0) P.energy[blockIdx.x] = e;
+    if (!it.y || m.nparam == 0) return;
+    for (int i = threadIdx.x; i < m.nsec; i += blockDim.x) sv[i] = psi[i];
+    __syncthreads();  // psi and sigma are in the save buffer
+    pack_sweep<V>(P, m, par, sv, sv + P.maxsec, s_raw);
 }
 
 template <class V>

@@ -234,11 +234,11 @@ class Evaluator:
 
 
 class Pack:
-    """Parameter sets of several dUCC problems evaluated in one launch
-    (qfb_pack_*): every problem must take the compact shared-memory path
+    """Parameter sets of several dUCC problems evaluated side by side in a few
+    launches (qfb_pack_*): every problem must take the compact shared-memory path
     (``Evaluator.path == 2``: up to ~16 qubits) with the same state storage.
     Item i of a run evaluates ``params[i]`` of problem ``members[i]`` (an index
-    into ``duccs``), with its gradient when asked; one CTA per item."""
+    into ``duccs``), with its gradient when asked."""
 
     def __init__(self, duccs, capacity=256):
         self.duccs = list(duccs)
