@@ -4775,6 +4775,11 @@ struct PoolHost {
 // a wide sector needs more.
 constexpr size_t kPoolSmem = 48 * 1024, kPoolSmemMax = 200 * 1024;
 
+// A beta list's own cost in pairs (its coefficients, signs and reduction): without it
+// a task of a few strings took thousands of lists of one pair (11 orbitals, 4
+// electrons, 10,340 operators: 137 us, with it 16; 5 electrons 97 and 36).
+constexpr int64_t kPoolList = 64;
+
 static size_t pool_smem(const SectorPlan &sp, bool real, int ne) {
     return (size_t)ne * 2 * (size_t)sp.nbeta * (real ? 16 : 32);
 }
@@ -4824,12 +4829,12 @@ static bool build_pool(const SectorPlan &sp, const std::vector<CStep> &cs, int n
             for (size_t k = 0; k < a.size(); ++k)
                 P.signs[(size_t)l.s0 + k / 32] |= (pt.a[k].s & 1u) << (k & 31);
             alpha[(size_t)ia.first->second].meets.emplace_back(l, c.param);
-            total += (int64_t)a.size() * sp2.y;
+            total += (int64_t)a.size() * sp2.y + kPoolList * (((int64_t)a.size() + ne_max - 1) / ne_max);
         }
     P.signs.push_back(0u);  // (a task reads two words)
     // pairs of a task: about six tasks an SM (three: 126 us where six take 116,
     // sixteen 125: rows staged more often)
-    const int64_t most = std::max<int64_t>(4096, total / (6 * (int64_t)sm_count()));
+    const int64_t most = std::max<int64_t>(1024, total / (6 * (int64_t)sm_count()));
     std::vector<std::vector<int32_t>> idx((size_t)nop);
     for (const Alpha &A : alpha) {
         const int e0 = (int)P.ents.size(), na = (int)A.list.size(), k0 = (int)P.lists.size();
@@ -4842,7 +4847,8 @@ static bool build_pool(const SectorPlan &sp, const std::vector<CStep> &cs, int n
             for (int k = 0; k < (int)A.meets.size();) {
                 int64_t pairs = 0;
                 int j = k;
-                while (j < (int)A.meets.size() && (j - k < 8 || pairs < most)) pairs += (int64_t)n * A.meets[(size_t)j++].first.nb;
+                while (j < (int)A.meets.size() && (j - k < 8 || pairs < most))
+                    pairs += (int64_t)n * A.meets[(size_t)j++].first.nb + kPoolList;
                 const int lw = j - k <= 1 ? 3 : j - k <= 2 ? 2 : j - k <= 4 ? 1 : 0;
                 P.task.push_back(qfbg::GPoolTask{e0 + e, n, k0 + k, j - k, P.npart, e, lw, 0});
                 for (int q = k; q < j; ++q)
