@@ -20,6 +20,7 @@ Circuits that are canonical Pauli strings are held in mask form throughout.
 
 import functools
 
+from . import device
 from .circuit import _MASKS_DROPPED, Circuit, _product_masks
 from .pauli import canonical_key, ipow_mul
 
@@ -193,14 +194,23 @@ class QubitOperator:
         non-Pauli gate.  ``applied``: the operator each circuit applies when
         its gates run in list order (Computer::apply_operator semantics);
         otherwise the left-to-right product (operator-algebra semantics)."""
-        out = []
+        return self._gathered(applied)[0]
+
+    def _gathered(self, applied):
+        """_pauli_terms' list, and whether every circuit is held as masks."""
+        out, held = [], True
         for c, circ in self._t:
+            p = circ._pauli
+            if p is not None:
+                out.append((c, p[0], p[1]))
+                continue
+            held = False
             m = circ._applied_pauli_masks() if applied else circ._pauli_masks()
             if m is None:
-                return None
+                return None, False
             x, z, e = m
             out.append((ipow_mul(c, e), x, z))
-        return out
+        return out, held
 
     def _device_sum(self):
         """The operator each circuit applies in list order as a DeviceSum, or
@@ -208,16 +218,14 @@ class QubitOperator:
         of terms take milliseconds to gather, so the sum is kept until a method
         changes the terms, or a circuit held as Pauli masks is changed (gate
         lists are gathered on each call)."""
-        from .device import sum_from_terms
-
         terms = self._t
         kept, drops = terms.compiled, _MASKS_DROPPED[0]
         if kept is not None and kept[1] == drops:
             return kept[0]
-        pt = self._pauli_terms(applied=True)
+        pt, held = self._gathered(applied=True)
         if pt is None:
             return None
-        ds = sum_from_terms(pt)
-        if all(circ._pauli is not None for _, circ in terms):
+        ds = device.sum_from_terms(pt)
+        if held:
             terms.compiled = (ds, drops)
         return ds
