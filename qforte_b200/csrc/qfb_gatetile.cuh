@@ -575,7 +575,10 @@ __host__ __device__ __forceinline__ uint32_t tpad_size_of(int b) {
 // them, copied while the phase before runs.  Read from global memory as they
 // came up, each was an L2 access on the path of a CTA that has nothing else to
 // do: 12 qubits, 8 layers (4 runs of 4 CTAs) 95 us on the device, this way
-// 70 us.
+// 70 us.  Only as many ops as the phase holds: sixteen each time cost tiles of a few
+// threads, and states of many CTAs, whose reads hide behind each other, more than they
+// gave (4 qubits, 28 gates 25.1 us, own ops 19.0, unstaged 20.3; complex64, 23 qubits,
+// 340 gates 3,153, 2,961 and 2,956).
 constexpr int kStageOps = 16;
 struct TStage {
     TPhase ph;
