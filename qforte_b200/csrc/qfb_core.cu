@@ -508,10 +508,11 @@ int launch_single(qfb_state s, const HGate &h) { return launch_single_t(s->d, s-
 // qubits 213 / 197, 18 qubits 395 / 367; fused 21 qubits 800 / 777, 23 qubits 2,756 /
 // 2,708, 27 qubits 45,791 / 45,020), 10 for complex64.
 constexpr int kGateTileDefault = 11, kGateTileC64 = 10;
-// Gates on so few qubits that 10 tile bits hold them are one run either way, and on
-// states from 128 MiB on, read from HBM, the smaller tiles' copies overlap better
-// (10 / 11 bits, us: 2 gates on 23 qubits 57.6 / 61.7, 5 gates on 24 qubits 123 / 135, on
-// 26 qubits 449 / 499).
+// Gates on so few qubits that 10 tile bits hold them are one run either way, one-qubit
+// gates alone often as many runs, and on states from 128 MiB on, read from HBM, the
+// smaller tiles' copies overlap better (10 / 11 bits, us: 2 gates on 23 qubits 57.6 /
+// 61.7, 5 gates on 24 qubits 123 / 135, on 26 qubits 449 / 499; 8 layers of one-qubit gates
+// on 23 qubits 257 / 275).
 constexpr uint64_t kFewQubitsMin = 1ull << 23;
 constexpr int kGateTileMax = 12;
 int g_gate_tile_bits = 0;  // 0: kGateTileDefault; -1: one pass per gate
@@ -1528,9 +1529,15 @@ int apply_gates_tiles(A *d, int n, int nbatch, const std::vector<HGate> &hg) {
     const bool fused = g_gate_fused == 1 ||
                        (g_gate_fused == 2 && sizeof(A) * nbasis * (uint64_t)nbatch >= (c64 ? kFusedMinBytesC64 : kFusedMinBytes));
     if (fused && g_gate_tile_bits == 0 && !c64 && nbasis * (uint64_t)nbatch >= kFewQubitsMin) {
-        uint64_t q = (1ull << L) - 1ull;
-        for (const HGate &h : hg) q |= h.qubits;
-        if (__builtin_popcountll(q) <= kGateTileDefault - 1) b = std::max(kGateTileDefault - 1, L + 2);
+        uint64_t q = 0, pairs = 0;
+        for (const HGate &h : hg) {
+            q |= h.qubits;
+            pairs |= h.qubits & (h.qubits - 1);
+        }
+        // runs that hold h qubits above the lowest L, t of them a tile (one run, or no
+        // two-qubit gate binds them)
+        const int h = __builtin_popcountll(q >> L), t = kGateTileDefault - 1 - L;
+        if (t >= 2 && (h <= t || (!pairs && (h + t - 1) / t == (h + t) / (t + 1)))) b = kGateTileDefault - 1;
     }
     int rc = gate_tile_smem();
     if (rc) return rc;
